@@ -178,40 +178,44 @@ struct DFar {
 };
 
 // --------------------------------------------------------------- barriers
-__device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ uint64_t globaltimer_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
 
-// Grid-wide barrier for persistent (cooperatively launched) kernels.
-// bar[0] = arrival count, bar[1] = generation.  The wait is bounded by
+// Grid-wide barrier for persistent (cooperatively launched) kernels.  bar is
+// one 64-bit arrival count (two words, cleared before the launch) that only
+// grows: a block's own arrival tells it which barrier this is, and the wait is
+// for the count to reach the end of that barrier.  The wait is bounded by
 // timeout_ns; on expiry DEV_ERR_TIMEOUT is raised in *err and the function
 // returns false so the caller can leave its loop.  Replaces
 // cooperative_groups::this_grid().sync() (gpu_intrinsics.h:113-117), whose wait
 // has no limit.
+//
+// A barrier is a chain of dependent L2 round trips (0.65 us each here with
+// gpu-scope ordering), not of bandwidth: with a generation word it took four
+// (read it, arrive, publish it, see it), 2.5 us at 304 blocks and 3.1 us at
+// 608; arriving and polling one count takes two, 1.5 us and 2.2 us.  64 bits,
+// because a loop of a 1.5 us barrier passes 2^32 arrivals within seconds.
+__device__ __forceinline__ uint64_t ld_acquire64(const uint32_t *p) {
+  uint64_t v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
 __device__ __forceinline__ bool grid_barrier(uint32_t *bar, uint32_t nblocks, int32_t *err,
                                              uint64_t timeout_ns) {
   __syncthreads();
   __shared__ int ok_s;
   if (threadIdx.x == 0) {
     ok_s = 1;
-    const uint32_t gen = ld_acquire(bar + 1);
-    __threadfence();
-    const uint32_t arrived = atomicAdd(bar, 1u);
-    if (arrived == nblocks - 1) {
-      atomicExch(bar, 0u);
-      __threadfence();
-      atomicAdd(bar + 1, 1u);
-    } else {
+    uint64_t old;
+    asm volatile("atom.add.acq_rel.gpu.global.u64 %0, [%1], 1;" : "=l"(old) : "l"(bar) : "memory");
+    const uint64_t end = (old / nblocks + 1) * nblocks;
+    if (old + 1 != end) {
       const uint64_t t0 = globaltimer_ns();
       uint32_t spins = 0;
-      while (ld_acquire(bar + 1) == gen) {
+      while (ld_acquire64(bar) < end) {
         if ((++spins & 255u) == 0) {
           if (*(volatile int32_t *)err & DEV_ERR_TIMEOUT) { ok_s = 0; break; }
           if (globaltimer_ns() - t0 > timeout_ns) {
@@ -220,7 +224,6 @@ __device__ __forceinline__ bool grid_barrier(uint32_t *bar, uint32_t nblocks, in
             break;
           }
         }
-        __nanosleep(32);
       }
     }
     __threadfence();
@@ -230,10 +233,10 @@ __device__ __forceinline__ bool grid_barrier(uint32_t *bar, uint32_t nblocks, in
 }
 
 // Waits, without arriving, until every other block has arrived at the next
-// grid_barrier (bar[0] counts arrivals and the previous barrier's last block
-// reset it, so nblocks-1 arrivals means all others are inside the wait).  The
-// caller then works alone and completes the barrier by calling grid_barrier
-// itself.  Bounded like grid_barrier; false after the limit.
+// grid_barrier (the count, modulo nblocks, is the arrivals of the barrier that is
+// open, and this block's is missing: nblocks-1 of them mean all others are inside
+// the wait).  The caller then works alone and completes the barrier by calling
+// grid_barrier itself.  Bounded like grid_barrier; false after the limit.
 __device__ __forceinline__ bool grid_wait_others(const uint32_t *bar, uint32_t nblocks, int32_t *err,
                                                  uint64_t timeout_ns) {
   __shared__ int ok_o;
@@ -241,7 +244,8 @@ __device__ __forceinline__ bool grid_wait_others(const uint32_t *bar, uint32_t n
     ok_o = 1;
     const uint64_t t0 = globaltimer_ns();
     uint32_t spins = 0;
-    while (ld_acquire(bar) < nblocks - 1) {
+    const uint64_t all = ld_acquire64(bar) / nblocks * nblocks + nblocks - 1;
+    while (ld_acquire64(bar) < all) {
       if ((++spins & 255u) == 0) {
         if (*(volatile int32_t *)err & DEV_ERR_TIMEOUT) { ok_o = 0; break; }
         if (globaltimer_ns() - t0 > timeout_ns) {

@@ -48,7 +48,7 @@ struct gg_graph {
   cudaStream_t stream = nullptr;
   cudaStream_t own_stream = nullptr;
   int32_t *d_err = nullptr;       // device status word (DEV_ERR_*)
-  uint32_t *d_bar = nullptr;      // grid barrier state [2]
+  uint32_t *d_bar = nullptr;      // grid barrier arrivals (one 64-bit count)
   int32_t *d_misc = nullptr;      // small device scratch (counters, flags), 64 ints
   int32_t *h_pinned = nullptr;    // pinned host scratch, 64 ints
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // whole trial

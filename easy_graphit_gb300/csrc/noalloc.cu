@@ -27,7 +27,8 @@
 namespace gg {
 
 constexpr int32_t kNoAllocMaxVertices = 1 << 20;
-constexpr int32_t kNoAllocHeader = 64;  // ints: counts[3], barrier[2], err, iterations
+constexpr int32_t kNoAllocHeader = 64;  // ints: counts[3], -, -, err, iterations, -, barrier[2]
+constexpr int32_t kNoAllocBar = 8;      // the barrier's 64-bit count, 8-byte aligned
 constexpr int kNoAllocMaxDevices = 64;
 
 static __device__ __align__(256) int32_t g_noalloc_scratch[kNoAllocHeader + 2 * kNoAllocMaxVertices];
@@ -66,8 +67,8 @@ __global__ void k_noalloc_init(int32_t *scratch, int32_t *depth, int32_t V, int3
     scratch[0] = 1;  // count of the first queue: {src}
     scratch[1] = 0;
     scratch[2] = 0;
-    scratch[3] = 0;  // barrier arrivals
-    scratch[4] = 0;  // barrier generation
+    scratch[kNoAllocBar] = 0;  // barrier arrivals (64 bits)
+    scratch[kNoAllocBar + 1] = 0;
     scratch[5] = 0;  // status word
     scratch[6] = 0;  // iterations
     scratch[kNoAllocHeader] = src;
@@ -78,7 +79,7 @@ __global__ void __launch_bounds__(512) k_noalloc_bfs(DGraph g, int32_t *scratch,
                                                      uint64_t timeout_ns) {
   extern __shared__ int4 smem[];
   int32_t *cnt3 = scratch;
-  uint32_t *bar = reinterpret_cast<uint32_t *>(scratch + 3);
+  uint32_t *bar = reinterpret_cast<uint32_t *>(scratch + kNoAllocBar);
   int32_t *err = scratch + 5;
   int32_t *qs[2] = {scratch + kNoAllocHeader, scratch + kNoAllocHeader + kNoAllocMaxVertices};
   int in = 0;
