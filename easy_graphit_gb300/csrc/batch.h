@@ -111,6 +111,8 @@ struct MsBfsState {
   int32_t *qstamp;            // V: last top-down level v was queued at
   int32_t *q[3];              // queue of level L in q[L % 3]
   int32_t *cnt4;              // [4] queue count of level L in cnt4[L % 4]
+  int32_t *hub_list, *hub3;   // hub chunks of a top-down level and their counts [L % 3]
+  int32_t hub_cap;
   const int32_t *toff, *tsrc; // in-lists, for bottom-up levels
   int32_t V;
   int32_t bu_div;             // bottom-up when the frontier holds more than V / bu_div vertices (<= 0: never)

@@ -54,6 +54,8 @@ struct BcState {
   uint32_t *bar;
   int32_t *err;
   uint64_t timeout_ns;
+  int32_t *hub_list;             // hub chunks of a relax (counts: ctr[21..23], by level)
+  int32_t hub_cap;
   int32_t *stats;                // [0] levels
   int32_t *stop;
   uint64_t loop_limit_ns;
@@ -193,6 +195,7 @@ __global__ void __launch_bounds__(512) k_bc_batch(DGraph g, BcState st) {
       st.loff[d + 1] = e_d;
       st.ctr[1 + (d & 1)] = 0;  // items of Q_{d+1}, filled by the publish below
       st.ctr[16 + ((d + 1) & 1)] = 0;  // hand-out counter of the next level's gather
+      st.ctr[21 + (d + 1) % 3] = 0;    // hub chunks of the next level's relax
     }
     // sigma of Q_d from Q_{d-1} (items made by the previous publish)
     if (d > 0) {
@@ -227,20 +230,22 @@ __global__ void __launch_bounds__(512) k_bc_batch(DGraph g, BcState st) {
       const int32_t n = e_d - b_d;
       const Enum en{st.lev + b_d, nullptr, n};
       const UMsBfs f{st.seen, bc_fr(st, d), st.acc, st.qstamp, d + 1};
+      const HubList hub{st.hub_list, st.ctr + 21 + d % 3, st.hub_cap, kHubWidths * (int32_t)blockDim.x};
       DOut out{};
       out.mode = OUT_SPARSE;
       out.q = st.lev;
       out.cnt = st.ctr + 0;
       out.cap = st.levcap;
       out.err = st.err;
-      const int32_t nv = ceil_div(n, blockDim.x / kStage1);
-      for (int32_t vc = blockIdx.x; vc < nv; vc += gridDim.x)
-        lb_twce<UMsBfs, true>(g, en, n, f, out, vc, *reinterpret_cast<TwceSmem *>(smem));
+      lb_twce_all(g, en, n, f, out, blockIdx.x, gridDim.x, *reinterpret_cast<TwceSmem *>(smem), hub);
+      alive = grid_barrier(st.bar, gridDim.x, st.err, st.timeout_ns);
+      const int32_t chunks = *(volatile int32_t *)hub.cnt;
+      if (alive && chunks > 0) {  // the hubs the level set aside, by all CTAs
+        lb_hubs(g, hub, chunks, f, out, blockIdx.x, gridDim.x);
+        alive = grid_barrier(st.bar, gridDim.x, st.err, st.timeout_ns);
+      }
     }
-    if (!grid_barrier(st.bar, gridDim.x, st.err, st.timeout_ns)) {
-      alive = false;
-      break;
-    }
+    if (!alive) break;
     // publish Q_{d+1}: masks, depths, and its sigma work items
     {
       e_next = min(*(volatile int32_t *)(st.ctr + 0), st.levcap);
@@ -427,6 +432,7 @@ gg_status bcb_buffers(gg_graph *g, bool owned, BcBuffers *b) {
     return set_error(GG_ERR_UNSUPPORTED, "batched BC holds 64 level-list entries per vertex in int32: "
                                          "V = %d is too large (use gg_bc)", V);
   GG_TRY(ensure_transpose(g));
+  GG_TRY(ensure_hubs(g));
   // walk the degree-ordered copy: the rows of the most-gathered vertices share L2
   GG_TRY(ensure_relabel(g));
   if (!g->symmetric) GG_TRY(ensure_relabel_csc(g));  // its in-lists (a symmetric copy serves both)
@@ -465,6 +471,8 @@ static BcState bcb_state(gg_graph *g, const BcBuffers &b, int32_t k) {
   S.levcap = (int32_t)bc_levcap(V);
   S.loff = S.lev + S.levcap;
   S.ctr = S.loff + kBcMaxLevels + 2;
+  S.hub_list = static_cast<int32_t *>(g->hubs.p);
+  S.hub_cap = hub_capacity(g);
   S.stats = S.ctr + 8;
   S.stop = S.ctr + 12;
   S.work = b.work;

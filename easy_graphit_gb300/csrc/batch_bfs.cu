@@ -74,6 +74,7 @@ __global__ void __launch_bounds__(512) k_msbfs(DGraph g, MsBfsState st) {
     if (tid == 0) {
       st.cnt4[(L + 2) & 3] = 0;
       st.actm[(L + 2) % 3] = 0ull;
+      st.hub3[(L + 1) % 3] = 0;
       for (int i = 0; i < 4; ++i) st.lstat[4 * ((L + 2) % 3) + i] = 0ull;
     }
     if (threadIdx.x == 0) {
@@ -110,19 +111,18 @@ __global__ void __launch_bounds__(512) k_msbfs(DGraph g, MsBfsState st) {
     const uint64_t *frc = ms_fr(st, L);
     uint64_t *frn = ms_fr(st, L + 1);
     int32_t *qn = ms_q(st, L + 1);
+    // top-down: acc[v] |= fr[u] & ~seen[v]; the first toucher queues v
+    const UMsBfs f{st.seen, frc, st.acc, st.qstamp, L + 1};
+    const HubList hub{st.hub_list, st.hub3 + L % 3, st.hub_cap, kHubWidths * (int32_t)blockDim.x};
+    DOut out{};
+    out.mode = OUT_SPARSE;
+    out.q = qn;
+    out.cnt = st.cnt4 + ((L + 1) & 3);
+    out.cap = st.V;  // qstamp admits each vertex once per level
+    out.err = st.err;
     if (!bu) {
-      // top-down: acc[v] |= fr[u] & ~seen[v]; the first toucher queues v
       const Enum en{ms_q(st, L), nullptr, n};
-      const UMsBfs f{st.seen, frc, st.acc, st.qstamp, L + 1};
-      DOut out{};
-      out.mode = OUT_SPARSE;
-      out.q = qn;
-      out.cnt = st.cnt4 + ((L + 1) & 3);
-      out.cap = st.V;  // qstamp admits each vertex once per level
-      out.err = st.err;
-      const int32_t nv = ceil_div(n, blockDim.x / kStage1);
-      for (int32_t v = blockIdx.x; v < nv; v += gridDim.x)
-        lb_twce<UMsBfs, true>(g, en, n, f, out, v, *reinterpret_cast<TwceSmem *>(smem));
+      lb_twce_all(g, en, n, f, out, blockIdx.x, gridDim.x, *reinterpret_cast<TwceSmem *>(smem), hub);
     } else {
       // bottom-up: 8-lane groups over the vertices still wanted by some source
       ++bu_levels;
@@ -161,6 +161,13 @@ __global__ void __launch_bounds__(512) k_msbfs(DGraph g, MsBfsState st) {
       }
     }
     if (!grid_barrier(st.bar, gridDim.x, st.err, st.timeout_ns)) break;
+    if (!bu) {  // the hubs the level set aside, by all CTAs
+      const int32_t chunks = *(volatile int32_t *)hub.cnt;
+      if (chunks > 0) {
+        lb_hubs(g, hub, chunks, f, out, blockIdx.x, gridDim.x);
+        if (!grid_barrier(st.bar, gridDim.x, st.err, st.timeout_ns)) break;
+      }
+    }
     // publish (top-down levels): new bits become the next level's masks
     if (!bu) {
       const int32_t m = min(*(volatile int32_t *)(st.cnt4 + ((L + 1) & 3)), st.V);
@@ -235,6 +242,7 @@ __global__ void k_msbfs_seed(MsBfsState st, const int32_t *__restrict__ srcs) {
   }
   for (int i = 0; i < 4; ++i) st.cnt4[i] = 0;
   st.cnt4[0] = n;
+  for (int i = 0; i < 3; ++i) st.hub3[i] = 0;
   for (int i = 0; i < 12; ++i) st.lstat[i] = 0ull;
   for (int32_t i = 0; i < n; ++i) {  // the sources' frontier
     const unsigned long long d = (unsigned long long)(st.off[st.q[0][i] + 1] - st.off[st.q[0][i]]);
@@ -257,6 +265,7 @@ MsBfsBuffers::~MsBfsBuffers() {
 
 gg_status msbfs_buffers(gg_graph *g, int32_t nsrc, bool owned, MsBfsBuffers *b) {
   GG_TRY(ensure_transpose(g));  // in-lists for the bottom-up levels
+  GG_TRY(ensure_hubs(g));
   const int32_t V = g->csr.V;
   b->owned = owned;
   const size_t sz[3] = {sizeof(uint64_t) * (5 * (size_t)V + 24), sizeof(int32_t) * (4 * (size_t)V + 64),
@@ -286,6 +295,9 @@ MsBfsState msbfs_state(gg_graph *g, const MsBfsBuffers &b, int32_t k, int32_t *d
   S.cnt4 = hdr;          // 4
   S.stats = hdr + 8;     // 2
   S.stop = hdr + 12;
+  S.hub3 = hdr + 16;     // 3
+  S.hub_list = static_cast<int32_t *>(g->hubs.p);
+  S.hub_cap = hub_capacity(g);
   S.toff = t.off;
   S.tsrc = t.dst;
   S.V = V;

@@ -69,6 +69,7 @@ gg_status gg_batch_plan_create(gg_graph *g, int32_t app, const int32_t *sources,
   GG_CUDA(cudaMalloc(&p->dstats, sizeof(int32_t) * 2 * p->ngroups));
   if (multi) {
     if (!g->app_frontier) GG_TRY(gg_frontier_create(g, 0, &g->app_frontier));
+    GG_TRY(ensure_hubs(g));
     if (app == GG_BATCH_BFS_MULTI) GG_CUDA(cudaMalloc(&p->parent, sizeof(int32_t) * std::max(V, 1)));
     if (app == GG_BATCH_SSSP_MULTI) GG_TRY(bq_alloc(g, &p->bq));
   } else if (app == GG_BATCH_BFS) {

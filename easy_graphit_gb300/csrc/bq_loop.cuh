@@ -13,7 +13,8 @@ namespace gg {
 // takes every nparts-th virtual CTA (nparts = 1: one CTA does all of it).
 template <int LB, class F>
 __device__ __forceinline__ void run_lb(const DGraph &g, const Enum &en, int32_t n, const F &f,
-                                       const DOut &out, int4 *smem, int32_t rank, int32_t nparts) {
+                                       const DOut &out, int4 *smem, int32_t rank, int32_t nparts,
+                                       const HubList &hub) {
   if (LB == GG_LB_VERTEX_BASED) {
     const int32_t nv = ceil_div(n, blockDim.x);
     for (int32_t v = rank; v < nv; v += nparts) lb_vertex(g, en, n, f, out, v);
@@ -21,9 +22,7 @@ __device__ __forceinline__ void run_lb(const DGraph &g, const Enum &en, int32_t 
     const int32_t nv = ceil_div(n, blockDim.x >> 5);
     for (int32_t v = rank; v < nv; v += nparts) lb_wm(g, en, n, f, out, v);
   } else if (LB == GG_LB_TWCE) {
-    const int32_t nv = ceil_div(n, blockDim.x / kStage1);
-    for (int32_t v = rank; v < nv; v += nparts)
-      lb_twce<F, true>(g, en, n, f, out, v, *reinterpret_cast<TwceSmem *>(smem));
+    lb_twce_all(g, en, n, f, out, rank, nparts, *reinterpret_cast<TwceSmem *>(smem), hub);
   } else {
     const int32_t nv = ceil_div(n, blockDim.x);
     for (int32_t v = rank; v < nv; v += nparts)
@@ -36,6 +35,8 @@ __device__ __forceinline__ void run_lb(const DGraph &g, const Enum &en, int32_t 
 // bucket_queue.cuh, as a sequence of steps, each one of
 //   relax     the frontier with cutoff cur+delta (improvements below it queue
 //             the vertex, the others park it on a far pile),
+//   hubs      the chunks of long lists that the relax set aside (lb.cuh), by
+//             all CTAs; part of that relax: same window, same output queue,
 //   lo-min    exact minimum of the low pile's live entries,
 //   lo-split  window entries to the frontier, the rest to the next low pile
 //             (a window reaching past the horizon splits the high pile too),
@@ -45,7 +46,7 @@ __device__ __forceinline__ void run_lb(const DGraph &g, const Enum &en, int32_t 
 // __syncthreads when one CTA runs them).  Frontier counts and minima rotate
 // through three slots: a step clears the slot two steps ahead, whose readers
 // finished before the previous synchronisation.
-enum : int32_t { BQ_RELAX = 0, BQ_LOMIN = 1, BQ_LOSPLIT = 2, BQ_HIMIN = 3, BQ_HISPLIT = 4, BQ_DONE = 5 };
+enum : int32_t { BQ_RELAX = 0, BQ_LOMIN = 1, BQ_LOSPLIT = 2, BQ_HIMIN = 3, BQ_HISPLIT = 4, BQ_DONE = 5, BQ_HUBS = 6 };
 constexpr uint64_t kSoloSliceNs = 1000000;
 
 struct BqArgs {
@@ -62,6 +63,8 @@ struct BqArgs {
   int32_t solo_pile_max;  // largest pile step (pile entries) CTA 0 runs alone
   int32_t fill_target;  // low-pile entries a refill aims for
   int32_t width0;       // first horizon width, in buckets
+  int32_t *hub_list;    // hub chunks (HubList); their counts are control words
+  int32_t hub_cap, hub_min;
 };
 
 // Loop state, the same in every CTA: every decision is taken from control
@@ -75,8 +78,9 @@ struct BqLoop {
   int32_t k;      // horizon width in buckets
   int32_t phase;  // 0: normal, 1: after a lo-min, 2: after a hi-min
   int32_t relax, adv;
+  int32_t hub;    // 1: the last step was a relax, whose hub chunks may be pending
 };
-constexpr int kBqLoopInts = 10;
+constexpr int kBqLoopInts = 11;
 static_assert(sizeof(BqLoop) == kBqLoopInts * sizeof(int32_t), "BqLoop is published as ints");
 
 struct BqStep {
@@ -86,13 +90,19 @@ struct BqStep {
 // Small enough for CTA 0 alone: frontier entries of a relax, pile entries of
 // the other steps (one load and a compare each).
 __device__ __forceinline__ bool bq_small(const BqStep &st, const BqArgs &a) {
-  return st.work <= (st.kind == BQ_RELAX ? a.solo_max : a.solo_pile_max);
+  return st.kind != BQ_HUBS && st.work <= (st.kind == BQ_RELAX ? a.solo_max : a.solo_pile_max);
 }
 
 // The next step (pure: every CTA computes the same one).
 __device__ __forceinline__ BqStep bq_decide(const BqLoop &s, const int32_t *ctl, int32_t delta) {
   const volatile int32_t *c = ctl;
   const int32_t prev = (s.it + 2) % 3;
+  if (s.hub) {
+    const int32_t n = c[BQ_NEAR + prev];  // loaded with the hub count: one round trip
+    const int32_t nh = c[BQ_HUB + (s.relax + 2) % 3];
+    if (nh > 0) return BqStep{BQ_HUBS, nh, 0};
+    if (n > 0) return BqStep{BQ_RELAX, n, 0};
+  }
   if (s.phase == 1) {
     const int32_t m = c[BQ_MIN + prev];
     if (m != INT_MAX) {
@@ -134,19 +144,36 @@ __device__ __forceinline__ void bq_step(BqLoop &s, const BqArgs &a, const BqStep
   front.cap = a.qcap;
   front.err = a.err;
   const int32_t lo_next = (s.g + 1) & 1;
-  switch (st.kind) {
-    case BQ_RELAX: {
-      const DFar far{a.b.stamp, a.b.lo[s.g & 1], ctl + BQ_LO + (s.g & 1), a.b.hi[s.gh & 1],
-                     ctl + BQ_HI + (s.gh & 1), bq_lo_tag(s.g), bq_hi_tag(s.gh), s.hz, a.b.V, a.err};
-      const EdgeF<USssp, false> f{USssp{a.dist, U, far}, DIn{IN_ALL, nullptr, nullptr},
-                                  DIn{IN_ALL, nullptr, nullptr}, false};
-      const int32_t n = (int64_t)st.work > a.qcap ? (int32_t)a.qcap : st.work;  // past qcap only after a flagged overflow
-      run_lb<LB>(a.g, Enum{qin, nullptr, n}, n, f, front, smem, rank, nparts);
-      s.in ^= 1;
-      s.relax++;
-      s.phase = 0;
-      break;
+  if (st.kind == BQ_RELAX || st.kind == BQ_HUBS) {
+    const bool hubs = st.kind == BQ_HUBS;
+    // a hub step finishes the relax before it: into that step's queue and count
+    if (hubs) {
+      front.q = qin;
+      front.cnt = ctl + BQ_NEAR + (s.it + 2) % 3;
     }
+    const DFar far{a.b.stamp, a.b.lo[s.g & 1], ctl + BQ_LO + (s.g & 1), a.b.hi[s.gh & 1],
+                   ctl + BQ_HI + (s.gh & 1), bq_lo_tag(s.g), bq_hi_tag(s.gh), s.hz, a.b.V, a.err};
+    const EdgeF<USssp, false> f{USssp{a.dist, U, far}, DIn{IN_ALL, nullptr, nullptr},
+                                DIn{IN_ALL, nullptr, nullptr}, false};
+    if (hubs) {
+      const HubList hub{a.hub_list, nullptr, a.hub_cap, 0};
+      lb_hubs(a.g, hub, st.work, f, front, rank, nparts);
+      s.hub = 0;
+      return;
+    }
+    if (lead) ctl[BQ_HUB + (s.relax + 1) % 3] = 0;
+    const HubList hub{a.hub_list, ctl + BQ_HUB + s.relax % 3, a.hub_cap, a.hub_min};
+    const int32_t n = (int64_t)st.work > a.qcap ? (int32_t)a.qcap : st.work;  // past qcap only after a flagged overflow
+    run_lb<LB>(a.g, Enum{qin, nullptr, n}, n, f, front, smem, rank, nparts, hub);
+    s.in ^= 1;
+    s.relax++;
+    s.phase = 0;
+    s.hub = 1;
+    s.it++;
+    return;
+  }
+  s.hub = 0;
+  switch (st.kind) {
     case BQ_LOMIN:
       if (s.phase == 0) s.adv++;
       if (lead) {

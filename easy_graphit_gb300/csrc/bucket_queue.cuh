@@ -52,9 +52,10 @@ enum : int32_t {
   BQ_LO = 6,      // [2] low-pile counts, by generation parity
   BQ_HI = 8,      // [2] high-pile counts, by generation parity
   BQ_FILL = 10,   // [2] entries a refill moved to the low pile, by high generation parity
-  BQ_STOP = 12,   // loop time-limit flag
-  BQ_STATS = 13,  // [2] relax steps, bucket advances
-  BQ_PUB = 16,    // [16] loop state published by the one-CTA mode
+  BQ_HUB = 12,    // [3] hub chunks, by relax step
+  BQ_STOP = 15,   // loop time-limit flag
+  BQ_STATS = 16,  // [2] relax steps, bucket advances
+  BQ_PUB = 20,    // [12] loop state published by the one-CTA mode
   BQ_CTL_INTS = 32
 };
 

@@ -64,6 +64,7 @@ struct gg_graph {
   gg_batch_tuning tuning[3] = {};  // batched BFS, SSSP, BC launch shapes (0 = default)
   const gg_selector *batch_selector[3] = {};  // learned per-level choices of the batched kernels
   gg::Scratch bq_cta;             // batched SSSP with a CTA per source
+  gg::Scratch hubs;               // hub chunks of TWCE in the persistent loops (ensure_hubs)
   int32_t max_degree = -1;        // largest out-degree (-1: not computed yet)
 };
 
@@ -135,6 +136,11 @@ inline cudaError_t dev_alloc(T **p, size_t bytes, cudaStream_t st) {
 gg_status ensure_transpose(gg_graph *g);
 gg_status ensure_coo(GraphStore &s, cudaStream_t st);
 gg_status ensure_blocked(gg_graph *g, bool reverse, int32_t block_size, const GraphStore **out);
+// The graph's hub list (lb.cuh HubList): room for every list cut into the
+// shortest chunks (the smallest CTA's) and as many ragged ends; allocated once,
+// so plans may keep its address.  Loops on the graph's stream share it.
+int32_t hub_capacity(const gg_graph *g);
+gg_status ensure_hubs(gg_graph *g);
 gg_status check_device_error(gg_graph *g, const char *what);
 gg_status scratch_get(gg_graph *g, int slot, size_t bytes, void **p);
 gg_status scratch_get_app(gg_graph *g, int slot, size_t bytes, void **p);

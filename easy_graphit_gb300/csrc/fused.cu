@@ -65,7 +65,16 @@ struct FusedArgs {
   int32_t *gmin2;  // SSSP bucket-advance minima [2]
   int32_t *stop;   // loop time limit flag (see LoopClock)
   uint64_t loop_limit_ns;
+  int32_t *hub_list;  // hub chunks (lb.cuh) of a level
+  int32_t *hub3;      // their rotating counts [3]
+  int32_t hub_cap, hub_min;
 };
+
+// The hub list of level `level`; its count is cleared two levels ahead, with
+// the queue's.
+__device__ __forceinline__ HubList level_hubs(const FusedArgs &a, int64_t level) {
+  return HubList{a.hub_list, a.hub3 + level % 3, a.hub_cap, a.hub_min};
+}
 
 __device__ __forceinline__ DOut sparse_out(const FusedArgs &a, int32_t *q, int64_t it) {
   DOut o{};
@@ -85,16 +94,28 @@ __global__ void __launch_bounds__(1024) k_bfs_fused(FusedArgs a) {
   int64_t level = 1;
   LoopClock clk;
   clk.start(a.loop_limit_ns);
+  int32_t n = *(volatile int32_t *)a.cnt3;
   for (;; ++level) {
-    const int32_t n = *(volatile int32_t *)(a.cnt3 + (level - 1) % 3);
     if (n == 0 || stopped(a.stop, (int32_t)level)) break;
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.cnt3[(level + 1) % 3] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      a.cnt3[(level + 1) % 3] = 0;
+      a.hub3[(level + 1) % 3] = 0;
+    }
     const Enum en{qs[in], nullptr, n};
+    const HubList hub = level_hubs(a, level);
     const EdgeF<UBfs, false> f{UBfs{a.vd.parent, a.vd.depth, (int32_t)level},
                                DIn{IN_ALL, nullptr, nullptr}, DIn{IN_ALL, nullptr, nullptr}, true};
-    run_lb<LB>(a.g, en, n, f, sparse_out(a, qs[in ^ 1], level), smem, blockIdx.x, gridDim.x);
+    const DOut out = sparse_out(a, qs[in ^ 1], level);
+    run_lb<LB>(a.g, en, n, f, out, smem, blockIdx.x, gridDim.x, hub);
     clk.tick(a.stop, (int32_t)level, a.err);
     if (!grid_barrier(a.bar, gridDim.x, a.err, a.timeout_ns)) break;
+    const int32_t chunks = *(volatile int32_t *)hub.cnt;
+    n = *(volatile int32_t *)out.cnt;
+    if (chunks) {  // the level's hubs, by all CTAs
+      lb_hubs(a.g, hub, chunks, f, out, blockIdx.x, gridDim.x);
+      if (!grid_barrier(a.bar, gridDim.x, a.err, a.timeout_ns)) break;
+      n = *(volatile int32_t *)out.cnt;
+    }
     in ^= 1;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) a.stats[0] = (int32_t)(level - 1);
@@ -157,7 +178,7 @@ __global__ void __launch_bounds__(1024) k_sssp_bq(BqArgs a) {
   extern __shared__ int4 smem[];
   __shared__ int32_t red[33];
   __shared__ int32_t sctl[BQ_STOP];  // counts and minima of a one-CTA session
-  BqLoop s{1, 0, 0, 0, 0, bq_clamp((int64_t)a.width0 * a.delta), a.width0, 0, 0, 0};
+  BqLoop s{1, 0, 0, 0, 0, bq_clamp((int64_t)a.width0 * a.delta), a.width0, 0, 0, 0, 0};
   int32_t *stop = a.b.ctl + BQ_STOP;
   LoopClock clk;
   clk.start(a.loop_limit_ns);
@@ -242,7 +263,7 @@ static size_t lb_smem(int lb, int cta) {
   return 0;
 }
 
-static FusedArgs make_args(gg_graph *g, gg_frontier *f, const VData &vd) {
+static FusedArgs make_args(gg_graph *g, gg_frontier *f, const VData &vd, int cta) {
   FusedArgs a{};
   a.g = g->csr.view();
   a.g.nbuckets = 0;
@@ -258,6 +279,10 @@ static FusedArgs make_args(gg_graph *g, gg_frontier *f, const VData &vd) {
   a.gmin2 = g->d_misc + 46;
   a.stop = g->d_misc + 48;
   a.loop_limit_ns = loop_timeout_ns();
+  a.hub_list = static_cast<int32_t *>(g->hubs.p);
+  a.hub3 = g->d_misc + 49;
+  a.hub_cap = hub_capacity(g);
+  a.hub_min = kHubWidths * cta;
   return a;
 }
 
@@ -273,7 +298,8 @@ static gg_status init_counts(gg_graph *g, int32_t n0) {
   h[6] = INT_MAX;
   h[7] = INT_MAX;
   h[8] = 0;  // stop flag
-  GG_CUDA(cudaMemcpyAsync(g->d_misc + 40, h, sizeof(int32_t) * 9, cudaMemcpyHostToDevice, g->stream));
+  h[9] = h[10] = h[11] = 0;  // hub chunk counts
+  GG_CUDA(cudaMemcpyAsync(g->d_misc + 40, h, sizeof(int32_t) * 12, cudaMemcpyHostToDevice, g->stream));
   return GG_OK;
 }
 
@@ -290,9 +316,10 @@ gg_status fused_bfs(gg_graph *g, const gg_schedule *s, int32_t n0, const VData &
                     int32_t *iters, bool *ran) {
   *ran = false;
   if (!fused_supported(s)) return GG_OK;
+  GG_TRY(ensure_hubs(g));
   GG_TRY(init_counts(g, n0));
-  FusedArgs a = make_args(g, f, vd);
   const int cta = s->cta_size;
+  FusedArgs a = make_args(g, f, vd, cta);
   const size_t sm = lb_smem(s->load_balancing, cta);
   switch (s->load_balancing) {
     case GG_LB_VERTEX_BASED: GG_TRY(coop_launch(g, k_bfs_fused<GG_LB_VERTEX_BASED>, cta, sm, a)); break;
@@ -436,6 +463,7 @@ __global__ void __launch_bounds__(kBfsDoMaxCta, 4) k_bfs_do(DoKernelArgs ka, uin
         s_pull = pull;
         if (blockIdx.x == 0) {
           a.cnt3[(level + 1) % 3] = 0;
+          a.hub3[(level + 1) % 3] = 0;
           if (d.stats)
             for (int i = 0; i < 4; ++i) d.lstat[4 * ((level + 1) % 3) + i] = 0ull;
           if (logged) {
@@ -450,55 +478,72 @@ __global__ void __launch_bounds__(kBfsDoMaxCta, 4) k_bfs_do(DoKernelArgs ka, uin
     const bool pull = s_pull != 0;
     DoStat *stat = d.stats ? &s_stat : nullptr;
     const DOut out = sparse_out(a, (level & 1) ? a.q1 : a.q0, level);
-    if (!pull) {
-      const Enum en{(level & 1) ? a.q0 : a.q1, nullptr, n};
-      const EdgeF<UBfsNote, false> f{UBfsNote{a.vd.parent, a.vd.depth, a.g.off, stat, level},
-                                     DIn{IN_ALL, nullptr, nullptr}, DIn{IN_ALL, nullptr, nullptr}, true};
-      run_lb<LB>(a.g, en, n, f, out, smem, blockIdx.x, gridDim.x);
-    } else {
-      if (threadIdx.x == 0) ++s_pulls;
-      const int32_t lane = threadIdx.x & 31, sub = lane & 7, gbase = lane & ~7;
-      const uint32_t gmask = 0xFFu << gbase;
-      const int32_t prev = level - 1;
-      for (int32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; v < a.g.V;
-           v += (gridDim.x * blockDim.x) >> 3) {
-        if (__ldcg(a.vd.parent + v) != -1) continue;
-        const int32_t kb = __ldg(d.t.off + v), ke = __ldg(d.t.off + v + 1);
-        const int32_t deg = stat && sub == 0 ? __ldg(a.g.off + v + 1) - __ldg(a.g.off + v) : 0;
-        int32_t hit = -1;
-        for (int32_t k0 = kb; k0 < ke; k0 += 8) {
-          int32_t u = -1;
-          if (k0 + sub < ke) {
-            u = __ldg(d.t.dst + k0 + sub);
-            if (__ldcg(a.vd.depth + u) != prev) u = -1;
+    const HubList hub = level_hubs(a, level);
+    // One pass over the frontier or the unreached vertices; a push level that
+    // set hubs aside (lb.cuh) has a second one, over their chunks by all CTAs.
+    bool ok;
+    for (int32_t chunks = 0;;) {
+      if (!pull) {
+        const Enum en{(level & 1) ? a.q0 : a.q1, nullptr, n};
+        const EdgeF<UBfsNote, false> f{UBfsNote{a.vd.parent, a.vd.depth, a.g.off, stat, level},
+                                       DIn{IN_ALL, nullptr, nullptr}, DIn{IN_ALL, nullptr, nullptr}, true};
+        if (chunks)
+          lb_hubs(a.g, hub, chunks, f, out, blockIdx.x, gridDim.x);
+        else
+          run_lb<LB>(a.g, en, n, f, out, smem, blockIdx.x, gridDim.x, hub);
+      } else {
+        if (threadIdx.x == 0) ++s_pulls;
+        const int32_t lane = threadIdx.x & 31, sub = lane & 7, gbase = lane & ~7;
+        const uint32_t gmask = 0xFFu << gbase;
+        const int32_t prev = level - 1;
+        for (int32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; v < a.g.V;
+             v += (gridDim.x * blockDim.x) >> 3) {
+          if (__ldcg(a.vd.parent + v) != -1) continue;
+          const int32_t kb = __ldg(d.t.off + v), ke = __ldg(d.t.off + v + 1);
+          const int32_t deg = stat && sub == 0 ? __ldg(a.g.off + v + 1) - __ldg(a.g.off + v) : 0;
+          int32_t hit = -1;
+          for (int32_t k0 = kb; k0 < ke; k0 += 8) {
+            int32_t u = -1;
+            if (k0 + sub < ke) {
+              u = __ldg(d.t.dst + k0 + sub);
+              if (__ldcg(a.vd.depth + u) != prev) u = -1;
+            }
+            const uint32_t bits = (__ballot_sync(gmask, u >= 0) >> gbase) & 0xFFu;
+            if (bits) {
+              hit = __shfl_sync(gmask, u, gbase + __ffs(bits) - 1);
+              break;
+            }
           }
-          const uint32_t bits = (__ballot_sync(gmask, u >= 0) >> gbase) & 0xFFu;
-          if (bits) {
-            hit = __shfl_sync(gmask, u, gbase + __ffs(bits) - 1);
-            break;
+          if (hit >= 0 && sub == 0) {
+            a.vd.parent[v] = hit;
+            a.vd.depth[v] = level;
+            out.sparse(v);
+            if (stat) do_note(stat, (uint32_t)deg);
           }
         }
-        if (hit >= 0 && sub == 0) {
-          a.vd.parent[v] = hit;
-          a.vd.depth[v] = level;
-          out.sparse(v);
-          if (stat) do_note(stat, (uint32_t)deg);
+      }
+      __syncthreads();
+      if (d.stats && threadIdx.x == 0) {
+        if (!chunks) {
+          s_vis[0] = fminf((float)a.g.V, s_vis[0] + s_in[0]);
+          s_vis[1] = fminf((float)a.g.E, s_vis[1] + s_in[1]);
+        }
+        if (s_stat.sum | s_stat.mx) {
+          unsigned long long *nx = d.lstat + 4 * (level % 3);
+          atomicAdd(nx, (unsigned long long)s_stat.sum);
+          atomicAdd(reinterpret_cast<double *>(nx + 1), (double)s_stat.sq);
+          atomicMax(nx + 2, (unsigned long long)s_stat.mx);
+          s_stat.sum = s_stat.mx = 0u;
+          s_stat.sq = 0.f;
         }
       }
+      if (!chunks) clk.tick(a.stop, level, a.err);
+      ok = grid_barrier(a.bar, gridDim.x, a.err, a.timeout_ns);
+      if (!ok || pull || chunks) break;
+      chunks = *(volatile int32_t *)hub.cnt;
+      if (!chunks) break;
     }
-    __syncthreads();
-    if (d.stats && threadIdx.x == 0) {
-      s_vis[0] = fminf((float)a.g.V, s_vis[0] + s_in[0]);
-      s_vis[1] = fminf((float)a.g.E, s_vis[1] + s_in[1]);
-      if (s_stat.sum | s_stat.mx) {
-        unsigned long long *nx = d.lstat + 4 * (level % 3);
-        atomicAdd(nx, (unsigned long long)s_stat.sum);
-        atomicAdd(reinterpret_cast<double *>(nx + 1), (double)s_stat.sq);
-        atomicMax(nx + 2, (unsigned long long)s_stat.mx);
-      }
-    }
-    clk.tick(a.stop, level, a.err);
-    if (!grid_barrier(a.bar, gridDim.x, a.err, a.timeout_ns)) break;
+    if (!ok) break;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     a.stats[0] = level - 1;
@@ -542,6 +587,7 @@ gg_status fused_bfs_do(gg_graph *g, const BfsDoPlan &p, int32_t n0, const VData 
   GG_CHECK_ARG(p.mode != DO_SELECTOR || p.sel, "no selector");
   GG_TRY(ensure_transpose(g));
   const GraphStore *t = g->csc ? g->csc.get() : &g->csr;
+  GG_TRY(ensure_hubs(g));
   void *ls = nullptr;
   GG_TRY(scratch_get_app(g, 7, sizeof(unsigned long long) * 12, &ls));
   GG_TRY(init_counts(g, n0));
@@ -549,7 +595,7 @@ gg_status fused_bfs_do(gg_graph *g, const BfsDoPlan &p, int32_t n0, const VData 
   k_bfs_do_seed<<<1, 256, 0, g->stream>>>(f->q_in, n0, g->csr.off, static_cast<unsigned long long *>(ls));
   GG_CUDA(cudaGetLastError());
   DoKernelArgs ka{};
-  ka.a = make_args(g, f, vd);
+  ka.a = make_args(g, f, vd, s->cta_size);
   ka.d.t = t->view();
   ka.d.t.nbuckets = 0;
   ka.d.lstat = static_cast<unsigned long long *>(ls);
@@ -606,6 +652,9 @@ static BqArgs bq_args(gg_graph *g, gg_frontier *f, const BqBuffers &b, int32_t *
   a.solo_pile_max = 8 * a.solo_max;
   a.fill_target = 1024;
   a.width0 = 16;
+  a.hub_list = static_cast<int32_t *>(g->hubs.p);
+  a.hub_cap = hub_capacity(g);
+  a.hub_min = kHubWidths * cta;
   return a;
 }
 
@@ -614,6 +663,7 @@ gg_status fused_sssp(gg_graph *g, const gg_schedule *s, int32_t n0, int32_t delt
   *ran = false;
   if (!fused_supported(s)) return GG_OK;
   const int cta = s->cta_size;
+  GG_TRY(ensure_hubs(g));
   GG_TRY(bq_start(pq->bq, n0, g->stream));
   BqArgs a = bq_args(g, pq->frontier, pq->bq, vd.dist, delta, cta);
   const size_t sm = lb_smem(s->load_balancing, cta);
@@ -648,7 +698,7 @@ __global__ void k_multi_reset(VData vd, int32_t sssp, int32_t V) {
 }
 
 __global__ void k_multi_seed(VData vd, int32_t sssp, const int32_t *__restrict__ srcs, int32_t n, int32_t *q,
-                             int32_t *cnt3, int32_t *stats, int32_t *gmin2, int32_t *stop) {
+                             int32_t *cnt3, int32_t *stats, int32_t *gmin2, int32_t *stop, int32_t *hub3) {
   for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int32_t s = srcs[i];
     if (sssp) {
@@ -668,6 +718,7 @@ __global__ void k_multi_seed(VData vd, int32_t sssp, const int32_t *__restrict__
     gmin2[0] = INT_MAX;
     gmin2[1] = INT_MAX;
     *stop = 0;
+    for (int i = 0; i < 3; ++i) hub3[i] = 0;
   }
 }
 
@@ -685,9 +736,9 @@ gg_status fused_multi_enqueue(gg_graph *g, cudaStream_t st, bool sssp, const int
     vd.depth = out;
   }
   vd.src = -1;
-  FusedArgs a = make_args(g, f, vd);
-  a.delta = delta;
   const int cta = 512;
+  FusedArgs a = make_args(g, f, vd, cta);
+  a.delta = delta;
   const size_t smem = twce_smem_bytes(cta);
   const void *kernel = sssp ? (const void *)k_sssp_bq<GG_LB_TWCE> : (const void *)k_bfs_fused<GG_LB_TWCE>;
   int per_sm = 0;
@@ -697,7 +748,7 @@ gg_status fused_multi_enqueue(gg_graph *g, cudaStream_t st, bool sssp, const int
   k_multi_reset<<<g->sm_count * 8, 256, 0, st>>>(vd, sssp, g->csr.V);
   note_launch();
   k_multi_seed<<<std::max(1, std::min(ceil_div(n, 256), g->sm_count)), 256, 0, st>>>(
-      vd, sssp, dsrc, n, a.q0, a.cnt3, a.stats, a.gmin2, a.stop);
+      vd, sssp, dsrc, n, a.q0, a.cnt3, a.stats, a.gmin2, a.stop, a.hub3);
   GG_CUDA(cudaMemsetAsync(g->d_bar, 0, sizeof(uint32_t) * 2, st));
   if (sssp) {
     GG_TRY(bq_start(*bq, n, st));

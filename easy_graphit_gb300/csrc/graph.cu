@@ -257,6 +257,16 @@ gg_status ensure_coo(GraphStore &s, cudaStream_t st) {
   return GG_OK;
 }
 
+int32_t hub_capacity(const gg_graph *g) { return g->csr.E / 256 + 4096; }
+
+gg_status ensure_hubs(gg_graph *g) {
+  if (g->hubs.p) return GG_OK;
+  const size_t bytes = sizeof(int32_t) * 3 * (size_t)hub_capacity(g);
+  GG_CUDA(dev_alloc(&g->hubs.p, bytes, g->stream));
+  g->hubs.bytes = bytes;
+  return GG_OK;
+}
+
 static void free_store(GraphStore &s, cudaStream_t st) {
   for (int32_t *p : {s.off, s.dst, s.w, s.src, s.bucket})
     if (p) cudaFreeAsync(p, st);
@@ -485,6 +495,7 @@ gg_status gg_graph_destroy(gg_graph *g) {
   for (auto &s : g->scratch)
     if (s.p) cudaFreeAsync(s.p, st);
   if (g->bq_cta.p) cudaFreeAsync(g->bq_cta.p, st);
+  if (g->hubs.p) cudaFreeAsync(g->hubs.p, st);
   for (void *p : {(void *)g->d_err, (void *)g->d_bar, (void *)g->d_misc})
     if (p) cudaFreeAsync(p, st);
   cudaStreamSynchronize(st);

@@ -39,12 +39,12 @@ struct lb_batch<F, decltype(void(F::kBatch))> {
 
 // Edges [b, e) of source s processed by `width` cooperating threads (rank r).
 // A functor with a batched range relax (push, no per-edge source test beyond
-// the first) takes the whole range at once.
-template <class F>
+// the first) takes the whole range at once, B edges of a thread in flight.
+template <int B = 4, class F>
 __device__ __forceinline__ void do_range(const DGraph &g, const F &f, const DOut &out, int32_t s,
                                          int32_t b, int32_t e, int32_t r, int32_t width) {
   if constexpr (lb_batch<F>::value) {
-    if (b + r < e && f.src_ok(s)) f.relax_range(g, out, s, b, e, r, width);
+    if (b + r < e && f.src_ok(s)) f.template relax_range<B>(g, out, s, b, e, r, width);
     return;
   }
   for (int32_t k = b + r; k < e; k += width) {
@@ -54,6 +54,7 @@ __device__ __forceinline__ void do_range(const DGraph &g, const F &f, const DOut
 }
 
 // ------------------------------------------------------------ VERTEX_BASED
+constexpr int kSerialInFlight = 4;
 // One thread per enumerated vertex, serial neighbour loop with the early exit
 // of operators.cpp:83-94.  Virtual CTA = blockDim.x vertices.
 template <class F>
@@ -62,7 +63,7 @@ __device__ __forceinline__ void lb_vertex(const DGraph &g, const Enum &en, int32
   const int32_t i = vcta * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int32_t s = en.at(i);
-  do_range(g, f, out, s, __ldg(g.off + s), __ldg(g.off + s + 1), 0, 1);
+  do_range<kSerialInFlight>(g, f, out, s, __ldg(g.off + s), __ldg(g.off + s + 1), 0, 1);
 }
 
 // ---------------------------------------------------------------------- WM
@@ -85,6 +86,16 @@ __device__ __forceinline__ void lb_wm(const DGraph &g, const Enum &en, int32_t n
 // a warp part (multiples of 32) and a remainder for the 8-thread group.
 // Warp-bin entries are taken round-robin by the warps, CTA-bin entries by the
 // whole CTA.  Virtual CTA = blockDim.x/8 vertices.
+//
+// Two things keep a skewed frontier from leaving the GPU idle behind one CTA:
+//  * slices: a frontier with fewer virtual CTAs than there are CTAs gives
+//    each virtual CTA `nslices` of them; all bin the same vertices and split
+//    every part of their lists between them;
+//  * hub list: a CTA part of at least hub.min edges (times the slices) goes to
+//    a global list as chunks of kHubChunk CTA widths, which all CTAs drain in a
+//    pass of their own (lb_chunk) -- one R-MAT hub is otherwise 10^2 rounds of
+//    one CTA while the others wait at the level's end.
+// A level-1 frontier of one 180,000-edge hub (R-MAT 22) took 376 us on one CTA.
 struct TwceSmem {
   int32_t nw, nc;
   int32_t data[1];  // 6 * (blockDim/8) ints: warp bin (s,b,e), CTA bin (s,b,e)
@@ -93,11 +104,36 @@ __host__ __device__ inline size_t twce_smem_bytes(int cta) {
   return sizeof(int32_t) * (2 + 6 * (cta / kStage1)) + 16;
 }
 
-template <class F, bool kCtaBin = true>
+constexpr int32_t kHubChunk = 4;   // CTA widths per chunk: one round of a 4-edges-in-flight relax
+constexpr int32_t kHubWidths = 8;  // CTA widths from which a list is split over the CTAs
+
+struct HubList {
+  int32_t *list = nullptr;  // [cap][3]: vertex, first edge, end edge; null: no list
+  int32_t *cnt = nullptr;   // chunks appended; may pass cap, the surplus was not written
+  int32_t cap = 0;
+  int32_t min = 0;          // edges of a CTA part from which it goes to the list
+};
+
+// Appends the chunks of [b, e) of vertex s; false (and no live chunk) when they
+// do not all fit.
+__device__ __forceinline__ bool hub_append(const HubList &hub, int32_t s, int32_t b, int32_t e) {
+  const int32_t chunk = kHubChunk * (int32_t)blockDim.x;
+  const int32_t nch = ceil_div(e - b, chunk);
+  const int32_t p = atomicAdd(hub.cnt, nch);
+  const bool fits = (int64_t)p + nch <= hub.cap;
+  for (int32_t c = 0; c < nch && (int64_t)p + c < hub.cap; ++c) {
+    int32_t *d = hub.list + 3 * (int64_t)(p + c);
+    d[0] = s;
+    d[1] = fits ? b + c * chunk : 0;
+    d[2] = fits ? min(b + (c + 1) * chunk, e) : 0;
+  }
+  return fits;
+}
+
+template <class F>
 __device__ __forceinline__ void lb_twce(const DGraph &g, const Enum &en, int32_t n, const F &f,
-                                        const DOut &out, int32_t vcta, TwceSmem &sm,
-                                        int32_t *chunk_list = nullptr, int32_t *chunk_cnt = nullptr,
-                                        int32_t chunk = 0) {
+                                          const DOut &out, int32_t vcta, int32_t slice, int32_t nslices,
+                                          TwceSmem &sm, const HubList &hub) {
   const int32_t per = blockDim.x / kStage1;
   int32_t *wv = sm.data, *wb = wv + per, *we = wb + per;
   int32_t *cv = we + per, *cb = cv + per, *ce = cb + per;
@@ -105,7 +141,6 @@ __device__ __forceinline__ void lb_twce(const DGraph &g, const Enum &en, int32_t
     sm.nw = 0;
     sm.nc = 0;
   }
-  __syncthreads();
   const int32_t sub = threadIdx.x & (kStage1 - 1);
   const int32_t i = vcta * per + (int32_t)(threadIdx.x / kStage1);
   int32_t s = -1, b = 0, e = 0;
@@ -113,56 +148,92 @@ __device__ __forceinline__ void lb_twce(const DGraph &g, const Enum &en, int32_t
     s = en.at(i);
     b = __ldg(g.off + s);
     e = __ldg(g.off + s + 1);
+  }
+  __syncthreads();
+  if (s >= 0) {
     const int32_t deg = e - b;
     const int32_t big = deg / (int32_t)blockDim.x * (int32_t)blockDim.x;
     const int32_t mid = (deg - big) / 32 * 32;
     if (sub == 0) {
-      if (big) {
-        if (kCtaBin) {
+      const bool is_hub = hub.list && big >= hub.min * (int64_t)nslices;
+      if (big && !(is_hub && slice != 0)) {
+        bool listed = false, alone = false;  // alone: one slice takes it all
+        if (is_hub) {
+          listed = hub_append(hub, s, b, b + big);
+          alone = !listed;
+        }
+        if (!listed) {
           const int32_t p = atomicAdd(&sm.nc, 1);
           cv[p] = s;
           cb[p] = b;
-          ce[p] = b + big;
-        } else {
-          // ETWC: hub edges become fixed-size chunks on a global list that all
-          // CTAs drain afterwards.
-          const int32_t nch = ceil_div(big, chunk);
-          const int32_t p = atomicAdd(chunk_cnt, nch);
-          for (int32_t c = 0; c < nch; ++c) {
-            chunk_list[3 * (p + c) + 0] = s;
-            chunk_list[3 * (p + c) + 1] = b + c * chunk;
-            chunk_list[3 * (p + c) + 2] = min(b + (c + 1) * chunk, b + big);
-          }
+          ce[p] = alone ? ~(b + big) : b + big;
         }
       }
       if (mid) {
-        const int32_t p = atomicAdd(&sm.nw, 1);
-        wv[p] = s;
-        wb[p] = b + big;
-        we[p] = b + big + mid;
+        // pieces of 32 edges, a run of them for each of the first slices counted
+        // from slice i (bins differ in order between slices, vertices do not)
+        const int32_t pieces = (mid + 31) >> 5, ways = min(nslices, pieces);
+        int32_t t = slice - i % nslices;
+        if (t < 0) t += nslices;
+        if (t < ways) {
+          const int32_t p = atomicAdd(&sm.nw, 1);
+          wv[p] = s;
+          wb[p] = b + big + pieces * t / ways * 32;
+          we[p] = min(b + big + pieces * (t + 1) / ways * 32, b + big + mid);
+        }
       }
     }
     b += big + mid;
   }
   __syncthreads();
-  if (s >= 0) do_range(g, f, out, s, b, e, sub, kStage1);  // stage 1
-  const int32_t nw = sm.nw;
-  for (int32_t j = (int32_t)(threadIdx.x >> 5); j < nw; j += (int32_t)(blockDim.x >> 5))  // stage 2
+  {  // stage 1: the remainders, 8 edges to each of the first slices
+    const int32_t ways = min(nslices, 32 / kStage1);
+    if (s >= 0 && slice < ways) do_range(g, f, out, s, b, e, slice * kStage1 + sub, kStage1 * ways);
+  }
+  const int32_t nw = sm.nw, warps = (int32_t)(blockDim.x >> 5);
+  for (int32_t j = (int32_t)(threadIdx.x >> 5); j < nw; j += warps)  // stage 2
     do_range(g, f, out, wv[j], wb[j], we[j], threadIdx.x & 31, 32);
-  if (kCtaBin) {
-    const int32_t nc = sm.nc;
-    for (int32_t j = 0; j < nc; ++j)  // stage 3
-      do_range(g, f, out, cv[j], cb[j], ce[j], threadIdx.x, blockDim.x);
+  const int32_t nc = sm.nc;
+  for (int32_t j = 0; j < nc; ++j) {  // stage 3
+    const int32_t end = ce[j];
+    if (end < 0)
+      do_range(g, f, out, cv[j], cb[j], ~end, threadIdx.x, blockDim.x);
+    else
+      do_range(g, f, out, cv[j], cb[j], end, slice * (int32_t)blockDim.x + threadIdx.x,
+               nslices * (int32_t)blockDim.x);
   }
   __syncthreads();
 }
 
-// ETWC second phase: a virtual CTA processes one hub chunk.
+// TWCE over n vertices by CTA `rank` of `nparts`: whole
+// virtual CTAs in turn, or slices of them when there are fewer than CTAs.
+template <class F>
+__device__ __forceinline__ void lb_twce_all(const DGraph &g, const Enum &en, int32_t n, const F &f,
+                                          const DOut &out, int32_t rank, int32_t nparts, TwceSmem &sm,
+                                          const HubList &hub) {
+  const int32_t nv = ceil_div(n, blockDim.x / kStage1);
+  if (nv >= nparts) {
+    for (int32_t v = rank; v < nv; v += nparts) lb_twce(g, en, n, f, out, v, 0, 1, sm, hub);
+  } else if (nv > 0) {
+    const int32_t slices = nparts / nv;
+    if (rank < nv * slices) lb_twce(g, en, n, f, out, rank % nv, rank / nv, slices, sm, hub);
+  }
+}
+
+// A virtual CTA processes one chunk of a hub list.
 template <class F>
 __device__ __forceinline__ void lb_chunk(const DGraph &g, const int32_t *chunk_list, const F &f,
                                          const DOut &out, int32_t vcta) {
-  const int32_t s = chunk_list[3 * vcta], b = chunk_list[3 * vcta + 1], e = chunk_list[3 * vcta + 2];
+  const int32_t *d = chunk_list + 3 * (int64_t)vcta;
+  const int32_t s = __ldcg(d), b = __ldcg(d + 1), e = __ldcg(d + 2);
   do_range(g, f, out, s, b, e, threadIdx.x, blockDim.x);
+}
+
+// CTA `rank` of `nparts` drains its share of a hub list of `chunks` entries.
+template <class F>
+__device__ __forceinline__ void lb_hubs(const DGraph &g, const HubList &hub, int32_t chunks, const F &f,
+                                        const DOut &out, int32_t rank, int32_t nparts) {
+  for (int32_t c = rank; c < min(chunks, hub.cap); c += nparts) lb_chunk(g, hub.list, f, out, c);
 }
 
 // ---------------------------------------------------------------------- CM

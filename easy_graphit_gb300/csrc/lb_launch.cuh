@@ -34,21 +34,17 @@ __global__ void __launch_bounds__(1024) k_cta(DGraph g, Enum en, F f, DOut out) 
   }
 }
 
-template <class F, bool kCtaBin>
-__global__ void __launch_bounds__(1024)
-    k_twce(DGraph g, Enum en, F f, DOut out, int32_t *chunks, int32_t *chunk_cnt, int32_t chunk) {
+// TWCE, and with a hub list that takes every CTA part ETWC.
+template <class F>
+__global__ void __launch_bounds__(1024) k_twce(DGraph g, Enum en, F f, DOut out, HubList hub) {
   extern __shared__ int4 smem_raw[];
-  TwceSmem &sm = *reinterpret_cast<TwceSmem *>(smem_raw);
-  const int32_t n = en.count();
-  const int32_t nv = ceil_div(n, blockDim.x / kStage1);
-  for (int32_t v = blockIdx.x; v < nv; v += gridDim.x)
-    lb_twce<F, kCtaBin>(g, en, n, f, out, v, sm, chunks, chunk_cnt, chunk);
+  lb_twce_all(g, en, en.count(), f, out, blockIdx.x, gridDim.x, *reinterpret_cast<TwceSmem *>(smem_raw), hub);
 }
 
 template <class F>
 __global__ void __launch_bounds__(1024)
-    k_chunks(DGraph g, const int32_t *chunks, const int32_t *chunk_cnt, F f, DOut out) {
-  const int32_t n = *(volatile const int32_t *)chunk_cnt;
+    k_chunks(DGraph g, const int32_t *chunks, const int32_t *chunk_cnt, int32_t cap, F f, DOut out) {
+  const int32_t n = min(*(volatile const int32_t *)chunk_cnt, cap);
   for (int32_t v = blockIdx.x; v < n; v += gridDim.x) lb_chunk(g, chunks, f, out, v);
 }
 
@@ -95,6 +91,24 @@ inline int grid_for(K kernel, int cta, size_t smem, int sm_count, int64_t nvcta)
   return (int)std::max<int64_t>(1, std::min<int64_t>(nvcta, res));
 }
 
+// Grid of a TWCE launch: the resident CTAs, or up to kTwceWaves times as many
+// slices when the frontier is small (a slice without work ends after one read
+// of its vertices, so hubs are split finely even where every CTA has some).
+constexpr int kTwceWaves = 4;
+template <class F>
+void launch_twce(const EdgeLaunch &L, const F &f, const HubList &hub) {
+  auto k = k_twce<F>;
+  const size_t sm = twce_smem_bytes(L.cta);
+  const int res = resident_grid((const void *)k, L.cta, sm, L.graph->sm_count);
+  int grid = res;
+  if (L.n_host >= 0) {
+    const int64_t nv = ceil_div(L.n_host, L.cta / kStage1);
+    if (nv < (int64_t)kTwceWaves * res) grid = (int)(nv * std::max<int64_t>(1, kTwceWaves * (int64_t)res / nv));
+  }
+  note_launch();
+  k<<<grid, L.cta, sm, L.graph->stream>>>(L.g, L.en, f, L.out, hub);
+}
+
 template <class F>
 gg_status launch_lb(const EdgeLaunch &L, const F &f) {
   gg_graph *G = L.graph;
@@ -126,25 +140,24 @@ gg_status launch_lb(const EdgeLaunch &L, const F &f) {
       break;
     }
     case GG_LB_TWCE: {
-      auto k = k_twce<F, true>;
-      const size_t sm = twce_smem_bytes(cta);
-      { gg::note_launch(); k<<<grid_for(k, cta, sm, sms, n < 0 ? -1 : ceil_div(n, cta / kStage1)), cta, sm, st>>>(
-          L.g, L.en, f, L.out, nullptr, nullptr, 0); }
+      launch_twce(L, f, HubList{});
       break;
     }
     case GG_LB_ETWC: {
       // Stage 1+2 in-CTA, hub edges as chunks of 4*cta edges on a global list.
-      const int32_t chunk = 4 * cta;
+      const int32_t chunk = kHubChunk * cta;
       int32_t *chunks = nullptr, *cnt = nullptr;
       const int64_t maxc = (int64_t)L.g.E / chunk + (n < 0 ? L.g.V : n) + 1;
       GG_TRY(etwc_scratch(G, maxc, &chunks, &cnt));
       GG_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t), st));
-      auto k = k_twce<F, false>;
-      const size_t sm = twce_smem_bytes(cta);
-      { gg::note_launch(); k<<<grid_for(k, cta, sm, sms, n < 0 ? -1 : ceil_div(n, cta / kStage1)), cta, sm, st>>>(
-          L.g, L.en, f, L.out, chunks, cnt, chunk); }
+      HubList hub;
+      hub.list = chunks;
+      hub.cnt = cnt;
+      hub.cap = (int32_t)maxc;
+      hub.min = 0;
+      launch_twce(L, f, hub);
       auto k2 = k_chunks<F>;
-      { gg::note_launch(); k2<<<grid_for(k2, cta, 0, sms, -1), cta, 0, st>>>(L.g, chunks, cnt, f, L.out); }
+      { gg::note_launch(); k2<<<grid_for(k2, cta, 0, sms, -1), cta, 0, st>>>(L.g, chunks, cnt, (int32_t)maxc, f, L.out); }
       break;
     }
     case GG_LB_CM: {

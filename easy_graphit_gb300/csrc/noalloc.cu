@@ -96,9 +96,7 @@ __global__ void __launch_bounds__(512) k_noalloc_bfs(DGraph g, int32_t *scratch,
     out.cnt = cnt3 + level % 3;
     out.cap = kNoAllocMaxVertices;  // each vertex is enqueued once (CAS)
     out.err = err;
-    const int32_t nv = ceil_div(n, blockDim.x / kStage1);
-    for (int32_t v = blockIdx.x; v < nv; v += gridDim.x)
-      lb_twce<UDepth, true>(g, en, n, f, out, v, *reinterpret_cast<TwceSmem *>(smem));
+    lb_twce_all(g, en, n, f, out, blockIdx.x, gridDim.x, *reinterpret_cast<TwceSmem *>(smem), HubList{});
     if (!grid_barrier(bar, gridDim.x, err, timeout_ns)) break;
     in ^= 1;
   }

@@ -36,7 +36,6 @@ struct UBfs {
 struct USssp {
   static constexpr bool kWeight = true;
   static constexpr bool kBatch = true;  // push relax over a range: relax_range
-  static constexpr int kEdgesInFlight = 4;
   int32_t *dist;
   int32_t cutoff;
   DFar far;
@@ -50,19 +49,18 @@ struct USssp {
     if (far.stamp) far.park(d, np);
     return false;
   }
-  // Edges k = b + r, b + r + width, ... of source s, kEdgesInFlight at a time:
+  // Edges k = b + r, b + r + width, ... of source s, B at a time:
   // their targets and weights, then the targets' distances, then the
   // atomicMins of the improving ones are each issued together, so one thread
   // keeps that many edges in flight instead of one (a hub's list on a thread
   // of VERTEX_BASED is otherwise a chain of dependent round trips).  Same
   // outcome as apply() per edge: an improvement below the cutoff queues the
   // target, one above it parks it.
-  template <class G, class Out>
+  template <int B, class G, class Out>
   __device__ __forceinline__ void relax_range(const G &g, const Out &out, int32_t s, int32_t b, int32_t e,
                                               int32_t r, int32_t width) const {
     const int32_t ds = vload(dist + s);
     if (ds == INT_MAX) return;
-    constexpr int B = kEdgesInFlight;
     for (int32_t k0 = b + r; k0 < e; k0 += B * width) {
       int32_t d[B], np[B], prev[B];
 #pragma unroll
@@ -192,10 +190,10 @@ struct EdgeF {
     return u.apply(s, d, w) ? d : -1;
   }
   // Only used when kBatch; the source filter (in_src) is checked by the caller.
-  template <class G, class Out>
+  template <int B, class G, class Out>
   __device__ __forceinline__ void relax_range(const G &g, const Out &out, int32_t s, int32_t b, int32_t e,
                                               int32_t r, int32_t width) const {
-    if constexpr (kBatch) u.relax_range(g, out, s, b, e, r, width);
+    if constexpr (kBatch) u.template relax_range<B>(g, out, s, b, e, r, width);
   }
 };
 
