@@ -159,6 +159,9 @@ __device__ __forceinline__ bool bc_take(int32_t *wc, int32_t ni, int32_t nwarps,
 
 __global__ void __launch_bounds__(512) k_bc_batch(DGraph g, BcState st) {
   extern __shared__ int4 smem[];
+  __shared__ Stage stage;
+  if (threadIdx.x == 0) stage.n = 0;
+  __syncthreads();
   const int32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int32_t nthreads = gridDim.x * blockDim.x;
   const int32_t lane = threadIdx.x & 31;
@@ -237,11 +240,14 @@ __global__ void __launch_bounds__(512) k_bc_batch(DGraph g, BcState st) {
       out.cnt = st.ctr + 0;
       out.cap = st.levcap;
       out.err = st.err;
+      out.stage = &stage;
       lb_twce_all(g, en, n, f, out, blockIdx.x, gridDim.x, *reinterpret_cast<TwceSmem *>(smem), hub);
+      stage_flush(out);
       alive = grid_barrier(st.bar, gridDim.x, st.err, st.timeout_ns);
       const int32_t chunks = *(volatile int32_t *)hub.cnt;
       if (alive && chunks > 0) {  // the hubs the level set aside, by all CTAs
         lb_hubs(g, hub, chunks, f, out, blockIdx.x, gridDim.x);
+        stage_flush(out);
         alive = grid_barrier(st.bar, gridDim.x, st.err, st.timeout_ns);
       }
     }

@@ -46,19 +46,45 @@ __device__ __forceinline__ void ms_depths(const MsBfsState &st, int32_t v, uint6
   }
 }
 
-// Adds the out-degree of v, entering the next level's queue, to the CTA's
-// statistics of that frontier.
-__device__ __forceinline__ void ms_note(const MsBfsState &st, unsigned long long *s_stat, int32_t v) {
-  const unsigned long long d = (unsigned long long)(__ldg(st.off + v + 1) - __ldg(st.off + v));
-  atomicAdd(s_stat, d);
-  atomicAdd(s_stat + 1, d * d);
-  atomicMax(s_stat + 2, d);
+// A thread's share of what a level adds to the next one's frontier: the sources
+// found and the out-degree statistics.  Kept in registers and folded into the
+// CTA's at the end of the level -- 64-bit shared-memory atomics per vertex (CAS
+// loops, all on the same words) serialised a CTA that found thousands.
+struct MsAcc {
+  unsigned long long act, sum, sq, mx;
+  __device__ __forceinline__ void note(const MsBfsState &st, int32_t v, uint64_t nb) {
+    const unsigned long long d = (unsigned long long)(__ldg(st.off + v + 1) - __ldg(st.off + v));
+    act |= nb;
+    sum += d;
+    sq += d * d;
+    mx = mx > d ? mx : d;
+  }
+};
+__device__ __forceinline__ void ms_fold(const MsAcc &t, unsigned long long *s_act, unsigned long long *s_stat) {
+  if (!__any_sync(0xffffffffu, t.act != 0ull)) return;
+  unsigned long long act = t.act, sum = t.sum, sq = t.sq, mx = t.mx;
+#pragma unroll
+  for (int i = 16; i > 0; i >>= 1) {
+    act |= __shfl_xor_sync(0xffffffffu, act, i);
+    sum += __shfl_xor_sync(0xffffffffu, sum, i);
+    sq += __shfl_xor_sync(0xffffffffu, sq, i);
+    const unsigned long long o = __shfl_xor_sync(0xffffffffu, mx, i);
+    mx = mx > o ? mx : o;
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicOr(s_act, act);
+    atomicAdd(s_stat, sum);
+    atomicAdd(s_stat + 1, sq);
+    atomicMax(s_stat + 2, mx);
+  }
 }
 
 __global__ void __launch_bounds__(512) k_msbfs(DGraph g, MsBfsState st) {
   extern __shared__ int4 smem[];
   __shared__ unsigned long long s_act;
   __shared__ unsigned long long s_stat[3];
+  __shared__ Stage stage;
+  if (threadIdx.x == 0) stage.n = 0;  // the first level's barrier comes before any append
   const int32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int32_t nthreads = gridDim.x * blockDim.x;
   const int32_t lane = threadIdx.x & 31;
@@ -120,6 +146,8 @@ __global__ void __launch_bounds__(512) k_msbfs(DGraph g, MsBfsState st) {
     out.cnt = st.cnt4 + ((L + 1) & 3);
     out.cap = st.V;  // qstamp admits each vertex once per level
     out.err = st.err;
+    out.stage = &stage;
+    MsAcc acc{0ull, 0ull, 0ull, 0ull};
     if (!bu) {
       const Enum en{ms_q(st, L), nullptr, n};
       lb_twce_all(g, en, n, f, out, blockIdx.x, gridDim.x, *reinterpret_cast<TwceSmem *>(smem), hub);
@@ -148,23 +176,20 @@ __global__ void __launch_bounds__(512) k_msbfs(DGraph g, MsBfsState st) {
           if (sub == 0) {
             st.seen[v] = sv | found;
             frn[v] = found;
-            const int32_t pos = atomicAdd(st.cnt4 + ((L + 1) & 3), 1);
-            if (pos < st.V)
-              qn[pos] = v;
-            else
-              atomicOr(st.err, DEV_ERR_OVERFLOW);
-            atomicOr(&s_act, (unsigned long long)found);
-            ms_note(st, s_stat, v);
+            out.sparse(v);
+            acc.note(st, v, found);
           }
           ms_depths(st, v, found, L + 1, sub, 8);
         }
       }
     }
+    stage_flush(out);
     if (!grid_barrier(st.bar, gridDim.x, st.err, st.timeout_ns)) break;
     if (!bu) {  // the hubs the level set aside, by all CTAs
       const int32_t chunks = *(volatile int32_t *)hub.cnt;
       if (chunks > 0) {
         lb_hubs(g, hub, chunks, f, out, blockIdx.x, gridDim.x);
+        stage_flush(out);
         if (!grid_barrier(st.bar, gridDim.x, st.err, st.timeout_ns)) break;
       }
     }
@@ -179,8 +204,7 @@ __global__ void __launch_bounds__(512) k_msbfs(DGraph g, MsBfsState st) {
         st.seen[v] = sv | nb;
         frn[v] = nb;
         st.acc[v] = 0;
-        atomicOr(&s_act, (unsigned long long)nb);
-        ms_note(st, s_stat, v);
+        acc.note(st, v, nb);
         ms_depths(st, v, nb, L + 1, 0, 1);
       }
     }
@@ -191,6 +215,7 @@ __global__ void __launch_bounds__(512) k_msbfs(DGraph g, MsBfsState st) {
       const int32_t m = min(*(volatile int32_t *)(st.cnt4 + ((L - 1) & 3)), st.V);
       for (int32_t i = tid; i < m; i += nthreads) old[__ldcg(qo + i)] = 0ull;
     }
+    ms_fold(acc, &s_act, s_stat);
     __syncthreads();
     if (threadIdx.x == 0) {
       if (s_act) atomicOr(st.actm + (L + 1) % 3, s_act);

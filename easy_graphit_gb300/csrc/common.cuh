@@ -86,6 +86,17 @@ __device__ __forceinline__ bool cas(int32_t *p, int32_t expect, int32_t v) {
   return atomicCAS(p, expect, v) == expect;
 }
 
+// A CTA's appends to a sparse queue, staged in shared memory and sent with one
+// reservation (stage_flush).  A queue has one count for the whole GPU: a level
+// that finds 10^6 vertices in groups of two to four lanes makes 10^5 atomics on
+// that one word, which the L2 takes one after another.  Appends past kStageCap
+// go to the queue directly.
+constexpr int32_t kStageCap = 1024;
+struct Stage {
+  int32_t n, base;
+  int32_t buf[kStageCap];
+};
+
 // Output frontier writer: the enqueue_* family of gpu_intrinsics.h:95-110.
 enum : int32_t {
   OUT_NONE = 0,
@@ -104,8 +115,16 @@ struct DOut {
   int32_t *dedup;
   int32_t epoch;
   int32_t *err;
+  Stage *stage;  // shared memory, or null: append directly
 
   __device__ __forceinline__ void sparse(int32_t v) const {
+    if (stage) {
+      const int32_t at = agg_inc(&stage->n);
+      if (at < kStageCap) {
+        stage->buf[at] = v;
+        return;
+      }
+    }
     const int32_t pos = agg_inc(cnt);
     if (pos < cap)
       q[pos] = v;
@@ -141,6 +160,27 @@ struct DOut {
     }
   }
 };
+
+// Sends what a CTA staged for `out` and empties the stage; the whole CTA calls
+// it.  Appends after it need a barrier first (every caller ends its step at one).
+__device__ __forceinline__ void stage_flush(Stage *st, int32_t *q, int32_t *cnt, int64_t cap, int32_t *err) {
+  __syncthreads();
+  const int32_t n = min(st->n, kStageCap);
+  if (n == 0) return;
+  if (threadIdx.x == 0) st->base = atomicAdd(cnt, n);
+  __syncthreads();
+  const int32_t base = st->base;
+  for (int32_t i = threadIdx.x; i < n; i += blockDim.x) {
+    if (base + i < cap)
+      q[base + i] = st->buf[i];
+    else
+      atomicOr(err, DEV_ERR_OVERFLOW);
+  }
+  if (threadIdx.x == 0) st->n = 0;
+}
+__device__ __forceinline__ void stage_flush(const DOut &out) {
+  stage_flush(out.stage, out.q, out.cnt, out.cap, out.err);
+}
 
 // Far piles of the single-source delta-stepping queue (bucket_queue.cuh).  A
 // relaxation that lowers P[v] to p at or above the window's cutoff parks v on
