@@ -31,6 +31,7 @@
 namespace gg {
 
 constexpr int32_t kBcWidth = 64;         // sources per pass (mask bits)
+constexpr int32_t kBcLight = 128;        // longest list that is one light work item
 constexpr int32_t kBcMaxLevels = 65534;  // depth is stored as uint16; 0xFFFF = unreached
 
 struct BcState {
@@ -45,7 +46,8 @@ struct BcState {
   int32_t wcap;
   int32_t chunk;                 // in-edges per work item (the graph's batch tuning)
   int32_t *ctr;                  // [0] level-list end, [1..2] forward items, [3..4] backward items,
-                                 // [16..19] hand-out counters, [20] end of Q_0
+                                 // [16..19] hand-out counters, [20] end of Q_0, [21..23] hub chunks;
+                                 // [24..27] long items and [28..31] their hand-out, as [1..4], [16..19]
   uint16_t *depth;               // [V][64]
   double *sigma, *dep;           // [V][64]
   const int32_t *toff, *tsrc;    // in-neighbours (the CSR itself for a symmetric graph)
@@ -61,10 +63,29 @@ struct BcState {
   uint64_t loop_limit_ns;
 };
 
-// Appends nch work items for this lane's vertex; the whole warp calls it
-// together (lanes without a vertex pass nch = 0).
-__device__ __forceinline__ void bc_push_items(const BcState &st, int32_t *wcnt, int32_t v, int32_t nch) {
+// Appends the work items of this lane's vertex (degree deg, -1 for a lane
+// without one); the whole warp calls it together.  Lists up to kBcLight edges
+// are one item at the front of the work array (count wcnt), longer ones items of
+// st.chunk edges from its back (count hcnt): the two are handed out differently.
+__device__ __forceinline__ void bc_push_items(const BcState &st, int32_t *wcnt, int32_t *hcnt, int32_t v,
+                                              int32_t deg) {
   const int32_t lane = threadIdx.x & 31;
+  const bool light = deg >= 0 && deg <= kBcLight;
+  const uint32_t lights = __ballot_sync(0xffffffffu, light);
+  if (lights) {
+    int32_t base = 0;
+    if (lane == __ffs(lights) - 1) base = atomicAdd(wcnt, __popc(lights));
+    base = __shfl_sync(0xffffffffu, base, __ffs(lights) - 1);
+    const int32_t at = base + __popc(lights & ((1u << lane) - 1));
+    if (light) {
+      if (at < st.wcap)
+        st.work[at] = (int64_t)v << 32;
+      else
+        atomicOr(st.err, DEV_ERR_OVERFLOW);
+    }
+  }
+  const int32_t nch = deg > kBcLight ? (deg + st.chunk - 1) / st.chunk : 0;
+  if (!__any_sync(0xffffffffu, nch > 0)) return;
   int32_t incl = nch;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
@@ -72,9 +93,8 @@ __device__ __forceinline__ void bc_push_items(const BcState &st, int32_t *wcnt, 
     if (lane >= d) incl += t;
   }
   const int32_t total = __shfl_sync(0xffffffffu, incl, 31);
-  if (total == 0) return;
   int32_t base = 0;
-  if (lane == 31) base = atomicAdd(wcnt, total);
+  if (lane == 31) base = atomicAdd(hcnt, total);
   base = __shfl_sync(0xffffffffu, base, 31);
   const int32_t first = base + incl - nch;
   for (int32_t c = 0; c < nch; ++c) {
@@ -82,7 +102,7 @@ __device__ __forceinline__ void bc_push_items(const BcState &st, int32_t *wcnt, 
       atomicOr(st.err, DEV_ERR_OVERFLOW);
       break;
     }
-    st.work[first + c] = ((int64_t)v << 32) | (uint32_t)c;
+    st.work[st.wcap - 1 - (first + c)] = ((int64_t)v << 32) | (uint32_t)c;
   }
 }
 
@@ -96,65 +116,117 @@ __device__ __forceinline__ uint64_t *bc_lm(const BcState &st, int32_t level) {
   return (level & 1) ? st.lm[1] : st.lm[0];
 }
 
-__device__ __forceinline__ int32_t bc_chunks(const BcState &st, int32_t v) {
-  const int32_t deg = __ldg(st.toff + v + 1) - __ldg(st.toff + v);
-  return deg <= st.chunk ? 1 : (deg + st.chunk - 1) / st.chunk;
+__device__ __forceinline__ int32_t bc_degree(const BcState &st, int32_t v) {
+  return __ldg(st.toff + v + 1) - __ldg(st.toff + v);
 }
 
 // Gather over one work item: lane sums, for its sources s in `own`, val[u][s]
-// over in-neighbours u whose mask has s.  Returns the two partial sums.
-__device__ __forceinline__ void bc_gather(const BcState &st, int32_t v, int32_t c, uint64_t own,
+// over in-neighbours u whose mask has s, in list order.  Returns the two
+// partial sums.  A warp reads 32 neighbours and their masks at once, a lane
+// each, and then only the rows of those whose mask survives, four in flight:
+// an item is bound by the round trips in a row, and reading neighbours, masks
+// and rows four at a time took eight times as many.
+__device__ __forceinline__ void bc_gather(const BcState &st, int32_t k0, int32_t k1, uint64_t own,
                                           const uint64_t *mask, const double *val, double &a0,
                                           double &a1) {
   const int32_t lane = threadIdx.x & 31;
-  const int32_t kb = __ldg(st.toff + v), ke = __ldg(st.toff + v + 1);
-  const int32_t k0 = kb + c * st.chunk, k1 = min(ke, k0 + st.chunk);
   a0 = 0.0;
   a1 = 0.0;
-  int32_t k = k0;
-  for (; k + 4 <= k1; k += 4) {
-    int32_t u[4];
-    uint64_t m[4];
+  int32_t u = k0 + lane < k1 ? __ldg(st.tsrc + k0 + lane) : -1;
+  for (int32_t k = k0; k < k1; k += 32) {
+    const int32_t next = k + 32 + lane < k1 ? __ldg(st.tsrc + k + 32 + lane) : -1;
+    const uint64_t m = u >= 0 ? __ldcg(mask + u) & own : 0ull;
+    uint32_t live = __ballot_sync(0xffffffffu, m != 0ull);
+    while (live) {
+      double x[4], y[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) u[j] = __ldg(st.tsrc + k + j);
+      for (int j = 0; j < 4; ++j) {
+        x[j] = y[j] = 0.0;
+        if (!live) continue;
+        const int32_t l = __ffs(live) - 1;
+        live &= live - 1;
+        const double *row = val + (int64_t)__shfl_sync(0xffffffffu, u, l) * kBcWidth;
+        const uint64_t ml = __shfl_sync(0xffffffffu, m, l);
+        if ((ml >> lane) & 1) x[j] = __ldcg(row + lane);
+        if ((ml >> (lane + 32)) & 1) y[j] = __ldcg(row + lane + 32);
+      }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) m[j] = __ldcg(mask + u[j]) & own;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (!m[j]) continue;
-      const double *row = val + (int64_t)u[j] * kBcWidth;
-      if ((m[j] >> lane) & 1) a0 += __ldcg(row + lane);
-      if ((m[j] >> (lane + 32)) & 1) a1 += __ldcg(row + lane + 32);
+      for (int j = 0; j < 4; ++j) {
+        a0 += x[j];
+        a1 += y[j];
+      }
     }
-  }
-  for (; k < k1; ++k) {
-    const int32_t u = __ldg(st.tsrc + k);
-    const uint64_t m = __ldcg(mask + u) & own;
-    if (!m) continue;
-    const double *row = val + (int64_t)u * kBcWidth;
-    if ((m >> lane) & 1) a0 += __ldcg(row + lane);
-    if ((m >> (lane + 32)) & 1) a1 += __ldcg(row + lane + 32);
+    u = next;
   }
 }
 
-// Guided hand-out of a phase's work items: a warp takes a batch of up to 32
-// (half of what is left, spread over the warps), so items of very different
-// cost still end the phase together instead of leaving CTAs idle at the grid
-// barrier.  False when none are left; [i0, i1) is the batch.
-__device__ __forceinline__ bool bc_take(int32_t *wc, int32_t ni, int32_t nwarps, int32_t &i0, int32_t &i1) {
+// Hand-out of a phase's work items to warps: the long ones first, one at a
+// time, then the light ones in batches of up to 8 (half of what is left, spread
+// over the warps), so that warps end the phase together.  With hub chunks and
+// short lists in one list and batches of 32, a warp that drew a hub's
+// neighbouring chunks worked for 3 ms while the rest of the GPU waited 2.2 ms
+// of it at the barrier (0.5 M vertices, degree 30).
+struct BcItems {
+  const int32_t *cnt, *hcnt;  // items: light, long
+  int32_t *wc, *hwc;          // hand-out counters
+};
+// False when none are left; items are work[i] for i in [i0, i1).
+__device__ __forceinline__ bool bc_take(const BcState &st, const BcItems &w, int32_t n_light, int32_t n_long,
+                                        int32_t nwarps, bool &longs, int32_t &i0, int32_t &i1) {
   const int32_t lane = threadIdx.x & 31;
   int32_t b = 0, B = 1;
+  if (longs) {
+    if (lane == 0) b = atomicAdd(w.hwc, 1);
+    b = __shfl_sync(0xffffffffu, b, 0);
+    if (b < n_long) {
+      i0 = st.wcap - 1 - b;
+      i1 = i0 + 1;
+      return true;
+    }
+    longs = false;
+  }
   if (lane == 0) {
-    const int32_t left = ni - *(volatile int32_t *)wc;
+    const int32_t left = n_light - *(volatile int32_t *)w.wc;
     const int32_t per = left > 0 ? (left / 2 + nwarps - 1) / nwarps : 1;
-    B = per < 1 ? 1 : (per > 32 ? 32 : per);
-    b = atomicAdd(wc, B);
+    B = per < 1 ? 1 : (per > 8 ? 8 : per);
+    b = atomicAdd(w.wc, B);
   }
   b = __shfl_sync(0xffffffffu, b, 0);
   B = __shfl_sync(0xffffffffu, B, 0);
   i0 = b;
-  i1 = min(b + B, ni);
-  return b < ni;
+  i1 = min(b + B, n_light);
+  return b < n_light;
+}
+
+// f(v, chunk, first in-edge, end in-edge, whole list in one item) over a
+// phase's items, a warp each.
+template <class Fn>
+__device__ __forceinline__ void bc_each_item(const BcState &st, const BcItems &w, int32_t nwarps, const Fn &f) {
+  const int32_t n_light = min(*(const volatile int32_t *)w.cnt, st.wcap);
+  const int32_t n_long = min(*(const volatile int32_t *)w.hcnt, st.wcap);
+  bool longs = n_long > 0;
+  for (int32_t i0, i1; bc_take(st, w, n_light, n_long, nwarps, longs, i0, i1);)
+    for (int32_t i = i0; i < i1; ++i) {
+      const int64_t it = __ldcg(st.work + i);
+      const int32_t v = (int32_t)(it >> 32), c = (int32_t)(uint32_t)it;
+      const int32_t kb = __ldg(st.toff + v), ke = __ldg(st.toff + v + 1);
+      if (ke - kb <= kBcLight)
+        f(v, 0, kb, ke, true);
+      else
+        f(v, c, kb + c * st.chunk, min(ke, kb + (c + 1) * st.chunk), ke - kb <= st.chunk);
+    }
+}
+
+// Items and hand-out counters of the gathers: forward, those of Q_{d+1} made by
+// iteration d; backward, those of level dd.  Two of each by parity: a level's
+// counts are cleared while the other's are in use.
+__device__ __forceinline__ BcItems bc_forward_items(const BcState &st, int32_t d) {
+  const int32_t i = d & 1;
+  return BcItems{st.ctr + 1 + i, st.ctr + 24 + i, st.ctr + 16 + (1 - i), st.ctr + 28 + (1 - i)};
+}
+__device__ __forceinline__ BcItems bc_backward_items(const BcState &st, int32_t dd) {
+  const int32_t i = dd & 1;
+  return BcItems{st.ctr + 3 + i, st.ctr + 26 + i, st.ctr + 18 + i, st.ctr + 30 + i};
 }
 
 __global__ void __launch_bounds__(512) k_bc_batch(DGraph g, BcState st) {
@@ -196,23 +268,19 @@ __global__ void __launch_bounds__(512) k_bc_batch(DGraph g, BcState st) {
     if (tid == 0) {
       st.loff[d] = b_d;
       st.loff[d + 1] = e_d;
-      st.ctr[1 + (d & 1)] = 0;  // items of Q_{d+1}, filled by the publish below
-      st.ctr[16 + ((d + 1) & 1)] = 0;  // hand-out counter of the next level's gather
+      st.ctr[1 + (d & 1)] = st.ctr[24 + (d & 1)] = 0;  // items of Q_{d+1}, filled by the publish below
+      st.ctr[16 + ((d + 1) & 1)] = st.ctr[28 + ((d + 1) & 1)] = 0;  // hand-out of the next level's gather
       st.ctr[21 + (d + 1) % 3] = 0;    // hub chunks of the next level's relax
     }
     // sigma of Q_d from Q_{d-1} (items made by the previous publish)
     if (d > 0) {
-      const int32_t ni = min(*(volatile int32_t *)(st.ctr + 1 + ((d - 1) & 1)), st.wcap);
       const uint64_t *pm = bc_fr(st, d - 1), *nm = bc_fr(st, d);
-      for (int32_t i0, i1; bc_take(st.ctr + 16 + (d & 1), ni, nwarps, i0, i1);)
-      for (int32_t i = i0; i < i1; ++i) {
-        const int64_t it = __ldcg(st.work + i);
-        const int32_t v = (int32_t)(it >> 32), c = (int32_t)(uint32_t)it;
+      bc_each_item(st, bc_forward_items(st, d - 1), nwarps,
+                   [&](int32_t v, int32_t, int32_t k0, int32_t k1, bool single) {
         const uint64_t own = __ldcg(nm + v);
         double a0, a1;
-        bc_gather(st, v, c, own, pm, st.sigma, a0, a1);
+        bc_gather(st, k0, k1, own, pm, st.sigma, a0, a1);
         double *row = st.sigma + (int64_t)v * kBcWidth;
-        const bool single = bc_chunks(st, v) == 1;
         if ((own >> lane) & 1) {
           if (single) row[lane] = a0;
           else if (a0 != 0.0) atomicAdd(row + lane, a0);
@@ -221,7 +289,7 @@ __global__ void __launch_bounds__(512) k_bc_batch(DGraph g, BcState st) {
           if (single) row[lane + 32] = a1;
           else if (a1 != 0.0) atomicAdd(row + lane + 32, a1);
         }
-      }
+      });
     }
     // the mask array P(d) writes next held Q_{d-2}: clear those entries
     if (d >= 2) {
@@ -259,7 +327,7 @@ __global__ void __launch_bounds__(512) k_bc_batch(DGraph g, BcState st) {
       const int32_t m_up = (m + 31) & ~31;
       uint64_t *nm = bc_fr(st, d + 1);
       for (int32_t i = tid; i < m_up; i += nthreads) {
-        int32_t v = -1, nch = 0;
+        int32_t v = -1, deg = -1;
         if (i < m) {
           v = __ldcg(st.lev + e_d + i);
           const uint64_t a = __ldcg(st.acc + v);
@@ -270,9 +338,9 @@ __global__ void __launch_bounds__(512) k_bc_batch(DGraph g, BcState st) {
           st.acc[v] = 0;
           uint16_t *drow = st.depth + (int64_t)v * kBcWidth;
           for (uint64_t b = nb; b; b &= b - 1) drow[__ffsll((long long)b) - 1] = (uint16_t)(d + 1);
-          nch = bc_chunks(st, v);
+          deg = bc_degree(st, v);
         }
-        bc_push_items(st, st.ctr + 1 + (d & 1), v, nch);
+        bc_push_items(st, st.ctr + 1 + (d & 1), st.ctr + 24 + (d & 1), v, deg);
       }
     }
     clk.tick(st.stop, d, st.err);
@@ -290,8 +358,8 @@ __global__ void __launch_bounds__(512) k_bc_batch(DGraph g, BcState st) {
   for (int32_t dd = L - 1, it = L + 1; alive && dd >= 0; --dd, ++it) {
     if (stopped(st.stop, it)) break;
     if (tid == 0) {
-      st.ctr[3 + ((dd + 1) & 1)] = 0;   // consumed by the gather of level dd + 1
-      st.ctr[18 + ((dd + 1) & 1)] = 0;  // that gather's hand-out counter
+      st.ctr[3 + ((dd + 1) & 1)] = st.ctr[26 + ((dd + 1) & 1)] = 0;   // consumed by the gather of level dd + 1
+      st.ctr[18 + ((dd + 1) & 1)] = st.ctr[30 + ((dd + 1) & 1)] = 0;  // that gather's hand-out
     }
     // sources at level dd + 1 become "deeper" for the gathers from here on
     if (dd + 1 < L) {
@@ -309,7 +377,7 @@ __global__ void __launch_bounds__(512) k_bc_batch(DGraph g, BcState st) {
       const int32_t m_up = (m + 31) & ~31;
       uint64_t *lmn = bc_lm(st, dd);
       for (int32_t i = tid; i < m_up; i += nthreads) {
-        int32_t v = -1, nch = 0;
+        int32_t v = -1, deg = -1;
         if (i < m) {
           v = __ldcg(st.lev + b + i);
           const uint4 *row = reinterpret_cast<const uint4 *>(st.depth + (int64_t)v * kBcWidth);
@@ -325,26 +393,22 @@ __global__ void __launch_bounds__(512) k_bc_batch(DGraph g, BcState st) {
             }
           }
           lmn[v] = mk;
-          nch = bc_chunks(st, v);
+          deg = bc_degree(st, v);
         }
-        bc_push_items(st, st.ctr + 3 + (dd & 1), v, nch);
+        bc_push_items(st, st.ctr + 3 + (dd & 1), st.ctr + 26 + (dd & 1), v, deg);
       }
     }
     if (!grid_barrier(st.bar, gridDim.x, st.err, st.timeout_ns)) break;
     // gather: dep'[v][s] = 1/sigma[v][s] + sum over deeper in-neighbours
     {
-      const int32_t ni = min(*(volatile int32_t *)(st.ctr + 3 + (dd & 1)), st.wcap);
       const uint64_t *lmn = bc_lm(st, dd);
-      for (int32_t i0, i1; bc_take(st.ctr + 18 + (dd & 1), ni, nwarps, i0, i1);)
-      for (int32_t i = i0; i < i1; ++i) {
-        const int64_t it = __ldcg(st.work + i);
-        const int32_t v = (int32_t)(it >> 32), c = (int32_t)(uint32_t)it;
+      bc_each_item(st, bc_backward_items(st, dd), nwarps,
+                   [&](int32_t v, int32_t c, int32_t k0, int32_t k1, bool single) {
         const uint64_t own = __ldcg(lmn + v);
         double a0, a1;
-        bc_gather(st, v, c, own, st.rmask, st.dep, a0, a1);
+        bc_gather(st, k0, k1, own, st.rmask, st.dep, a0, a1);
         const double *srow = st.sigma + (int64_t)v * kBcWidth;
         double *row = st.dep + (int64_t)v * kBcWidth;
-        const bool single = bc_chunks(st, v) == 1;
         if ((own >> lane) & 1) {
           const double t = a0 + (c == 0 ? 1.0 / __ldcg(srow + lane) : 0.0);
           if (single) row[lane] = t;
@@ -355,7 +419,7 @@ __global__ void __launch_bounds__(512) k_bc_batch(DGraph g, BcState st) {
           if (single) row[lane + 32] = t;
           else atomicAdd(row + lane + 32, t);
         }
-      }
+      });
     }
     clk.tick(st.stop, it, st.err);
     if (!grid_barrier(st.bar, gridDim.x, st.err, st.timeout_ns)) break;
