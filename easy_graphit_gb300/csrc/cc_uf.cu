@@ -7,7 +7,8 @@
 //            sorted, so that is v's smallest neighbour)
 //   sample   compress init's chains; union(v, first neighbour of v) where that
 //            neighbour is larger (init joined a smaller one) and union(v, second
-//            neighbour of v); compress every vertex to its root
+//            neighbour of v), a few scouts before the rest; compress every
+//            vertex to its root
 //   giant    c = the most frequent root among 1,024 spread-out vertices
 //   finish   every vertex whose root is not c unions with the rest of its
 //            neighbours -- out-neighbours after the two sampled ones and, on a
@@ -30,11 +31,17 @@
 
 namespace gg {
 
+// Reads go through L1.  Once trees have merged, most walks end at the same few
+// roots, and with every read sent to L2 those lines served one warp at a time
+// (second sampling pass on a symmetrized R-MAT 22: 646 us; 268 us through L1).
+// A stale line is harmless: it holds an older ancestor of x, so the walk stays
+// in x's tree, stores only ancestors, and a stale root is found out by the CAS
+// in uf_union, whose answer is the true parent.
 __device__ __forceinline__ int32_t uf_find(int32_t *parent, int32_t x) {
   for (;;) {
-    const int32_t p = __ldcg(parent + x);
+    const int32_t p = __ldca(parent + x);
     if (p == x) return x;
-    const int32_t gp = __ldcg(parent + p);
+    const int32_t gp = __ldca(parent + p);
     if (gp == p) return p;
     parent[x] = gp;  // path halving
     x = gp;
@@ -64,11 +71,20 @@ __global__ void k_uf_init(const int32_t *__restrict__ off, const int32_t *__rest
   }
 }
 
-// Link v with its out-neighbour number r (the sampling rounds).
+// Link v with its out-neighbour number r (the sampling rounds), over the
+// groups of 32 vertices that `part` names: all of them, the scouts (every
+// `every`-th group) or the others.
+enum : int32_t { UF_ALL = 0, UF_SCOUTS = 1, UF_OTHERS = 2 };
 __global__ void k_uf_sample(const int32_t *__restrict__ off, const int32_t *__restrict__ dst, int32_t V, int32_t r,
-                            int32_t *__restrict__ parent) {
-  for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-    const int32_t b = off[v];
+                            int32_t part, int32_t every, int32_t *__restrict__ parent) {
+  const int32_t groups = ceil_div(V, 32), lane = threadIdx.x & 31;
+  const int32_t scouts = ceil_div(groups, every);
+  const int32_t n = part == UF_ALL ? groups : (part == UF_SCOUTS ? scouts : groups - scouts);
+  for (int32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
+    const int32_t gi = part == UF_ALL ? i : (part == UF_SCOUTS ? i * every : i + i / (every - 1) + 1);
+    const int64_t v64 = (int64_t)gi * 32 + lane;
+    if (v64 >= V) continue;
+    const int32_t v = (int32_t)v64, b = off[v];
     if (off[v + 1] - b > r) {
       const int32_t u = dst[b + r];
       if (u != v && (r > 0 || u > v)) uf_union(parent, v, u);  // init joined a smaller first one
@@ -127,6 +143,7 @@ __global__ void k_uf_final(int32_t *__restrict__ parent, int32_t V, int32_t *__r
 }
 
 constexpr int32_t kUfProbes = 1024;
+constexpr int32_t kUfScouts = 16384;  // vertices of the second sampling round that go first
 
 gg_status cc_union_find(gg_graph *g, int32_t *labels, int32_t *parent) {
   const GraphStore &f = g->csr;
@@ -140,10 +157,21 @@ gg_status cc_union_find(gg_graph *g, int32_t *labels, int32_t *parent) {
   // flatten init's first-neighbour chains before the unions walk them
   note_launch();
   k_uf_compress<<<grid, 256, 0, st>>>(parent, V);
-  for (int32_t r = 0; r < 2; ++r) {
+  note_launch();
+  k_uf_sample<<<grid, 256, 0, st>>>(f.off, f.dst, V, 0, UF_ALL, 2, parent);
+  // The second round is where the big trees meet: with every thread of the GPU
+  // hooking the same few roots at once it is bound by failed CASes.  A few
+  // thousand scouts join those trees first; the rest then find one root
+  // (symmetrized R-MAT 22, both launches: 268 us unsplit, 270 with 262,144
+  // scouts, 145 with 65,536, 114 with 16,384, 104 with 4,096 but a slower whole).
+  // A graph whose scouts would be more than a sixteenth goes in one launch.
+  const int32_t every = V / kUfScouts;
+  if (every >= 16) {
     note_launch();
-    k_uf_sample<<<grid, 256, 0, st>>>(f.off, f.dst, V, r, parent);
+    k_uf_sample<<<grid, 256, 0, st>>>(f.off, f.dst, V, 1, UF_SCOUTS, every, parent);
   }
+  note_launch();
+  k_uf_sample<<<grid, 256, 0, st>>>(f.off, f.dst, V, 1, every >= 16 ? UF_OTHERS : UF_ALL, std::max(every, 2), parent);
   note_launch();
   k_uf_compress<<<grid, 256, 0, st>>>(parent, V);
   // the giant tree's root, by majority over spread-out vertices
