@@ -163,6 +163,10 @@ struct BcBuffers {
 };
 gg_status bcb_buffers(gg_graph *g, bool owned, BcBuffers *b);
 
+// Whether a batch's kernels may write their rows to `out` themselves: memory of
+// the graph's own device.  Anything else goes through a device buffer and a copy.
+bool rows_on_device(const gg_graph *g, const void *out);
+
 // The persistent kernels (for occupancy queries).
 const void *bsssp_kernel();
 const void *msbfs_kernel();

@@ -443,21 +443,37 @@ __global__ void __launch_bounds__(512, 2) k_bc_batch(DGraph g, BcState st) {
   }
 }
 
-// Seeds the k sources (one thread: sources are few; duplicates share a vertex).
-__global__ void k_bcb_seed(BcState st, const int32_t *__restrict__ srcs) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  int32_t n = 0;
-  for (int32_t s = 0; s < st.nsrc; ++s) {
-    const int32_t v = st.perm ? st.perm[srcs[s]] : srcs[s];
-    if (!st.seen[v]) st.lev[n++] = v;
-    st.seen[v] |= 1ull << s;
-    st.fr[0][v] |= 1ull << s;
+// Seeds the sources, a thread of one 64-thread block per source (one thread
+// walking them took 88 us); sources on the same vertex share its list entry.
+__global__ void __launch_bounds__(kBcWidth) k_bcb_seed(BcState st, const int32_t *__restrict__ srcs) {
+  __shared__ int32_t sv[kBcWidth];
+  __shared__ uint32_t firsts[2];
+  const int32_t s = threadIdx.x;
+  if (blockIdx.x != 0) return;
+  const int32_t v = s >= st.nsrc ? -1 : (st.perm ? st.perm[srcs[s]] : srcs[s]);
+  sv[s] = v;
+  __syncthreads();
+  uint64_t same = 0;  // sources on this vertex
+  for (int32_t i = 0; i < st.nsrc; ++i)
+    if (sv[i] == v) same |= 1ull << i;
+  const bool first = v >= 0 && __ffsll((long long)same) - 1 == s;
+  const uint32_t ballot = __ballot_sync(0xffffffffu, first);
+  if ((s & 31) == 0) firsts[s >> 5] = ballot;
+  __syncthreads();
+  if (first) {
+    st.lev[__popc(ballot & ((1u << (s & 31)) - 1)) + (s >= 32 ? __popc(firsts[0]) : 0)] = v;
+    st.seen[v] = same;
+    st.fr[0][v] = same;
+  }
+  if (v >= 0) {
     st.depth[(int64_t)v * kBcWidth + s] = 0;
     st.sigma[(int64_t)v * kBcWidth + s] = 1.0;
   }
-  st.ctr[0] = n;
-  st.ctr[20] = n;  // Q_0's end, read by every CTA before any appends to ctr[0]
-  *st.stop = 0;
+  if (s == 0) {
+    st.ctr[0] = __popc(firsts[0]) + __popc(firsts[1]);
+    st.ctr[20] = st.ctr[0];  // Q_0's end, read by every CTA before any appends to ctr[0]
+    *st.stop = 0;
+  }
 }
 
 // delta[s][v] = (dep'[p][s] - 1/sigma[p][s]) * sigma[p][s] as fp32 rows (v an
@@ -601,7 +617,7 @@ gg_status bcb_enqueue(gg_graph *g, cudaStream_t st, const BcBuffers &b, int32_t 
   GG_CUDA(cudaMemsetAsync(b.depth, 0xff, b.bytes_depth, st));
   GG_CUDA(cudaMemsetAsync(b.vals, 0, b.bytes_vals, st));
   note_launch();
-  k_bcb_seed<<<1, 32, 0, st>>>(S, dsrc);
+  k_bcb_seed<<<1, kBcWidth, 0, st>>>(S, dsrc);
   GG_CUDA(cudaMemsetAsync(S.bar, 0, sizeof(uint32_t) * 2, st));
   DGraph dg = (S0.perm != nullptr) ? g->rel->g.view() : g->csr.view();
   dg.nbuckets = 0;
@@ -633,7 +649,8 @@ extern "C" gg_status gg_bc_batch(gg_graph *g, const int32_t *sources, int32_t ns
   BcBuffers b;
   GG_TRY(bcb_buffers(g, false, &b));
   float *rows = nullptr;
-  GG_TRY(scratch_get_app(g, 6, sizeof(float) * (size_t)std::min(nsrc, kBcWidth) * V, (void **)&rows));
+  const bool direct = rows_on_device(g, dep_out);
+  if (!direct) GG_TRY(scratch_get_app(g, 6, sizeof(float) * (size_t)std::min(nsrc, kBcWidth) * V, (void **)&rows));
   unsigned long long *reached = reinterpret_cast<unsigned long long *>(b.dsrc + kBcWidth);
   const uint64_t l0 = launches();
   GG_CUDA(cudaMemsetAsync(reached, 0, sizeof(unsigned long long), st));
@@ -643,8 +660,10 @@ extern "C" gg_status gg_bc_batch(gg_graph *g, const int32_t *sources, int32_t ns
   for (int32_t base = 0; base < nsrc; base += kBcWidth) {
     const int32_t k = std::min(kBcWidth, nsrc - base);
     GG_CUDA(cudaMemcpyAsync(b.dsrc, sources + base, sizeof(int32_t) * k, cudaMemcpyDefault, st));
-    GG_TRY(bcb_enqueue(g, st, b, k, b.dsrc, rows, V, reached, nullptr, true));
-    GG_CUDA(cudaMemcpyAsync(dep_out + (size_t)base * V, rows, sizeof(float) * (size_t)k * V, cudaMemcpyDefault, st));
+    float *out = direct ? dep_out + (size_t)base * V : rows;
+    GG_TRY(bcb_enqueue(g, st, b, k, b.dsrc, out, V, reached, nullptr, true));
+    if (!direct)
+      GG_CUDA(cudaMemcpyAsync(dep_out + (size_t)base * V, out, sizeof(float) * (size_t)k * V, cudaMemcpyDefault, st));
     const BcState S = bcb_state(g, b, k);
     GG_CUDA(cudaMemcpyAsync(g->h_pinned + 30, S.stats, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     GG_CUDA(cudaStreamSynchronize(st));

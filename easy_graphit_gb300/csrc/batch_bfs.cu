@@ -252,33 +252,45 @@ __global__ void k_msbfs_init(MsBfsState st) {
   }
 }
 
-// Sources seeded (one thread: sources are few; duplicates share a vertex).
-__global__ void k_msbfs_seed(MsBfsState st, const int32_t *__restrict__ srcs) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  int32_t n = 0;
-  unsigned long long all = 0;
-  for (int32_t s = 0; s < st.nsrc; ++s) {
-    const int32_t v = srcs[s];
-    if (!st.seen[v]) st.q[0][n++] = v;
-    st.seen[v] |= 1ull << s;
-    st.fr[0][v] |= 1ull << s;
-    all |= 1ull << s;
-    st.depth[(int64_t)s * st.depth_stride + v] = 0;
+// Control words and sources, a thread of one 64-thread block per source (one
+// thread walking the sources took 91 us of dependent round trips); sources on
+// the same vertex share its queue entry.
+__global__ void __launch_bounds__(kMsBfsWidth) k_msbfs_seed(MsBfsState st, const int32_t *__restrict__ srcs) {
+  __shared__ int32_t sv[kMsBfsWidth];
+  __shared__ unsigned long long stat[3];
+  const int32_t s = threadIdx.x;
+  if (blockIdx.x != 0) return;
+  const int32_t v = s < st.nsrc ? srcs[s] : -1;
+  sv[s] = v;
+  if (s < 3) stat[s] = 0ull;
+  __syncthreads();
+  uint64_t same = 0;  // sources on this vertex
+  for (int32_t i = 0; i < st.nsrc; ++i)
+    if (sv[i] == v) same |= 1ull << i;
+  const bool first = v >= 0 && __ffsll((long long)same) - 1 == s;
+  const uint32_t ballot = __ballot_sync(0xffffffffu, first);
+  __shared__ uint32_t firsts[2];
+  if ((s & 31) == 0) firsts[s >> 5] = ballot;
+  __syncthreads();
+  if (first) {
+    const int32_t pos = __popc(ballot & ((1u << (s & 31)) - 1)) + (s >= 32 ? __popc(firsts[0]) : 0);
+    st.q[0][pos] = v;
+    st.seen[v] = same;
+    st.fr[0][v] = same;
+    const unsigned long long d = (unsigned long long)(st.off[v + 1] - st.off[v]);  // the sources' frontier
+    atomicAdd(stat, d);
+    atomicAdd(stat + 1, d * d);
+    atomicMax(stat + 2, d);
   }
-  for (int i = 0; i < 4; ++i) st.cnt4[i] = 0;
-  st.cnt4[0] = n;
-  for (int i = 0; i < 3; ++i) st.hub3[i] = 0;
-  for (int i = 0; i < 12; ++i) st.lstat[i] = 0ull;
-  for (int32_t i = 0; i < n; ++i) {  // the sources' frontier
-    const unsigned long long d = (unsigned long long)(st.off[st.q[0][i] + 1] - st.off[st.q[0][i]]);
-    st.lstat[0] += d;
-    st.lstat[1] += d * d;
-    st.lstat[2] = st.lstat[2] > d ? st.lstat[2] : d;
+  if (v >= 0) st.depth[(int64_t)s * st.depth_stride + v] = 0;
+  __syncthreads();
+  if (s < 12) st.lstat[s] = s < 3 ? stat[s] : 0ull;
+  if (s < 4) st.cnt4[s] = s == 0 ? __popc(firsts[0]) + __popc(firsts[1]) : 0;
+  if (s < 3) {
+    st.hub3[s] = 0;
+    st.actm[s] = s == 0 ? (st.nsrc >= 64 ? ~0ull : (1ull << st.nsrc) - 1) : 0ull;
   }
-  st.actm[0] = all;
-  st.actm[1] = 0;
-  st.actm[2] = 0;
-  *st.stop = 0;
+  if (s == 0) *st.stop = 0;
 }
 
 // ------------------------------------------------------------------ host
@@ -342,6 +354,15 @@ MsBfsState msbfs_state(gg_graph *g, const MsBfsBuffers &b, int32_t k, int32_t *d
   return S;
 }
 
+bool rows_on_device(const gg_graph *g, const void *out) {
+  cudaPointerAttributes pa{};
+  if (cudaPointerGetAttributes(&pa, out) != cudaSuccess) {
+    cudaGetLastError();  // not an address CUDA knows: the copy decides
+    return false;
+  }
+  return pa.type == cudaMemoryTypeDevice && pa.device == g->device && reinterpret_cast<uintptr_t>(out) % 4 == 0;
+}
+
 const void *msbfs_kernel() { return (const void *)k_msbfs; }
 
 // One pass of k <= 64 sources: reset, seed, the persistent loop writing the
@@ -356,7 +377,7 @@ gg_status msbfs_enqueue(gg_graph *g, cudaStream_t st, const MsBfsState &S, const
   note_launch();
   k_msbfs_init<<<g->sm_count * 8, 256, 0, st>>>(S);
   note_launch();
-  k_msbfs_seed<<<1, 32, 0, st>>>(S, dsrc);
+  k_msbfs_seed<<<1, kMsBfsWidth, 0, st>>>(S, dsrc);
   GG_CUDA(cudaMemsetAsync(S.bar, 0, sizeof(uint32_t) * 2, st));
   DGraph dg = g->csr.view();
   dg.nbuckets = 0;
@@ -386,18 +407,21 @@ extern "C" gg_status gg_bfs_batch(gg_graph *g, const int32_t *sources, int32_t n
   MsBfsBuffers b;
   GG_TRY(msbfs_buffers(g, nsrc, false, &b));
   int32_t *depth = nullptr;
-  GG_TRY(scratch_get_app(g, 3, sizeof(int32_t) * (size_t)std::min(nsrc, kMsBfsWidth) * V, (void **)&depth));
+  const bool direct = rows_on_device(g, depth_out);
+  if (!direct)
+    GG_TRY(scratch_get_app(g, 3, sizeof(int32_t) * (size_t)std::min(nsrc, kMsBfsWidth) * V, (void **)&depth));
   const uint64_t l0 = launches();
   cudaEventRecord(g->ev0, st);
   float loop_ms = 0;
   int32_t levels = 0;
   for (int32_t base = 0; base < nsrc; base += kMsBfsWidth) {
     const int32_t k = std::min(kMsBfsWidth, nsrc - base);
-    const MsBfsState S = msbfs_state(g, b, k, depth);
+    const MsBfsState S = msbfs_state(g, b, k, direct ? depth_out + (size_t)base * V : depth);
     GG_CUDA(cudaMemcpyAsync(b.dsrc, sources + base, sizeof(int32_t) * k, cudaMemcpyDefault, st));
     GG_TRY(msbfs_enqueue(g, st, S, b.dsrc, true));
-    GG_CUDA(cudaMemcpyAsync(depth_out + (size_t)base * V, depth, sizeof(int32_t) * (size_t)k * V,
-                            cudaMemcpyDefault, st));
+    if (!direct)
+      GG_CUDA(cudaMemcpyAsync(depth_out + (size_t)base * V, depth, sizeof(int32_t) * (size_t)k * V,
+                              cudaMemcpyDefault, st));
     GG_CUDA(cudaMemcpyAsync(g->h_pinned + 30, S.stats, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     GG_CUDA(cudaStreamSynchronize(st));
     float ms = 0;

@@ -720,26 +720,25 @@ __global__ void k_bsssp_init(BsState S, const int32_t *__restrict__ srcs, int32_
   }
 }
 
+// Control words and sources, a lane per source (one thread walking the sources
+// took 61 us of dependent round trips); a shared vertex is queued once.
 __global__ void k_bsssp_seed(BsState S, const int32_t *__restrict__ srcs, int32_t nsrc) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  for (int32_t i = 0; i < 8; ++i) S.cnt[i] = 0;
-  for (int32_t i = 0; i < 3; ++i) {
-    S.wctr[i] = 0;
-    S.hcnt[i] = 0;
-  }
-  *S.stop = 0;
-  for (int32_t s = 0; s < kLanes; ++s) {
-    S.cur[s] = s < nsrc ? 0 : INT_MAX;
-    S.cur[kLanes + s] = S.cur[s];
-    S.gmin[s] = INT_MAX;
-    S.gmin[kLanes + s] = INT_MAX;
-  }
-  for (int32_t s = 0; s < nsrc; ++s) {
-    const int32_t v = S.perm[srcs[s]];
-    S.dist[(int64_t)v * kLanes + s] = 0;
-    if (!S.fr[v]) bs_enqueue(S, S.q[0], S.cnt + 0, v);
-    S.fr[v] |= 1u << s;
-  }
+  const int32_t s = threadIdx.x;
+  if (blockIdx.x != 0 || s >= kLanes) return;
+  if (s < 8) S.cnt[s] = 0;
+  if (s < 3) S.wctr[s] = S.hcnt[s] = 0;
+  if (s == 0) *S.stop = 0;
+  S.cur[s] = S.cur[kLanes + s] = s < nsrc ? 0 : INT_MAX;
+  S.gmin[s] = S.gmin[kLanes + s] = INT_MAX;
+  __threadfence();
+  __syncwarp();
+  const int32_t v = s < nsrc ? S.perm[srcs[s]] : -1;
+  const uint32_t same = __match_any_sync(0xffffffffu, v);
+  if (v < 0) return;
+  S.dist[(int64_t)v * kLanes + s] = 0;
+  if (s != __ffs(same) - 1) return;
+  S.fr[v] = same;
+  bs_enqueue(S, S.q[0], S.cnt + 0, v);
 }
 
 // Rows out[s][v] = dist[perm[v]][s] for s < nsrc (v an original id), through
@@ -874,6 +873,7 @@ extern "C" gg_status gg_sssp_batch(gg_graph *g, const int32_t *sources, int32_t 
     GG_CHECK_ARG(sources[i] >= 0 && sources[i] < V, "source out of range");
   if (stats) *stats = gg_stats{};
   cudaStream_t st = g->stream;
+  const bool direct = rows_on_device(g, dist_out);
   bool per_cta = false;
   GG_TRY(bsssp_use_cta(g, &per_cta));
   if (per_cta) {  // a CTA per source (batch_sssp_cta.cu)
@@ -887,9 +887,11 @@ extern "C" gg_status gg_sssp_batch(gg_graph *g, const int32_t *sources, int32_t 
     for (int32_t base = 0; base < nsrc; base += W) {
       const int32_t k = std::min(W, nsrc - base);
       GG_CUDA(cudaMemcpyAsync(cb.dsrc, sources + base, sizeof(int32_t) * k, cudaMemcpyDefault, st));
-      GG_TRY(bsssp_cta_run(g, st, cb, cb.rows, k, delta, true));
-      GG_CUDA(cudaMemcpyAsync(dist_out + (size_t)base * V, cb.rows, sizeof(int32_t) * (size_t)k * V,
-                              cudaMemcpyDefault, st));
+      int32_t *rows = direct ? dist_out + (size_t)base * V : cb.rows;
+      GG_TRY(bsssp_cta_run(g, st, cb, rows, k, delta, true));
+      if (!direct)
+        GG_CUDA(cudaMemcpyAsync(dist_out + (size_t)base * V, rows, sizeof(int32_t) * (size_t)k * V,
+                                cudaMemcpyDefault, st));
       GG_CUDA(cudaMemcpyAsync(g->h_pinned + 30, cb.stats, sizeof(int32_t) * 2, cudaMemcpyDeviceToHost, st));
       GG_CUDA(cudaStreamSynchronize(st));
       float ms = 0;
@@ -921,9 +923,11 @@ extern "C" gg_status gg_sssp_batch(gg_graph *g, const int32_t *sources, int32_t 
   for (int32_t base = 0; base < nsrc; base += kLanes) {
     const int32_t k = std::min(kLanes, nsrc - base);
     GG_CUDA(cudaMemcpyAsync(b.dsrc, sources + base, sizeof(int32_t) * k, cudaMemcpyDefault, st));
-    GG_TRY(bsssp_enqueue(g, st, S, b.dsrc, k, b.out, true));
-    GG_CUDA(cudaMemcpyAsync(dist_out + (size_t)base * V, b.out, sizeof(int32_t) * (size_t)k * V,
-                            cudaMemcpyDefault, st));
+    int32_t *rows = direct ? dist_out + (size_t)base * V : b.out;
+    GG_TRY(bsssp_enqueue(g, st, S, b.dsrc, k, rows, true));
+    if (!direct)
+      GG_CUDA(cudaMemcpyAsync(dist_out + (size_t)base * V, rows, sizeof(int32_t) * (size_t)k * V,
+                              cudaMemcpyDefault, st));
     GG_CUDA(cudaMemcpyAsync(g->h_pinned + 30, S.stats, sizeof(int32_t) * 2, cudaMemcpyDeviceToHost, st));
     GG_CUDA(cudaStreamSynchronize(st));
     float ms = 0;
