@@ -76,19 +76,23 @@ __device__ __forceinline__ HubList level_hubs(const FusedArgs &a, int64_t level)
   return HubList{a.hub_list, a.hub3 + level % 3, a.hub_cap, a.hub_min};
 }
 
-__device__ __forceinline__ DOut sparse_out(const FusedArgs &a, int32_t *q, int64_t it) {
+__device__ __forceinline__ DOut sparse_out(const FusedArgs &a, int32_t *q, int64_t it, Stage *stage) {
   DOut o{};
   o.mode = OUT_SPARSE;
   o.q = q;
   o.cnt = a.cnt3 + it % 3;
   o.cap = a.cap;
   o.err = a.err;
+  o.stage = stage;
   return o;
 }
 
 template <int LB>
 __global__ void __launch_bounds__(1024) k_bfs_fused(FusedArgs a) {
   extern __shared__ int4 smem[];
+  __shared__ Stage stage;
+  if (threadIdx.x == 0) stage.n = 0;
+  __syncthreads();
   int32_t *qs[2] = {a.q0, a.q1};
   int in = 0;
   int64_t level = 1;
@@ -105,14 +109,16 @@ __global__ void __launch_bounds__(1024) k_bfs_fused(FusedArgs a) {
     const HubList hub = level_hubs(a, level);
     const EdgeF<UBfs, false> f{UBfs{a.vd.parent, a.vd.depth, (int32_t)level},
                                DIn{IN_ALL, nullptr, nullptr}, DIn{IN_ALL, nullptr, nullptr}, true};
-    const DOut out = sparse_out(a, qs[in ^ 1], level);
+    const DOut out = sparse_out(a, qs[in ^ 1], level, &stage);
     run_lb<LB>(a.g, en, n, f, out, smem, blockIdx.x, gridDim.x, hub);
+    stage_flush(out);
     clk.tick(a.stop, (int32_t)level, a.err);
     if (!grid_barrier(a.bar, gridDim.x, a.err, a.timeout_ns)) break;
     const int32_t chunks = *(volatile int32_t *)hub.cnt;
     n = *(volatile int32_t *)out.cnt;
     if (chunks) {  // the level's hubs, by all CTAs
       lb_hubs(a.g, hub, chunks, f, out, blockIdx.x, gridDim.x);
+      stage_flush(out);
       if (!grid_barrier(a.bar, gridDim.x, a.err, a.timeout_ns)) break;
       n = *(volatile int32_t *)out.cnt;
     }
@@ -374,14 +380,26 @@ struct DoStat {
   float sq;
 };
 
-// Adds the out-degree k of a vertex entering the next frontier: one reduction
-// over the threads that reach this point together, one shared atomic each.
-__device__ __forceinline__ void do_note(DoStat *s, uint32_t k) {
-  cg::coalesced_group g = cg::coalesced_threads();
-  const uint32_t sum = cg::reduce(g, k, cg::plus<uint32_t>());
-  const float sq = cg::reduce(g, (float)k * (float)k, cg::plus<float>());
-  const uint32_t mx = cg::reduce(g, k, cg::greater<uint32_t>());
-  if (g.thread_rank() == 0) {
+// A thread's share of them, folded into the CTA's at the end of the level: an
+// atomic per vertex (on floats a CAS loop in shared memory) would serialise a
+// CTA that finds thousands.
+struct DoAcc {
+  uint32_t sum, mx;
+  float sq;
+  __device__ __forceinline__ void note(uint32_t k) {
+    sum += k;
+    mx = max(mx, k);
+    sq += (float)k * (float)k;
+  }
+};
+
+__device__ __forceinline__ void do_fold(DoStat *s, const DoAcc &t) {
+  const uint32_t sum = __reduce_add_sync(0xffffffffu, t.sum), mx = __reduce_max_sync(0xffffffffu, t.mx);
+  if (!(sum | mx)) return;
+  float sq = t.sq;
+#pragma unroll
+  for (int i = 16; i > 0; i >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, i);
+  if ((threadIdx.x & 31) == 0) {
     atomicAdd(&s->sum, sum);
     atomicAdd(&s->sq, sq);
     atomicMax(&s->mx, mx);
@@ -394,18 +412,99 @@ struct UBfsNote {
   static constexpr bool kWeight = false;
   int32_t *parent, *depth;
   const int32_t *off;
-  DoStat *stat;  // shared memory; null: no statistics
+  DoAcc *acc;  // this thread's; null: no statistics
   int32_t level;
   __device__ __forceinline__ bool filter(int32_t v) const { return vload(parent + v) == -1; }
   __device__ __forceinline__ bool apply(int32_t s, int32_t d, int32_t) const {
     // the degree is loaded alongside the CAS (not after it): one round trip
-    const int32_t o0 = stat ? __ldg(off + d) : 0, o1 = stat ? __ldg(off + d + 1) : 0;
+    const int32_t o0 = acc ? __ldg(off + d) : 0, o1 = acc ? __ldg(off + d + 1) : 0;
     if (!cas(parent + d, -1, s)) return false;
     depth[d] = level;
-    if (stat) do_note(stat, (uint32_t)(o1 - o0));
+    if (acc) acc->note((uint32_t)(o1 - o0));
     return true;
   }
 };
+
+// A pull level: every vertex without a parent looks for an in-neighbour at the
+// previous level (depth doubles as the frontier bitmap) and takes the first.
+// A lane per vertex reads the parents (coalesced), drops vertices without
+// in-edges, and tests its vertex's first kPullFirst in-neighbours, all in flight
+// together -- where a pull level pays, the frontier is large and most vertices
+// end there.  The lists still open are finished by 8-lane groups, four vertices
+// at a time.  An 8-lane group per vertex from the start needed a round trip per
+// 4 vertices of a warp just to skip the visited ones (directed R-MAT 22, the
+// level that finds 1.1 M vertices: 650 us, 470 with staged appends, now 63).
+constexpr int kPullFirst = 4;
+__device__ __forceinline__ void do_pull_level(const FusedArgs &a, const DoArgs &d, int32_t level, const DOut &out,
+                                              DoAcc *acc) {
+  const int32_t lane = threadIdx.x & 31, sub = lane & 7, gi = lane >> 3;
+  const uint32_t gmask = 0xFFu << (gi * 8);
+  const int32_t prev = level - 1, V = a.g.V;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  int32_t since = 0;  // vertices a CTA can have staged since the stage last had room for a round
+  for (int64_t first = (int64_t)blockIdx.x * blockDim.x; first < V; first += stride) {
+    if (since + (int32_t)blockDim.x > kStageCap / 2) {
+      __syncthreads();
+      stage_make_room(out, kStageCap / 2 + (int32_t)blockDim.x);
+      __syncthreads();
+      since = 0;
+    }
+    since += (int32_t)blockDim.x;
+    const int64_t base = first + (threadIdx.x & ~31);
+    const int32_t v = (int32_t)base + lane;
+    int32_t kb = 0, ke = 0;
+    if (base + lane < V && __ldcg(a.vd.parent + v) == -1) {
+      kb = __ldg(d.t.off + v);
+      ke = __ldg(d.t.off + v + 1);
+    }
+    int32_t hit = -1, u[kPullFirst], du[kPullFirst];
+#pragma unroll
+    for (int j = 0; j < kPullFirst; ++j) u[j] = kb + j < ke ? __ldg(d.t.dst + kb + j) : -1;
+#pragma unroll
+    for (int j = 0; j < kPullFirst; ++j) du[j] = u[j] >= 0 ? __ldcg(a.vd.depth + u[j]) : -2;
+#pragma unroll
+    for (int j = kPullFirst - 1; j >= 0; --j)
+      if (du[j] == prev) hit = u[j];
+    uint32_t open = __ballot_sync(0xffffffffu, hit < 0 && ke - kb > kPullFirst);
+    while (open) {
+      int32_t l[4];  // the next four open vertices, a group each (-1: none)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        l[j] = __ffs(open) - 1;
+        open &= open - 1;
+      }
+      const int32_t mine = gi == 0 ? l[0] : (gi == 1 ? l[1] : (gi == 2 ? l[2] : l[3]));
+      const int32_t b = __shfl_sync(0xffffffffu, kb, mine & 31) + kPullFirst;
+      const int32_t e = __shfl_sync(0xffffffffu, ke, mine & 31);
+      int32_t found = -1;
+      if (mine >= 0)
+        for (int32_t k0 = b; k0 < e; k0 += 8) {
+          int32_t w = -1;
+          if (k0 + sub < e) {
+            w = __ldg(d.t.dst + k0 + sub);
+            if (__ldcg(a.vd.depth + w) != prev) w = -1;
+          }
+          const uint32_t bits = __ballot_sync(gmask, w >= 0) >> (gi * 8) & 0xFFu;
+          if (bits) {
+            found = __shfl_sync(gmask, w, gi * 8 + __ffs(bits) - 1);
+            break;
+          }
+        }
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int32_t h = __shfl_sync(0xffffffffu, found, j * 8);
+        if (lane == l[j]) hit = h;
+      }
+    }
+    if (hit >= 0) {
+      a.vd.parent[v] = hit;
+      a.vd.depth[v] = level;
+      out.sparse(v);
+      if (acc) acc->note((uint32_t)(__ldg(a.g.off + v + 1) - __ldg(a.g.off + v)));
+    }
+  }
+}
 
 // Dynamic shared memory: the push strategy's, then (DO_SELECTOR) the staged
 // network parameters.
@@ -415,6 +514,7 @@ template <int LB>
 __global__ void __launch_bounds__(kBfsDoMaxCta, 4) k_bfs_do(DoKernelArgs ka, uint32_t lb_bytes) {
   extern __shared__ int4 smem[];
   __shared__ DoStat s_stat;
+  __shared__ Stage stage;
   __shared__ float s_x[16 + 64];
   __shared__ int32_t s_pull;
   __shared__ float s_in[4];    // n, out-degree sum, sum of squares, maximum of this level's frontier
@@ -427,6 +527,7 @@ __global__ void __launch_bounds__(kBfsDoMaxCta, 4) k_bfs_do(DoKernelArgs ka, uin
   if (threadIdx.x == 0) {
     s_vis[0] = s_vis[1] = 0.f;
     s_pulls = 0;
+    stage.n = 0;
   }
   __syncthreads();
   int32_t level = 1;
@@ -476,13 +577,14 @@ __global__ void __launch_bounds__(kBfsDoMaxCta, 4) k_bfs_do(DoKernelArgs ka, uin
     }
     __syncthreads();
     const bool pull = s_pull != 0;
-    DoStat *stat = d.stats ? &s_stat : nullptr;
-    const DOut out = sparse_out(a, (level & 1) ? a.q1 : a.q0, level);
+    const DOut out = sparse_out(a, (level & 1) ? a.q1 : a.q0, level, &stage);
     const HubList hub = level_hubs(a, level);
     // One pass over the frontier or the unreached vertices; a push level that
     // set hubs aside (lb.cuh) has a second one, over their chunks by all CTAs.
     bool ok;
     for (int32_t chunks = 0;;) {
+      DoAcc acc{0u, 0u, 0.f};
+      DoAcc *stat = d.stats ? &acc : nullptr;
       if (!pull) {
         const Enum en{(level & 1) ? a.q0 : a.q1, nullptr, n};
         const EdgeF<UBfsNote, false> f{UBfsNote{a.vd.parent, a.vd.depth, a.g.off, stat, level},
@@ -493,36 +595,10 @@ __global__ void __launch_bounds__(kBfsDoMaxCta, 4) k_bfs_do(DoKernelArgs ka, uin
           run_lb<LB>(a.g, en, n, f, out, smem, blockIdx.x, gridDim.x, hub);
       } else {
         if (threadIdx.x == 0) ++s_pulls;
-        const int32_t lane = threadIdx.x & 31, sub = lane & 7, gbase = lane & ~7;
-        const uint32_t gmask = 0xFFu << gbase;
-        const int32_t prev = level - 1;
-        for (int32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; v < a.g.V;
-             v += (gridDim.x * blockDim.x) >> 3) {
-          if (__ldcg(a.vd.parent + v) != -1) continue;
-          const int32_t kb = __ldg(d.t.off + v), ke = __ldg(d.t.off + v + 1);
-          const int32_t deg = stat && sub == 0 ? __ldg(a.g.off + v + 1) - __ldg(a.g.off + v) : 0;
-          int32_t hit = -1;
-          for (int32_t k0 = kb; k0 < ke; k0 += 8) {
-            int32_t u = -1;
-            if (k0 + sub < ke) {
-              u = __ldg(d.t.dst + k0 + sub);
-              if (__ldcg(a.vd.depth + u) != prev) u = -1;
-            }
-            const uint32_t bits = (__ballot_sync(gmask, u >= 0) >> gbase) & 0xFFu;
-            if (bits) {
-              hit = __shfl_sync(gmask, u, gbase + __ffs(bits) - 1);
-              break;
-            }
-          }
-          if (hit >= 0 && sub == 0) {
-            a.vd.parent[v] = hit;
-            a.vd.depth[v] = level;
-            out.sparse(v);
-            if (stat) do_note(stat, (uint32_t)deg);
-          }
-        }
+        do_pull_level(a, d, level, out, stat);
       }
-      __syncthreads();
+      if (d.stats) do_fold(&s_stat, acc);
+      stage_flush(out);  // its first barrier also ends the CTA's statistics
       if (d.stats && threadIdx.x == 0) {
         if (!chunks) {
           s_vis[0] = fminf((float)a.g.V, s_vis[0] + s_in[0]);

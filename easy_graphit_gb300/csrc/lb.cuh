@@ -213,7 +213,10 @@ __device__ __forceinline__ void lb_twce_all(const DGraph &g, const Enum &en, int
                                           const HubList &hub) {
   const int32_t nv = ceil_div(n, blockDim.x / kStage1);
   if (nv >= nparts) {
-    for (int32_t v = rank; v < nv; v += nparts) lb_twce(g, en, n, f, out, v, 0, 1, sm, hub);
+    for (int32_t v = rank; v < nv; v += nparts) {
+      lb_twce(g, en, n, f, out, v, 0, 1, sm, hub);
+      stage_make_room(out, kStageCap / 2);
+    }
   } else if (nv > 0) {
     const int32_t slices = nparts / nv;
     if (rank < nv * slices) lb_twce(g, en, n, f, out, rank % nv, rank / nv, slices, sm, hub);
@@ -233,7 +236,14 @@ __device__ __forceinline__ void lb_chunk(const DGraph &g, const int32_t *chunk_l
 template <class F>
 __device__ __forceinline__ void lb_hubs(const DGraph &g, const HubList &hub, int32_t chunks, const F &f,
                                         const DOut &out, int32_t rank, int32_t nparts) {
-  for (int32_t c = rank; c < min(chunks, hub.cap); c += nparts) lb_chunk(g, hub.list, f, out, c);
+  for (int32_t c = rank; c < min(chunks, hub.cap); c += nparts) {
+    lb_chunk(g, hub.list, f, out, c);
+    if (out.stage) {
+      __syncthreads();
+      stage_make_room(out, kStageCap / 2);
+      __syncthreads();
+    }
+  }
 }
 
 // ---------------------------------------------------------------------- CM
