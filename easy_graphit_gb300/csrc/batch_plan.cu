@@ -71,7 +71,10 @@ gg_status gg_batch_plan_create(gg_graph *g, int32_t app, const int32_t *sources,
     if (!g->app_frontier) GG_TRY(gg_frontier_create(g, 0, &g->app_frontier));
     GG_TRY(ensure_hubs(g));
     if (app == GG_BATCH_BFS_MULTI) GG_CUDA(cudaMalloc(&p->parent, sizeof(int32_t) * std::max(V, 1)));
-    if (app == GG_BATCH_SSSP_MULTI) GG_TRY(bq_alloc(g, &p->bq));
+    if (app == GG_BATCH_SSSP_MULTI) {
+      GG_TRY(fused_multi_setup(g));
+      GG_TRY(bq_alloc(g, &p->bq));
+    }
   } else if (app == GG_BATCH_BFS) {
     GG_TRY(msbfs_buffers(g, nsrc, true, &p->ms));
   } else if (app == GG_BATCH_SSSP) {

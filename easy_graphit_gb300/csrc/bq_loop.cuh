@@ -65,6 +65,7 @@ struct BqArgs {
   int32_t width0;       // first horizon width, in buckets
   int32_t *hub_list;    // hub chunks (HubList); their counts are control words
   int32_t hub_cap, hub_min;
+  int32_t mesh;         // largest out-degree <= 32: one-CTA sessions run in shared memory (bq_mesh_session)
 };
 
 // Loop state, the same in every CTA: every decision is taken from control
@@ -244,6 +245,322 @@ __device__ __forceinline__ void bq_step(BqLoop &s, const BqArgs &a, const BqStep
       break;
   }
   s.it++;
+}
+
+// ---------------------------------------------------------- mesh sessions
+// CTA 0's one-CTA mode on a graph of short lists (largest out-degree at most
+// kMeshMaxDegree): the same rule and the same counts, with the frontier and the
+// low pile in shared memory.  A bucket is bound by its dependent L2 round trips.
+// In bq_step's form an advance is two steps (minimum, split) and a relax reads
+// queue, offsets, edges, targets and answers of the stamp exchanges one after the
+// other, 15 to 20 trips and as many barriers a bucket; here
+//  * an advance reads the pile's priorities once (one trip), reduces them and
+//    splits the pile from shared memory;
+//  * a relax has two trips: a vertex's edges, then the targets' distances,
+//    stamps and edge ranges together; what it queues carries priority and edge
+//    range.  Four lanes share a vertex, an edge each;
+//  * a park decides by the stamp it read and marks the vertex with a plain
+//    store: a vertex parked twice in one round may be listed twice, which the
+//    exchange at the end of the session (mesh_writeback) undoes, so the piles in
+//    global memory hold a vertex once.
+// An entry that an advance takes or finds settled can never be parked again
+// (its distance stays below every later cutoff), so a session needs one mark.
+// 700 x 501 grid, delta 128 (1,344 buckets, 3 relaxes each): 24-29 -> 12.9 ms;
+// a session's relax of 250 vertices takes 5,000 cycles, of 8 2,300, an advance
+// over a pile of 900 3,900 (bq_step: 7,300 a step).
+constexpr int32_t kMeshMaxDegree = 32;
+constexpr int32_t kMeshNear = 2048;  // frontier entries a session holds
+constexpr int32_t kMeshLow = 2048;   // low-pile entries
+constexpr int32_t kMeshHigh = 1024;  // high parks buffered between flushes
+struct BqMeshSmem {
+  int4 near_[2][kMeshNear];  // v, priority, first edge, end edge
+  int4 lo[2][kMeshLow];      // v, priority at the last scan, first edge, end edge
+  int32_t hi[kMeshHigh];
+  int32_t n_near[2], n_lo[2], n_hi, spill, full, min3[3], quit;
+};
+
+// Places of a warp's appends to up to three lists, `to` the list of this lane's
+// entry (-1: none) and `cnt` on lane i list i's count: one shared-memory atomic
+// a list.  The whole warp calls it.
+__device__ __forceinline__ int32_t mesh_places(int32_t to, int32_t *cnt) {
+  const int32_t lane = threadIdx.x & 31;
+  const uint32_t m0 = __ballot_sync(0xffffffffu, to == 0), m1 = __ballot_sync(0xffffffffu, to == 1),
+                 m2 = __ballot_sync(0xffffffffu, to == 2);
+  if (!(m0 | m1 | m2)) return 0;
+  const int32_t own = __popc(lane == 0 ? m0 : (lane == 1 ? m1 : m2));
+  int32_t base = 0;
+  if (lane < 3 && own) base = atomicAdd(cnt, own);
+  base = __shfl_sync(0xffffffffu, base, to & 3);
+  return base + __popc((to == 0 ? m0 : (to == 1 ? m1 : m2)) & ((1u << lane) - 1));
+}
+
+// Buffered high parks to the high pile of generation gh; the whole CTA calls it
+// between barriers.
+__device__ __forceinline__ void mesh_flush_high(const BqLoop &s, const BqArgs &a, int32_t *sctl, BqMeshSmem &m,
+                                                int32_t mark_lo) {
+  const int32_t n = min(m.n_hi, kMeshHigh), tag = bq_hi_tag(s.gh), lo_tag = bq_lo_tag(s.g);
+  for (int32_t i = threadIdx.x; i < n; i += blockDim.x) {
+    const int32_t v = m.hi[i], t = __ldcg(a.b.stamp + v);
+    if (t == mark_lo || t == lo_tag || t == bq_lo_tag(s.g + 1)) continue;  // since parked lower
+    if (atomicExch(a.b.stamp + v, tag) == tag) continue;
+    const int32_t pos = agg_inc(sctl + BQ_HI + (s.gh & 1));
+    if (pos < a.b.V)
+      a.b.hi[s.gh & 1][pos] = v;
+    else
+      atomicOr(a.err, DEV_ERR_OVERFLOW);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) m.n_hi = 0;
+}
+
+struct BqMeshMarks {
+  int32_t lo_tag, hi_tag, next_tag, mark_lo, mark_hi;
+};
+
+// Relaxes the n vertices of near_[in]: improvements below U to near_[in ^ 1]
+// (count *n_out, the queue q when that is full), the others parked.  Four lanes
+// share a vertex, an edge each, J vertices of a lane in flight.
+template <int J>
+__device__ __forceinline__ void mesh_relax_pass(const BqLoop &s, const BqArgs &a, int32_t *sctl, BqMeshSmem &m,
+                                                const BqMeshMarks &mk, int32_t n, int32_t in, int32_t L, int32_t U,
+                                                int32_t *n_out, int32_t *q) {
+  const int32_t per = blockDim.x >> 2, lane = threadIdx.x & 31, lo_next = (s.g + 1) & 1;
+  int32_t *cnt = lane == 0 ? n_out : (lane == 1 ? &m.n_lo[L] : &m.n_hi);
+  // a warp without a vertex leaves at once: in a round of a few vertices the
+  // others' empty instructions would cost more than the loads
+  for (int32_t w0 = (threadIdx.x & ~31) >> 2; w0 < n; w0 += J * per) {
+    bool more = true;
+    for (int32_t hop = threadIdx.x & 3; more; hop += 4) {
+      int32_t d[J], np[J], prev[J], st[J], db[J], de[J];
+      more = false;
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const int32_t i = w0 + (lane >> 2) + j * per;
+        const int4 x = i < n ? m.near_[in][i] : make_int4(0, 0, 0, 0);
+        const int32_t k = x.z + hop;
+        const bool ok = k < x.w;
+        d[j] = ok ? __ldg(a.g.dst + k) : -1;
+        np[j] = ok ? x.y + __ldg(a.g.w + k) : INT_MAX;
+        more |= k + 4 < x.w;
+      }
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const bool ok = d[j] >= 0;
+        prev[j] = ok ? __ldcg(a.dist + d[j]) : INT_MIN;
+        st[j] = ok ? __ldcg(a.b.stamp + d[j]) : 0;
+        db[j] = ok ? __ldg(a.g.off + d[j]) : 0;
+        de[j] = ok ? __ldg(a.g.off + d[j] + 1) : 0;
+      }
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const int32_t v = d[j], p = np[j];
+        int32_t to = -1;  // 0 frontier, 1 low pile, 2 high pile
+        if (p < prev[j]) {
+          asm volatile("red.relaxed.gpu.global.min.s32 [%0], %1;" ::"l"(__cvta_generic_to_global(a.dist + v)), "r"(p)
+                       : "memory");
+          if (p < U)
+            to = 0;
+          else if (p < s.hz)
+            to = st[j] == mk.lo_tag || st[j] == mk.mark_lo || st[j] == mk.next_tag ? -1 : 1;
+          else
+            to = st[j] == mk.hi_tag || st[j] == mk.mark_hi ? -1 : 2;
+        }
+        const int32_t pos = mesh_places(to, cnt);
+        if (to == 0) {
+          if (pos < kMeshNear) {
+            m.near_[in ^ 1][pos] = make_int4(v, p, db[j], de[j]);
+          } else {
+            m.full = 1;
+            const int32_t qp = atomicAdd(&m.spill, 1);
+            if (qp < a.qcap)
+              q[qp] = v;
+            else
+              atomicOr(a.err, DEV_ERR_OVERFLOW);
+          }
+        } else if (to == 1) {
+          if (pos < kMeshLow) {
+            a.b.stamp[v] = mk.mark_lo;
+            m.lo[L][pos] = make_int4(v, p, db[j], de[j]);
+          } else {
+            m.full = 1;
+            if (atomicExch(a.b.stamp + v, mk.next_tag) != mk.next_tag) {
+              const int32_t gp = atomicAdd(sctl + BQ_LO + lo_next, 1);
+              if (gp < a.b.V)
+                a.b.lo[lo_next][gp] = v;
+              else
+                atomicOr(a.err, DEV_ERR_OVERFLOW);
+            }
+          }
+        } else if (to == 2) {
+          if (pos < kMeshHigh) {
+            a.b.stamp[v] = mk.mark_hi;
+            m.hi[pos] = v;
+          } else if (atomicExch(a.b.stamp + v, mk.hi_tag) != mk.hi_tag) {
+            const int32_t gp = atomicAdd(sctl + BQ_HI + (s.gh & 1), 1);
+            if (gp < a.b.V)
+              a.b.hi[s.gh & 1][gp] = v;
+            else
+              atomicOr(a.err, DEV_ERR_OVERFLOW);
+          }
+        }
+      }
+      more = __any_sync(0xffffffffu, more);
+    }
+  }
+}
+
+// Runs relaxes and advances while they fit; `session` numbers the sessions of
+// the run (its marks).  On return the loop state and control words are as after
+// a bq_step, ready for bq_decide.
+__device__ __forceinline__ void bq_mesh_session(BqLoop &s, const BqArgs &a, int32_t *sctl, BqMeshSmem &m,
+                                                int32_t session, int32_t n, uint64_t t0) {
+  const int32_t mark_lo = -2 * session - 1, mark_hi = -2 * session - 2;  // below every pile tag
+  const int32_t lo_tag = bq_lo_tag(s.g), hi_tag = bq_hi_tag(s.gh), next_tag = bq_lo_tag(s.g + 1);
+  const int32_t lo_next = (s.g + 1) & 1, T = blockDim.x, lane = threadIdx.x & 31;
+  int32_t *const q = s.in ? a.q1 : a.q0;
+  int32_t nl = sctl[BQ_LO + (s.g & 1)];
+  for (int32_t i = threadIdx.x; i < n; i += T) {
+    const int32_t v = __ldcg(q + i);
+    m.near_[0][i] = make_int4(v, __ldcg(a.dist + v), __ldg(a.g.off + v), __ldg(a.g.off + v + 1));
+  }
+  for (int32_t i = threadIdx.x; i < nl; i += T) {
+    const int32_t v = __ldcg(a.b.lo[s.g & 1] + i);
+    m.lo[0][i] = make_int4(v, 0, __ldg(a.g.off + v), __ldg(a.g.off + v + 1));
+  }
+  __syncthreads();  // nl is read by every thread before it changes
+  if (threadIdx.x == 0) {
+    m.n_near[0] = m.n_near[1] = 0;
+    m.n_lo[0] = nl;
+    m.n_hi = 0;
+    m.spill = m.full = m.quit = 0;
+    m.min3[0] = m.min3[1] = m.min3[2] = INT_MAX;
+    sctl[BQ_LO + lo_next] = 0;  // low parks that do not fit, then the write-back
+  }
+  int32_t in = 0, L = 0, adv = 0, cross = INT_MAX;
+  for (int32_t round = 1;; ++round) {
+    __syncthreads();
+    const int32_t U = bq_clamp((int64_t)s.cur + a.delta);
+    if (n > 0) {
+      // ---- relax: near_[in] -> near_[in ^ 1], lo[L], hi
+      int32_t *n_out = &m.n_near[in ^ 1];
+      const BqMeshMarks mk{lo_tag, hi_tag, next_tag, mark_lo, mark_hi};
+      // a second vertex per lane only where the frontier has that many
+      if (n <= T >> 2)
+        mesh_relax_pass<1>(s, a, sctl, m, mk, n, in, L, U, n_out, q);
+      else
+        mesh_relax_pass<2>(s, a, sctl, m, mk, n, in, L, U, n_out, q);
+      s.relax++;
+      if (threadIdx.x == 0 && (round & 15) == 0)  // the session's time slice, and overflows
+        m.quit = globaltimer_ns() - t0 > kSoloSliceNs || (*(volatile int32_t *)a.err & DEV_ERR_OVERFLOW) != 0;
+      __syncthreads();
+      in ^= 1;
+      n = min(m.n_near[in], kMeshNear);
+      const bool leave = m.full || m.quit;
+      const bool flush = m.n_hi > kMeshHigh / 2;
+      __syncthreads();
+      if (threadIdx.x == 0) m.n_near[in ^ 1] = 0;
+      if (flush) mesh_flush_high(s, a, sctl, m, mark_lo);
+      if (leave) break;
+    } else {
+      // ---- advance: the exact minimum of the live entries, then the split
+      nl = min(m.n_lo[L], kMeshLow);
+      int32_t mn = INT_MAX;
+      constexpr int kIn = 4;  // priorities a thread reads at once
+      for (int32_t i0 = threadIdx.x; i0 < nl; i0 += kIn * T) {
+        int32_t p[kIn];
+#pragma unroll
+        for (int j = 0; j < kIn; ++j) p[j] = i0 + j * T < nl ? __ldcg(a.dist + m.lo[L][i0 + j * T].x) : -1;
+#pragma unroll
+        for (int j = 0; j < kIn; ++j) {
+          if (i0 + j * T < nl) m.lo[L][i0 + j * T].y = p[j];
+          if (p[j] >= U) mn = min(mn, p[j]);
+        }
+      }
+      mn = __reduce_min_sync(0xffffffffu, mn);
+      if ((threadIdx.x & 31) == 0 && mn != INT_MAX) atomicMin(&m.min3[adv % 3], mn);
+      __syncthreads();
+      mn = m.min3[adv % 3];
+      if (threadIdx.x == 0) {
+        m.min3[(adv + 1) % 3] = INT_MAX;
+        m.n_lo[L ^ 1] = 0;
+        if (mn == INT_MAX) m.n_lo[L] = 0;  // nothing live below the horizon: a refill is next
+      }
+      __syncthreads();
+      if (mn == INT_MAX) break;
+      if (bq_clamp((int64_t)mn + a.delta) > s.hz) {  // the window reaches the high pile: bq_step's split
+        cross = mn;
+        break;
+      }
+      const int32_t win = bq_clamp((int64_t)mn + a.delta);
+      int32_t *cnt = lane == 0 ? &m.n_near[in] : &m.n_lo[L ^ 1];
+      for (int32_t i0 = 0; i0 < nl; i0 += T) {
+        const int32_t i = i0 + threadIdx.x;
+        const int4 x = i < nl ? m.lo[L][i] : make_int4(0, -1, 0, 0);
+        const int32_t to = x.y < U ? -1 : (x.y < win ? 0 : 1);  // below U: settled since it was parked
+        const int32_t pos = mesh_places(to, cnt);
+        if (to == 1) m.lo[L ^ 1][pos] = x;
+        if (to == 0) {
+          if (pos < kMeshNear) {
+            m.near_[in][pos] = x;
+          } else {
+            m.full = 1;
+            const int32_t qp = atomicAdd(&m.spill, 1);
+            if (qp < a.qcap)
+              q[qp] = x.x;
+            else
+              atomicOr(a.err, DEV_ERR_OVERFLOW);
+          }
+        }
+      }
+      L ^= 1;
+      s.cur = mn;
+      s.adv++;
+      adv++;
+      __syncthreads();
+      n = min(m.n_near[in], kMeshNear);
+      if (m.full) break;
+    }
+  }
+  // ---- back to the queues and piles in global memory, a vertex once per pile
+  __syncthreads();
+  mesh_flush_high(s, a, sctl, m, mark_lo);
+  nl = min(m.n_lo[L], kMeshLow);
+  for (int32_t i = threadIdx.x; i < nl; i += T) {
+    const int32_t v = m.lo[L][i].x;
+    if (atomicExch(a.b.stamp + v, next_tag) == next_tag) continue;
+    const int32_t pos = agg_inc(sctl + BQ_LO + lo_next);
+    if (pos < a.b.V)
+      a.b.lo[lo_next][pos] = v;
+    else
+      atomicOr(a.err, DEV_ERR_OVERFLOW);
+  }
+  const int32_t sp = (int32_t)min((int64_t)m.spill, a.qcap);
+  for (int32_t i = threadIdx.x; i < n; i += T) {
+    if (sp + i < a.qcap)
+      q[sp + i] = m.near_[in][i].x;
+    else
+      atomicOr(a.err, DEV_ERR_OVERFLOW);
+  }
+  s.g++;
+  s.phase = 0;
+  s.hub = 0;
+  if (cross != INT_MAX) {  // as after a lo-min that found it
+    s.phase = 1;
+    s.adv++;
+  }
+  if (threadIdx.x == 0) {
+    sctl[BQ_NEAR + (s.it + 2) % 3] = sp + n;
+    sctl[BQ_NEAR + s.it % 3] = sctl[BQ_NEAR + (s.it + 1) % 3] = 0;
+    sctl[BQ_MIN + (s.it + 2) % 3] = cross;
+    sctl[BQ_MIN + s.it % 3] = sctl[BQ_MIN + (s.it + 1) % 3] = INT_MAX;
+    sctl[BQ_HUB] = sctl[BQ_HUB + 1] = sctl[BQ_HUB + 2] = 0;
+    if (cross != INT_MAX) {  // what a lo-min clears for the next generations
+      sctl[BQ_LO + ((s.g + 1) & 1)] = 0;
+      sctl[BQ_HI + ((s.gh + 1) & 1)] = 0;
+      sctl[BQ_FILL + ((s.gh + 1) & 1)] = 0;
+    }
+  }
+  __syncthreads();
 }
 
 }  // namespace gg

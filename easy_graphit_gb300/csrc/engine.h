@@ -217,6 +217,8 @@ bool fused_supported(const gg_schedule *s);
 // loop, every step on the device (capturable); sources in device memory.
 // SSSP uses the bucket-queue buffers *bq; *stats receives the device address of
 // the run's {iterations, bucket advances}.
+// fused_multi_setup first, outside any capture, for SSSP.
+gg_status fused_multi_setup(gg_graph *g);
 gg_status fused_multi_enqueue(gg_graph *g, cudaStream_t st, bool sssp, const int32_t *dsrc, int32_t n,
                               int32_t delta, int32_t *parent, int32_t *out, const BqBuffers *bq,
                               const int32_t **stats);

@@ -11,6 +11,7 @@
 
 #include <cstdlib>
 
+#include "batch.h"
 #include "bq_loop.cuh"
 #include "bucket_queue.cuh"
 #include "engine.h"
@@ -157,20 +158,29 @@ __device__ __forceinline__ void bq_publish(const BqLoop &s, int32_t *ctl) {
 // global memory at its end.  The whole CTA calls it.
 template <int LB>
 __device__ __forceinline__ void bq_solo(BqLoop &s, const BqArgs &a, BqStep st, int4 *smem, int32_t *red,
-                                        int32_t *flag, int32_t *sctl) {
+                                        int32_t *flag, int32_t *sctl, int32_t *session) {
   for (int i = threadIdx.x; i < BQ_STOP; i += blockDim.x) sctl[i] = __ldcg(a.b.ctl + i);
   uint64_t t0 = 0;
   if (threadIdx.x == 0) t0 = globaltimer_ns();
   __syncthreads();
-  for (;;) {
-    bq_step<LB>(s, a, st, sctl, 0, 1, smem, red);
-    __syncthreads();
-    if (threadIdx.x == 0)
-      *flag = (*(volatile int32_t *)a.err & DEV_ERR_OVERFLOW) != 0 || globaltimer_ns() - t0 > kSoloSliceNs;
-    __syncthreads();
-    const bool quit = *flag != 0;
-    __syncthreads();
-    if (quit) break;
+  for (int32_t steps = 1;; ++steps) {
+    const int32_t near_n = st.kind == BQ_RELAX ? st.work : 0;
+    if (a.mesh && (st.kind == BQ_RELAX || st.kind == BQ_LOMIN) && near_n <= kMeshNear / 4 * 3 &&
+        sctl[BQ_LO + (s.g & 1)] <= kMeshLow) {
+      bq_mesh_session(s, a, sctl, *reinterpret_cast<BqMeshSmem *>(smem), ++*session, near_n, t0);
+      steps |= 7;  // long enough to check the clock
+    } else {
+      bq_step<LB>(s, a, st, sctl, 0, 1, smem, red);
+      __syncthreads();
+    }
+    if ((steps & 7) == 7) {  // a read of the error word is a round trip
+      if (threadIdx.x == 0)
+        *flag = (*(volatile int32_t *)a.err & DEV_ERR_OVERFLOW) != 0 || globaltimer_ns() - t0 > kSoloSliceNs;
+      __syncthreads();
+      const bool quit = *flag != 0;
+      __syncthreads();
+      if (quit) break;
+    }
     st = bq_decide(s, sctl, a.delta);
     if (st.kind == BQ_DONE || !bq_small(st, a)) break;
   }
@@ -186,6 +196,7 @@ __global__ void __launch_bounds__(1024) k_sssp_bq(BqArgs a) {
   __shared__ int32_t sctl[BQ_STOP];  // counts and minima of a one-CTA session
   BqLoop s{1, 0, 0, 0, 0, bq_clamp((int64_t)a.width0 * a.delta), a.width0, 0, 0, 0, 0};
   int32_t *stop = a.b.ctl + BQ_STOP;
+  int32_t session = 0;  // mesh sessions run (CTA 0)
   LoopClock clk;
   clk.start(a.loop_limit_ns);
   // Grid iterations (one barrier each), numbered for the stop word: the clock
@@ -202,7 +213,7 @@ __global__ void __launch_bounds__(1024) k_sssp_bq(BqArgs a) {
       // has taken its decision from them and arrived at the barrier.
       if (blockIdx.x == 0) {
         if (grid_wait_others(a.bar, gridDim.x, a.err, a.timeout_ns))
-          bq_solo<LB>(s, a, st, smem, red, red + 32, sctl);
+          bq_solo<LB>(s, a, st, smem, red, red + 32, sctl, &session);
         else
           bq_publish(s, a.b.ctl);
       }
@@ -710,6 +721,11 @@ static int32_t bq_solo_per_thread() {
   return env >= 0 ? (int32_t)env : 4;
 }
 
+// Shared memory of the SSSP loop: the strategy's, or a mesh session's.
+static size_t bq_smem(int lb, int cta, bool mesh) {
+  return mesh ? std::max(lb_smem(lb, cta), sizeof(BqMeshSmem)) : lb_smem(lb, cta);
+}
+
 static BqArgs bq_args(gg_graph *g, gg_frontier *f, const BqBuffers &b, int32_t *dist, int32_t delta, int cta) {
   BqArgs a{};
   a.g = g->csr.view();
@@ -726,11 +742,15 @@ static BqArgs bq_args(gg_graph *g, gg_frontier *f, const BqBuffers &b, int32_t *
   a.delta = delta;
   a.solo_max = bq_solo_per_thread() * cta;
   a.solo_pile_max = 8 * a.solo_max;
-  a.fill_target = 1024;
   a.width0 = 16;
   a.hub_list = static_cast<int32_t *>(g->hubs.p);
   a.hub_cap = hub_capacity(g);
   a.hub_min = kHubWidths * cta;
+  a.mesh = g->max_degree >= 0 && g->max_degree <= kMeshMaxDegree && a.solo_max > 0;
+  // Low-pile entries of a refill.  A mesh session reads them at every advance
+  // (2048^2 grid, delta 8: 1123 ms with 2,048, 580 with 1,024, 398 with 512); the
+  // other form pays more for a refill.
+  a.fill_target = a.mesh ? 512 : 1024;
   return a;
 }
 
@@ -740,9 +760,11 @@ gg_status fused_sssp(gg_graph *g, const gg_schedule *s, int32_t n0, int32_t delt
   if (!fused_supported(s)) return GG_OK;
   const int cta = s->cta_size;
   GG_TRY(ensure_hubs(g));
+  int32_t max_degree = 0;
+  GG_TRY(graph_max_degree(g, &max_degree));  // kept with the graph
   GG_TRY(bq_start(pq->bq, n0, g->stream));
   BqArgs a = bq_args(g, pq->frontier, pq->bq, vd.dist, delta, cta);
-  const size_t sm = lb_smem(s->load_balancing, cta);
+  const size_t sm = bq_smem(s->load_balancing, cta, a.mesh);
   switch (s->load_balancing) {
     case GG_LB_VERTEX_BASED: GG_TRY(coop_launch(g, k_sssp_bq<GG_LB_VERTEX_BASED>, cta, sm, a)); break;
     case GG_LB_WM: GG_TRY(coop_launch(g, k_sssp_bq<GG_LB_WM>, cta, sm, a)); break;
@@ -798,6 +820,15 @@ __global__ void k_multi_seed(VData vd, int32_t sssp, const int32_t *__restrict__
   }
 }
 
+gg_status fused_multi_setup(gg_graph *g) {
+  int32_t max_degree = 0;
+  GG_TRY(graph_max_degree(g, &max_degree));
+  if (max_degree <= kMeshMaxDegree)
+    GG_CUDA(cudaFuncSetAttribute(k_sssp_bq<GG_LB_TWCE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)bq_smem(GG_LB_TWCE, 512, true)));
+  return GG_OK;
+}
+
 gg_status fused_multi_enqueue(gg_graph *g, cudaStream_t st, bool sssp, const int32_t *dsrc, int32_t n,
                               int32_t delta, int32_t *parent, int32_t *out, const BqBuffers *bq,
                               const int32_t **stats) {
@@ -815,7 +846,8 @@ gg_status fused_multi_enqueue(gg_graph *g, cudaStream_t st, bool sssp, const int
   const int cta = 512;
   FusedArgs a = make_args(g, f, vd, cta);
   a.delta = delta;
-  const size_t smem = twce_smem_bytes(cta);
+  const bool mesh = sssp && g->max_degree >= 0 && g->max_degree <= kMeshMaxDegree;
+  const size_t smem = sssp ? bq_smem(GG_LB_TWCE, cta, mesh) : twce_smem_bytes(cta);
   const void *kernel = sssp ? (const void *)k_sssp_bq<GG_LB_TWCE> : (const void *)k_bfs_fused<GG_LB_TWCE>;
   int per_sm = 0;
   GG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, cta, smem));
