@@ -4,6 +4,8 @@
 // Unfused loops read the frontier size once per iteration, as the generated
 // host code does (vertex_frontier.h:109-113); fuse=1 with a simple schedule
 // runs the BFS/SSSP loop in one persistent kernel (fused.cu).
+#include <cstring>
+#include <initializer_list>
 #include <vector>
 
 #include "engine.h"
@@ -64,6 +66,51 @@ __global__ void k_reach(const int32_t *__restrict__ val, const int32_t *__restri
     atomicAdd(out, r);
     atomicAdd(out + 1, e);
   }
+}
+
+// The end of a fused single-source trial, in one launch: the reached vertices and
+// their out-degrees (val null: not wanted), then -- by the last block -- these
+// sums, the loop's counters and the status word into pinned host memory.  The sums
+// start at zero and are left there.
+__global__ void k_trial_end(const int32_t *__restrict__ val, const int32_t *__restrict__ off, int32_t V,
+                            const int32_t *__restrict__ stats, const int32_t *__restrict__ err,
+                            unsigned long long *sums, TrialOut *out) {
+  unsigned long long r = 0, e = 0;
+  if (val)
+    for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
+      const int32_t x = val[v];
+      if (x >= 0 && x != INT_MAX) {
+        ++r;
+        e += off[v + 1] - off[v];
+      }
+    }
+  for (int d = 16; d > 0; d >>= 1) {
+    r += __shfl_xor_sync(0xffffffffu, r, d);
+    e += __shfl_xor_sync(0xffffffffu, e, d);
+  }
+  __shared__ unsigned long long s_r[32], s_e[32];
+  if ((threadIdx.x & 31) == 0) {
+    s_r[threadIdx.x >> 5] = r;
+    s_e[threadIdx.x >> 5] = e;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (uint32_t w = 1; w < blockDim.x >> 5; ++w) {
+    r += s_r[w];
+    e += s_e[w];
+  }
+  if (r) {
+    atomicAdd(sums, r);
+    atomicAdd(sums + 1, e);
+  }
+  __threadfence();
+  if (atomicAdd(sums + 2, 1ull) != gridDim.x - 1) return;
+  out->reached = atomicExch(sums, 0ull);
+  out->edges = atomicExch(sums + 1, 0ull);
+  out->stats[0] = stats[0];
+  out->stats[1] = stats[1];
+  out->err = *(const volatile int32_t *)err;
+  sums[2] = 0ull;
 }
 
 __global__ void k_sigma_to_reach(const double *__restrict__ sigma, int32_t V, int32_t *__restrict__ o) {
@@ -139,6 +186,60 @@ struct Trial {
     return GG_OK;
   }
 };
+
+// Ends a fused single-source trial whose results are still on the device: the
+// events, k_trial_end, the results copied out, one synchronisation.  `outs` are
+// pairs of host-or-device destinations (null: not wanted) and device arrays of V
+// ints.
+struct TrialCopy {
+  int32_t *to;
+  const int32_t *from;
+};
+gg_status end_trial(Trial &t, const char *what, const int32_t *val, const int32_t *stats, gg_stats *st,
+                    std::initializer_list<TrialCopy> outs) {
+  gg_graph *g = t.g;
+  cudaStream_t s = g->stream;
+  const int32_t V = g->csr.V;
+  const size_t bytes = sizeof(int32_t) * (size_t)V;
+  GG_CUDA(cudaEventRecord(g->ev1, s));
+  const int32_t launched = (int32_t)(launches() - t.l0);
+  note_launch();
+  k_trial_end<<<std::max(1, std::min(ceil_div(V, 256), g->sm_count * 4)), 256, 0, s>>>(
+      st ? val : nullptr, g->csr.off, V, stats, g->d_err, reinterpret_cast<unsigned long long *>(g->d_misc + 64),
+      g->h_out);
+  GG_CUDA(cudaGetLastError());
+  // Small results for pageable memory go through the graph's pinned buffer: a
+  // pageable copy of a few KB is staged and waited for by the driver, one by one.
+  size_t staged = 0;
+  struct {
+    void *to;
+    size_t at;
+  } later[2];
+  int nlater = 0;
+  for (const TrialCopy &o : outs) {
+    if (!o.to) continue;
+    cudaPointerAttributes pa{};
+    const bool pageable = bytes <= kStageBytes - staged && nlater < 2 &&
+                          cudaPointerGetAttributes(&pa, o.to) == cudaSuccess && pa.type == cudaMemoryTypeUnregistered;
+    if (pageable) {
+      GG_CUDA(cudaMemcpyAsync((char *)g->h_stage + staged, o.from, bytes, cudaMemcpyDeviceToHost, s));
+      later[nlater++] = {o.to, staged};
+      staged += bytes;
+    } else {
+      GG_CUDA(cudaMemcpyAsync(o.to, o.from, bytes, cudaMemcpyDefault, s));
+    }
+  }
+  GG_CUDA(cudaStreamSynchronize(s));
+  for (int i = 0; i < nlater; ++i) memcpy(later[i].to, (char *)g->h_stage + later[i].at, bytes);
+  if (st) {
+    GG_CUDA(cudaEventElapsedTime(&st->device_ms, g->ev0, g->ev1));
+    if (g->loop_timed) GG_CUDA(cudaEventElapsedTime(&st->loop_ms, g->ev2, g->ev3));
+    st->launches = launched;
+    st->vertices_reached = (int64_t)g->h_out->reached;
+    st->edges_traversed = (int64_t)g->h_out->edges;
+  }
+  return device_error(g, g->h_out->err, what);
+}
 
 // Brackets an unfused traversal loop with ev2/ev3.
 struct LoopTimer {
@@ -236,6 +337,30 @@ static bool bfs_do_plan(const gg_app_schedule *s, BfsDoPlan *p) {
     return true;
   }
   return false;
+}
+
+// A single-source BFS in one fused loop, launched only (end_trial reads its
+// results); false when the schedule has no fused form.
+gg_status launch_bfs_single(gg_graph *g, const gg_app_schedule *s, int32_t src, int32_t *parent, int32_t *depth,
+                            bool *ran) {
+  *ran = false;
+  BfsDoPlan dp;
+  const bool simple = s->fuse && s->kind == GG_SCHED_SIMPLE && fused_supported(&s->s1);
+  if (!simple && !(s->fuse && bfs_do_plan(s, &dp))) return GG_OK;
+  gg_frontier *f = nullptr;
+  GG_TRY(app_frontier(g, &f));
+  VData vd{};
+  vd.parent = parent;
+  vd.depth = depth;
+  vd.src = src;
+  GG_TRY(fused_setup(g, vd, f, src, nullptr, !simple));
+  if (simple) {
+    GG_TRY(fused_bfs(g, &s->s1, 1, vd, f, nullptr, ran));
+  } else {
+    GG_TRY(fused_bfs_do(g, dp, 1, vd, f, nullptr, nullptr));
+    *ran = true;
+  }
+  return GG_OK;
 }
 
 gg_status run_bfs(gg_graph *g, const gg_app_schedule *s, const int32_t *srcs, int32_t nsrc,
@@ -360,6 +485,18 @@ gg_status gg_bfs(gg_graph *g, const gg_app_schedule *s, int32_t src, int32_t *de
   GG_TRY(app_array(g, 0, V, &parent));
   GG_TRY(app_array(g, 1, V, &depth));
   Trial t(g);
+  bool ran = false;
+  GG_TRY(launch_bfs_single(g, s, src, parent, depth, &ran));
+  if (ran) {
+    GG_TRY(end_trial(t, "bfs", depth, g->d_misc + 44, st, {{depth_out, depth}, {parent_out, parent}}));
+    if (st) {
+      st->iterations = g->h_out->stats[0];
+      st->pull_iterations = s->kind == GG_SCHED_SIMPLE ? 0 : g->h_out->stats[1];
+      st->push_iterations = st->iterations - st->pull_iterations;
+      st->fused = 1;
+    }
+    return GG_OK;
+  }
   GG_TRY(run_bfs(g, s, &src, 1, parent, depth, st));
   GG_TRY(t.stop(st));
   if (depth_out) GG_CUDA(cudaMemcpyAsync(depth_out, depth, sizeof(int32_t) * V, cudaMemcpyDefault, g->stream));
@@ -448,6 +585,27 @@ gg_status gg_sssp(gg_graph *g, const gg_app_schedule *s, int32_t src, int32_t de
   int32_t *dist = nullptr;
   GG_TRY(app_array(g, 2, V, &dist));
   Trial t(g);
+  if (s->fuse && s->kind == GG_SCHED_SIMPLE && fused_supported(&s->s1)) {
+    if (!g->app_pq) GG_TRY(gg_pq_create(g, dist, 0, delta, src, &g->app_pq));
+    gg_pq *pq = g->app_pq;
+    pq->prio = dist;
+    pq_reset_host(pq, 0, delta);
+    VData vd{};
+    vd.dist = dist;
+    vd.src = src;
+    bool ran = false;
+    GG_TRY(fused_setup(g, vd, pq->frontier, src, &pq->bq, false));
+    GG_TRY(fused_sssp(g, &s->s1, 1, delta, vd, pq, nullptr, nullptr, &ran));
+    if (ran) {
+      GG_TRY(end_trial(t, "sssp", dist, pq->bq.ctl + BQ_STATS, st, {{dist_out, dist}}));
+      if (st) {
+        st->iterations = st->push_iterations = g->h_out->stats[0];
+        st->bucket_advances = g->h_out->stats[1];
+        st->fused = 1;
+      }
+      return GG_OK;
+    }
+  }
   GG_TRY(run_sssp(g, s, &src, 1, delta, dist, st));
   GG_TRY(t.stop(st));
   if (dist_out) GG_CUDA(cudaMemcpyAsync(dist_out, dist, sizeof(int32_t) * V, cudaMemcpyDefault, g->stream));

@@ -39,6 +39,18 @@ struct Scratch {
 
 }  // namespace gg
 
+namespace gg {
+// What a single-source fused trial leaves for the host, in pinned memory that
+// its last kernel writes (k_trial_end, apps.cu).
+struct TrialOut {
+  unsigned long long reached, edges;  // vertices reached, their out-degrees
+  int32_t stats[2];                   // the loop's counters
+  int32_t err;                        // device status word
+};
+constexpr int32_t kPinnedInts = 64;         // h_pinned: small copies
+constexpr size_t kStageBytes = 60 * 1024;   // h_stage: results up to this size
+}  // namespace gg
+
 struct gg_graph {
   gg::GraphStore csr;                        // forward CSR (+ COO src)
   std::unique_ptr<gg::GraphStore> csc;       // get_transposed_graph()
@@ -49,8 +61,10 @@ struct gg_graph {
   cudaStream_t own_stream = nullptr;
   int32_t *d_err = nullptr;       // device status word (DEV_ERR_*)
   uint32_t *d_bar = nullptr;      // grid barrier arrivals (one 64-bit count)
-  int32_t *d_misc = nullptr;      // small device scratch (counters, flags), 64 ints
-  int32_t *h_pinned = nullptr;    // pinned host scratch, 64 ints
+  int32_t *d_misc = nullptr;      // small device scratch (counters, flags), 64 ints, and k_trial_end's sums
+  int32_t *h_pinned = nullptr;    // pinned host scratch, kPinnedInts; the two below share its allocation
+  gg::TrialOut *h_out = nullptr;
+  void *h_stage = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // whole trial
   cudaEvent_t ev2 = nullptr, ev3 = nullptr;  // traversal loop
   bool loop_timed = false;                   // ev2/ev3 bracket the last loop
@@ -142,6 +156,7 @@ gg_status ensure_blocked(gg_graph *g, bool reverse, int32_t block_size, const Gr
 int32_t hub_capacity(const gg_graph *g);
 gg_status ensure_hubs(gg_graph *g);
 gg_status check_device_error(gg_graph *g, const char *what);
+gg_status device_error(gg_graph *g, int32_t e, const char *what);  // the same for a status word already read
 gg_status scratch_get(gg_graph *g, int slot, size_t bytes, void **p);
 gg_status scratch_get_app(gg_graph *g, int slot, size_t bytes, void **p);
 // stats->vertices_reached / edges_traversed of a result array (reached: >= 0
@@ -206,6 +221,7 @@ gg_status vertexset_apply_impl(gg_graph *g, gg_frontier *set, int32_t vudf, cons
 gg_status pq_finished(gg_pq *pq, bool *fin);
 gg_status pq_dequeue(gg_pq *pq);
 gg_status pq_reset(gg_pq *pq, int32_t init_priority, int32_t delta, int32_t src);
+void pq_reset_host(gg_pq *pq, int32_t init_priority, int32_t delta);  // its host state alone
 int32_t pq_cutoff(const gg_pq *pq);
 DFar pq_far(const gg_pq *pq);  // far piles the relax parks into
 
@@ -222,6 +238,9 @@ gg_status fused_multi_setup(gg_graph *g);
 gg_status fused_multi_enqueue(gg_graph *g, cudaStream_t st, bool sssp, const int32_t *dsrc, int32_t n,
                               int32_t delta, int32_t *parent, int32_t *out, const BqBuffers *bq,
                               const int32_t **stats);
+// With iters (pulls, advances) null the loop's counters and control words were
+// set by fused_setup and its results are left for the trial's end: launches only.
+gg_status fused_setup(gg_graph *g, const VData &vd, gg_frontier *f, int32_t src, const BqBuffers *bq, bool lstat);
 gg_status fused_bfs(gg_graph *g, const gg_schedule *s, int32_t n0, const VData &vd,
                     gg_frontier *f, int32_t *iters, bool *ran);
 // Direction-optimising fused BFS (fused.cu k_bfs_do): each level pushes with

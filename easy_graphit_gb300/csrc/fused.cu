@@ -257,14 +257,18 @@ gg_status bq_start(const BqBuffers &b, int32_t n0, cudaStream_t st) {
 }
 
 template <class K, class A, class... More>
-static gg_status coop_launch(gg_graph *g, K kernel, int cta, size_t smem, A &a, More &...more) {
+static gg_status coop_launch(gg_graph *g, bool prepared, K kernel, int cta, size_t smem, A &a, More &...more) {
   int per_sm = 0;
   if (smem > 48 * 1024)
     GG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   GG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, cta, smem));
   if (per_sm < 1) return set_error(GG_ERR_UNSUPPORTED, "fused kernel does not fit on an SM");
-  const int grid = per_sm * g->sm_count;
-  GG_CUDA(cudaMemsetAsync(g->d_bar, 0, sizeof(uint32_t) * 2, g->stream));
+  // A small graph takes fewer CTAs: 8 lanes for every vertex or a thread for
+  // every edge, whichever is more.  What the others would do is wait (a barrier of
+  // 41 CTAs takes 1.3 us, of 608 2.2).
+  const int64_t want = std::max(ceil_div((int64_t)g->csr.V * kStage1, cta), ceil_div((int64_t)g->csr.E, cta));
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(per_sm * g->sm_count, want));
+  if (!prepared) GG_CUDA(cudaMemsetAsync(g->d_bar, 0, sizeof(uint32_t) * 2, g->stream));
   void *args[] = {&a, &more...};
   GG_CUDA(cudaEventRecord(g->ev2, g->stream));
   note_launch();
@@ -329,22 +333,92 @@ static gg_status read_stats(gg_graph *g, int32_t *iters, int64_t *adv) {
   return GG_OK;
 }
 
+// Everything a single-source trial needs before its loop, in one launch: the
+// vertex data reset with the source's values, the frontier {src}, the loop's
+// counters, control words and barrier, the statistics of the first frontier.
+// Separate memsets, copies and kernels (seven to ten stream operations) cost a
+// small traversal more than its levels.
+struct SetupArgs {
+  VData vd;
+  int32_t *stamp, *ctl;          // SSSP
+  const int32_t *off;
+  int32_t *q, *cnt;              // frontier queue and its two counts
+  int32_t *misc;                 // d_misc + 40, as init_counts
+  uint32_t *bar;
+  unsigned long long *lstat;     // k_bfs_do's statistics, or null
+  int32_t V, src;
+};
+__global__ void k_fused_setup(SetupArgs a) {
+  for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.V; v += gridDim.x * blockDim.x) {
+    if (a.ctl) {
+      a.vd.dist[v] = v == a.src ? 0 : INT_MAX;
+      a.stamp[v] = 0;
+    } else {
+      a.vd.parent[v] = v == a.src ? v : -1;
+      a.vd.depth[v] = v == a.src ? 0 : -1;
+    }
+  }
+  if (blockIdx.x != 0) return;
+  const int32_t t = threadIdx.x;
+  if (t < 12) a.misc[t] = t == 0 ? 1 : (t == 6 || t == 7 ? INT_MAX : 0);
+  if (t < 2) {
+    a.bar[t] = 0;
+    a.cnt[t] = t == 0;
+  }
+  if (t == 0) a.q[0] = a.src;
+  if (a.ctl && t < BQ_CTL_INTS)
+    a.ctl[t] = t == BQ_NEAR ? 1 : (t >= BQ_MIN && t < BQ_MIN + 3 ? INT_MAX : (t == BQ_FILL ? -1 : 0));
+  if (a.lstat && t < 12) {
+    const unsigned long long k = (unsigned long long)(a.off[a.src + 1] - a.off[a.src]);
+    a.lstat[t] = t == 0 || t == 2 ? k : (t == 1 ? (unsigned long long)__double_as_longlong((double)k * (double)k) : 0ull);
+  }
+}
+
+gg_status fused_setup(gg_graph *g, const VData &vd, gg_frontier *f, int32_t src, const BqBuffers *bq, bool lstat) {
+  SetupArgs a{};
+  a.vd = vd;
+  if (bq) {
+    a.stamp = bq->stamp;
+    a.ctl = bq->ctl;
+  }
+  a.off = g->csr.off;
+  a.q = f->q_in;
+  a.cnt = f->cnt;
+  f->cnt_in = f->cnt;
+  f->cnt_out = f->cnt + 1;
+  a.misc = g->d_misc + 40;
+  a.bar = g->d_bar;
+  a.V = g->csr.V;
+  a.src = src;
+  if (lstat) {
+    void *ls = nullptr;
+    GG_TRY(scratch_get_app(g, 7, sizeof(unsigned long long) * 12, &ls));
+    a.lstat = static_cast<unsigned long long *>(ls);
+  }
+  f->fmt = GG_FMT_SPARSE;
+  note_launch();
+  k_fused_setup<<<std::max(1, std::min(ceil_div(a.V, 256), g->sm_count * 8)), 256, 0, g->stream>>>(a);
+  GG_CUDA(cudaGetLastError());
+  return GG_OK;
+}
+
 gg_status fused_bfs(gg_graph *g, const gg_schedule *s, int32_t n0, const VData &vd, gg_frontier *f,
                     int32_t *iters, bool *ran) {
   *ran = false;
   if (!fused_supported(s)) return GG_OK;
   GG_TRY(ensure_hubs(g));
-  GG_TRY(init_counts(g, n0));
+  const bool prepared = !iters;
+  if (!prepared) GG_TRY(init_counts(g, n0));
   const int cta = s->cta_size;
   FusedArgs a = make_args(g, f, vd, cta);
   const size_t sm = lb_smem(s->load_balancing, cta);
   switch (s->load_balancing) {
-    case GG_LB_VERTEX_BASED: GG_TRY(coop_launch(g, k_bfs_fused<GG_LB_VERTEX_BASED>, cta, sm, a)); break;
-    case GG_LB_WM: GG_TRY(coop_launch(g, k_bfs_fused<GG_LB_WM>, cta, sm, a)); break;
-    case GG_LB_TWCE: GG_TRY(coop_launch(g, k_bfs_fused<GG_LB_TWCE>, cta, sm, a)); break;
-    default: GG_TRY(coop_launch(g, k_bfs_fused<GG_LB_CM>, cta, sm, a)); break;
+    case GG_LB_VERTEX_BASED: GG_TRY(coop_launch(g, prepared, k_bfs_fused<GG_LB_VERTEX_BASED>, cta, sm, a)); break;
+    case GG_LB_WM: GG_TRY(coop_launch(g, prepared, k_bfs_fused<GG_LB_WM>, cta, sm, a)); break;
+    case GG_LB_TWCE: GG_TRY(coop_launch(g, prepared, k_bfs_fused<GG_LB_TWCE>, cta, sm, a)); break;
+    default: GG_TRY(coop_launch(g, prepared, k_bfs_fused<GG_LB_CM>, cta, sm, a)); break;
   }
-  GG_TRY(read_stats(g, iters, nullptr));
+  if (!prepared) GG_TRY(read_stats(g, iters, nullptr));
   *ran = true;
   return GG_OK;
 }
@@ -677,10 +751,13 @@ gg_status fused_bfs_do(gg_graph *g, const BfsDoPlan &p, int32_t n0, const VData 
   GG_TRY(ensure_hubs(g));
   void *ls = nullptr;
   GG_TRY(scratch_get_app(g, 7, sizeof(unsigned long long) * 12, &ls));
-  GG_TRY(init_counts(g, n0));
-  note_launch();
-  k_bfs_do_seed<<<1, 256, 0, g->stream>>>(f->q_in, n0, g->csr.off, static_cast<unsigned long long *>(ls));
-  GG_CUDA(cudaGetLastError());
+  const bool prepared = !iters;
+  if (!prepared) {
+    GG_TRY(init_counts(g, n0));
+    note_launch();
+    k_bfs_do_seed<<<1, 256, 0, g->stream>>>(f->q_in, n0, g->csr.off, static_cast<unsigned long long *>(ls));
+    GG_CUDA(cudaGetLastError());
+  }
   DoKernelArgs ka{};
   ka.a = make_args(g, f, vd, s->cta_size);
   ka.d.t = t->view();
@@ -698,11 +775,12 @@ gg_status fused_bfs_do(gg_graph *g, const BfsDoPlan &p, int32_t n0, const VData 
   uint32_t lbb = (uint32_t)lb_smem(s->load_balancing, cta);
   const size_t sm = p.mode == DO_SELECTOR ? do_lb_smem_aligned(lbb) + sizeof(float) * kSelectorParams : lbb;
   switch (s->load_balancing) {
-    case GG_LB_VERTEX_BASED: GG_TRY(coop_launch(g, k_bfs_do<GG_LB_VERTEX_BASED>, cta, sm, ka, lbb)); break;
-    case GG_LB_WM: GG_TRY(coop_launch(g, k_bfs_do<GG_LB_WM>, cta, sm, ka, lbb)); break;
-    case GG_LB_TWCE: GG_TRY(coop_launch(g, k_bfs_do<GG_LB_TWCE>, cta, sm, ka, lbb)); break;
-    default: GG_TRY(coop_launch(g, k_bfs_do<GG_LB_CM>, cta, sm, ka, lbb)); break;
+    case GG_LB_VERTEX_BASED: GG_TRY(coop_launch(g, prepared, k_bfs_do<GG_LB_VERTEX_BASED>, cta, sm, ka, lbb)); break;
+    case GG_LB_WM: GG_TRY(coop_launch(g, prepared, k_bfs_do<GG_LB_WM>, cta, sm, ka, lbb)); break;
+    case GG_LB_TWCE: GG_TRY(coop_launch(g, prepared, k_bfs_do<GG_LB_TWCE>, cta, sm, ka, lbb)); break;
+    default: GG_TRY(coop_launch(g, prepared, k_bfs_do<GG_LB_CM>, cta, sm, ka, lbb)); break;
   }
+  if (prepared) return GG_OK;
   int64_t np = 0;
   GG_TRY(read_stats(g, iters, &np));
   *pulls = (int32_t)np;
@@ -762,21 +840,23 @@ gg_status fused_sssp(gg_graph *g, const gg_schedule *s, int32_t n0, int32_t delt
   GG_TRY(ensure_hubs(g));
   int32_t max_degree = 0;
   GG_TRY(graph_max_degree(g, &max_degree));  // kept with the graph
-  GG_TRY(bq_start(pq->bq, n0, g->stream));
+  const bool prepared = !iters;
+  if (!prepared) GG_TRY(bq_start(pq->bq, n0, g->stream));
   BqArgs a = bq_args(g, pq->frontier, pq->bq, vd.dist, delta, cta);
   const size_t sm = bq_smem(s->load_balancing, cta, a.mesh);
   switch (s->load_balancing) {
-    case GG_LB_VERTEX_BASED: GG_TRY(coop_launch(g, k_sssp_bq<GG_LB_VERTEX_BASED>, cta, sm, a)); break;
-    case GG_LB_WM: GG_TRY(coop_launch(g, k_sssp_bq<GG_LB_WM>, cta, sm, a)); break;
-    case GG_LB_TWCE: GG_TRY(coop_launch(g, k_sssp_bq<GG_LB_TWCE>, cta, sm, a)); break;
-    default: GG_TRY(coop_launch(g, k_sssp_bq<GG_LB_CM>, cta, sm, a)); break;
+    case GG_LB_VERTEX_BASED: GG_TRY(coop_launch(g, prepared, k_sssp_bq<GG_LB_VERTEX_BASED>, cta, sm, a)); break;
+    case GG_LB_WM: GG_TRY(coop_launch(g, prepared, k_sssp_bq<GG_LB_WM>, cta, sm, a)); break;
+    case GG_LB_TWCE: GG_TRY(coop_launch(g, prepared, k_sssp_bq<GG_LB_TWCE>, cta, sm, a)); break;
+    default: GG_TRY(coop_launch(g, prepared, k_sssp_bq<GG_LB_CM>, cta, sm, a)); break;
   }
+  *ran = true;
+  if (prepared) return GG_OK;
   GG_CUDA(cudaMemcpyAsync(g->h_pinned + 50, pq->bq.ctl + BQ_STATS, sizeof(int32_t) * 2, cudaMemcpyDeviceToHost,
                           g->stream));
   GG_CUDA(cudaStreamSynchronize(g->stream));
   *iters = g->h_pinned[50];
   *advances = g->h_pinned[51];
-  *ran = true;
   return GG_OK;
 }
 

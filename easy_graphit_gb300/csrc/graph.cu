@@ -384,7 +384,10 @@ gg_status ensure_blocked(gg_graph *g, bool reverse, int32_t block_size, const Gr
 gg_status check_device_error(gg_graph *g, const char *what) {
   GG_CUDA(cudaMemcpyAsync(g->h_pinned + 63, g->d_err, sizeof(int32_t), cudaMemcpyDeviceToHost, g->stream));
   GG_CUDA(cudaStreamSynchronize(g->stream));
-  const int32_t e = g->h_pinned[63];
+  return device_error(g, g->h_pinned[63], what);
+}
+
+gg_status device_error(gg_graph *g, int32_t e, const char *what) {
   if (!e) return GG_OK;
   GG_CUDA(cudaMemsetAsync(g->d_err, 0, sizeof(int32_t), g->stream));
   if (e & DEV_ERR_TIMEOUT)
@@ -449,11 +452,13 @@ static gg_status graph_init(gg_graph *g, const int32_t *offsets, const int32_t *
   }
   GG_CUDA(dev_alloc(&g->d_err, sizeof(int32_t), st));
   GG_CUDA(dev_alloc(&g->d_bar, sizeof(uint32_t) * 2, st));
-  GG_CUDA(dev_alloc(&g->d_misc, sizeof(int32_t) * 64, st));
+  GG_CUDA(dev_alloc(&g->d_misc, sizeof(int32_t) * 128, st));
   GG_CUDA(cudaMemsetAsync(g->d_err, 0, sizeof(int32_t), st));
   GG_CUDA(cudaMemsetAsync(g->d_bar, 0, sizeof(uint32_t) * 2, st));
-  GG_CUDA(cudaMemsetAsync(g->d_misc, 0, sizeof(int32_t) * 64, st));
-  GG_CUDA(cudaMallocHost(&g->h_pinned, sizeof(int32_t) * 64));
+  GG_CUDA(cudaMemsetAsync(g->d_misc, 0, sizeof(int32_t) * 128, st));
+  GG_CUDA(cudaMallocHost(&g->h_pinned, sizeof(int32_t) * kPinnedInts + 256 + kStageBytes));
+  g->h_out = reinterpret_cast<TrialOut *>(g->h_pinned + kPinnedInts);
+  g->h_stage = reinterpret_cast<char *>(g->h_out) + 256;
   GG_CUDA(cudaEventCreate(&g->ev0));
   GG_CUDA(cudaEventCreate(&g->ev1));
   GG_CUDA(cudaEventCreate(&g->ev2));

@@ -177,7 +177,7 @@ gg_status pq_dequeue(gg_pq *pq) {
   return GG_OK;
 }
 
-gg_status pq_reset(gg_pq *pq, int32_t init_priority, int32_t delta, int32_t src) {
+void pq_reset_host(gg_pq *pq, int32_t init_priority, int32_t delta) {
   pq->cur = init_priority;
   pq->delta = delta;
   pq->window_upper = 0;
@@ -187,6 +187,11 @@ gg_status pq_reset(gg_pq *pq, int32_t init_priority, int32_t delta, int32_t src)
   pq->gen_hi = 0;
   pq->width = 16;
   pq->horizon = bq_clamp((int64_t)init_priority + (int64_t)pq->width * delta);
+  pq->frontier->fmt = GG_FMT_SPARSE;
+}
+
+gg_status pq_reset(gg_pq *pq, int32_t init_priority, int32_t delta, int32_t src) {
+  pq_reset_host(pq, init_priority, delta);
   gg_frontier *f = pq->frontier;
   gg_graph *g = pq->g;
   GG_TRY(bq_start(pq->bq, 0, g->stream));
@@ -196,7 +201,6 @@ gg_status pq_reset(gg_pq *pq, int32_t init_priority, int32_t delta, int32_t src)
   if (src >= 0) GG_CUDA(cudaMemcpyAsync(f->q_in, g->h_pinned + 7, sizeof(int32_t), cudaMemcpyHostToDevice, g->stream));
   GG_CUDA(cudaMemcpyAsync(f->cnt_in, g->h_pinned + 8, sizeof(int32_t), cudaMemcpyHostToDevice, g->stream));
   GG_CUDA(cudaStreamSynchronize(g->stream));
-  f->fmt = GG_FMT_SPARSE;
   return GG_OK;
 }
 
