@@ -125,12 +125,16 @@ __device__ __forceinline__ BqStep bq_decide(const BqLoop &s, const int32_t *ctl,
   return nh > 0 ? BqStep{BQ_HIMIN, nh, 0} : BqStep{BQ_DONE, 0, 0};
 }
 
+// Mark of the vertices relax step `step` queues (the last step's for its hubs);
+// a mesh session's queue marks lie between them.
+__device__ __forceinline__ int32_t bq_near_tag(int32_t step) { return INT_MIN + 2 + 2 * step; }
+
 // One step, CTA `rank` of `nparts` taking its share.
 // `ctl` holds the control words: global memory in grid mode, CTA 0's shared
-// copy in a one-CTA session.
+// copy in a one-CTA session.  `stages`: three in shared memory, empty.
 template <int LB>
 __device__ __forceinline__ void bq_step(BqLoop &s, const BqArgs &a, const BqStep &st, int32_t *ctl,
-                                        int32_t rank, int32_t nparts, int4 *smem, int32_t *red) {
+                                        int32_t rank, int32_t nparts, int4 *smem, int32_t *red, Stage *stages) {
   const bool lead = rank == 0 && threadIdx.x == 0;
   if (lead) {
     ctl[BQ_NEAR + (s.it + 1) % 3] = 0;
@@ -144,6 +148,11 @@ __device__ __forceinline__ void bq_step(BqLoop &s, const BqArgs &a, const BqStep
   front.cnt = ctl + BQ_NEAR + s.it % 3;
   front.cap = a.qcap;
   front.err = a.err;
+  // appends are staged where many CTAs share the counts; one CTA has them in
+  // shared memory anyway
+  const bool staged = nparts > 1;
+  if (staged) front.stage = &stages[0];
+  Stage *st_lo = staged ? &stages[1] : nullptr, *st_hi = staged ? &stages[2] : nullptr;
   const int32_t lo_next = (s.g + 1) & 1;
   if (st.kind == BQ_RELAX || st.kind == BQ_HUBS) {
     const bool hubs = st.kind == BQ_HUBS;
@@ -153,12 +162,17 @@ __device__ __forceinline__ void bq_step(BqLoop &s, const BqArgs &a, const BqStep
       front.cnt = ctl + BQ_NEAR + (s.it + 2) % 3;
     }
     const DFar far{a.b.stamp, a.b.lo[s.g & 1], ctl + BQ_LO + (s.g & 1), a.b.hi[s.gh & 1],
-                   ctl + BQ_HI + (s.gh & 1), bq_lo_tag(s.g), bq_hi_tag(s.gh), s.hz, a.b.V, a.err};
+                   ctl + BQ_HI + (s.gh & 1), bq_lo_tag(s.g), bq_hi_tag(s.gh), s.hz, a.b.V, a.err, st_lo, st_hi,
+                   bq_near_tag(s.relax - (hubs ? 1 : 0))};
     const EdgeF<USssp, false> f{USssp{a.dist, U, far}, DIn{IN_ALL, nullptr, nullptr},
                                 DIn{IN_ALL, nullptr, nullptr}, false};
     if (hubs) {
       const HubList hub{a.hub_list, nullptr, a.hub_cap, 0};
       lb_hubs(a.g, hub, st.work, f, front, rank, nparts);
+      if (staged) {
+        stage_flush(front);
+        far.flush();
+      }
       s.hub = 0;
       return;
     }
@@ -166,6 +180,10 @@ __device__ __forceinline__ void bq_step(BqLoop &s, const BqArgs &a, const BqStep
     const HubList hub{a.hub_list, ctl + BQ_HUB + s.relax % 3, a.hub_cap, a.hub_min};
     const int32_t n = (int64_t)st.work > a.qcap ? (int32_t)a.qcap : st.work;  // past qcap only after a flagged overflow
     run_lb<LB>(a.g, Enum{qin, nullptr, n}, n, f, front, smem, rank, nparts, hub);
+    if (staged) {
+      stage_flush(front);
+      far.flush();
+    }
     s.in ^= 1;
     s.relax++;
     s.phase = 0;
@@ -190,19 +208,22 @@ __device__ __forceinline__ void bq_step(BqLoop &s, const BqArgs &a, const BqStep
       const int32_t n_lo = min(*(volatile int32_t *)(ctl + BQ_LO + (s.g & 1)), a.b.V);
       if (win <= s.hz) {
         const BqSplitOut o{a.b.stamp, a.b.lo[lo_next], ctl + BQ_LO + lo_next, bq_lo_tag(s.g + 1),
-                           nullptr, nullptr, 0, INT_MAX, nullptr, a.b.V, false};
+                           nullptr, nullptr, 0, INT_MAX, nullptr, a.b.V, false, st_lo, st_hi};
         bq_pile_split(a.b.lo[s.g & 1], n_lo, a.dist, U, win, front, o, a.err, rank, nparts);
+        o.flush(a.err);
       } else {
         // the window reaches past the horizon: split both piles under a new one
         const int32_t hi_next = (s.gh + 1) & 1;
         s.k = bq_adapt_width(s.k, *(volatile int32_t *)(ctl + BQ_FILL + (s.gh & 1)), a.fill_target);
         const int32_t hz = bq_clamp((int64_t)st.m + (int64_t)s.k * a.delta);
         BqSplitOut o{a.b.stamp, a.b.lo[lo_next], ctl + BQ_LO + lo_next, bq_lo_tag(s.g + 1),
-                     a.b.hi[hi_next], ctl + BQ_HI + hi_next, bq_hi_tag(s.gh + 1), hz, nullptr, a.b.V, true};
+                     a.b.hi[hi_next], ctl + BQ_HI + hi_next, bq_hi_tag(s.gh + 1), hz, nullptr, a.b.V, true,
+                     st_lo, st_hi};
         bq_pile_split(a.b.lo[s.g & 1], n_lo, a.dist, U, win, front, o, a.err, rank, nparts);
         o.fill = ctl + BQ_FILL + hi_next;
         bq_pile_split(a.b.hi[s.gh & 1], min(*(volatile int32_t *)(ctl + BQ_HI + (s.gh & 1)), a.b.V), a.dist, U,
                       win, front, o, a.err, rank, nparts);
+        o.flush(a.err);
         s.hz = hz;
         s.gh++;
       }
@@ -230,9 +251,10 @@ __device__ __forceinline__ void bq_step(BqLoop &s, const BqArgs &a, const BqStep
       const int32_t hz = bq_clamp((int64_t)st.m + (int64_t)s.k * a.delta);
       const BqSplitOut o{a.b.stamp, a.b.lo[lo_next], ctl + BQ_LO + lo_next, bq_lo_tag(s.g + 1),
                          a.b.hi[hi_next], ctl + BQ_HI + hi_next, bq_hi_tag(s.gh + 1), hz,
-                         ctl + BQ_FILL + hi_next, a.b.V, false};
+                         ctl + BQ_FILL + hi_next, a.b.V, false, st_lo, st_hi};
       bq_pile_split(a.b.hi[s.gh & 1], min(st.work, a.b.V), a.dist, U, bq_clamp((int64_t)st.m + a.delta), front,
                     o, a.err, rank, nparts);
+      o.flush(a.err);
       s.cur = st.m;
       s.hz = hz;
       s.g++;
@@ -244,6 +266,7 @@ __device__ __forceinline__ void bq_step(BqLoop &s, const BqArgs &a, const BqStep
     default:
       break;
   }
+  if (staged) stage_flush(front);
   s.it++;
 }
 
@@ -261,8 +284,8 @@ __device__ __forceinline__ void bq_step(BqLoop &s, const BqArgs &a, const BqStep
 //    range.  Four lanes share a vertex, an edge each;
 //  * a park decides by the stamp it read and marks the vertex with a plain
 //    store: a vertex parked twice in one round may be listed twice, which the
-//    exchange at the end of the session (mesh_writeback) undoes, so the piles in
-//    global memory hold a vertex once.
+//    exchange at the end of the session undoes: the piles and the queue in
+//    global memory get a vertex once.
 // An entry that an advance takes or finds settled can never be parked again
 // (its distance stays below every later cutoff), so a session needs one mark.
 // 700 x 501 grid, delta 128 (1,344 buckets, 3 relaxes each): 24-29 -> 12.9 ms;
@@ -314,10 +337,23 @@ __device__ __forceinline__ void mesh_flush_high(const BqLoop &s, const BqArgs &a
 }
 
 struct BqMeshMarks {
-  int32_t lo_tag, hi_tag, next_tag, mark_lo, mark_hi;
+  int32_t lo_tag, hi_tag, next_tag, mark_lo, mark_hi, spill;
 };
 
-// Relaxes the n vertices of near_[in]: improvements below U to near_[in ^ 1]
+// A window vertex to the frontier queue in global memory, once a session: it is
+// below the cutoff and never parks again, so its stamp is free to say so.
+__device__ __forceinline__ void mesh_spill(const BqArgs &a, BqMeshSmem &m, int32_t tag, int32_t *q, int32_t v) {
+  if (atomicExch(a.b.stamp + v, tag) == tag) return;
+  const int32_t qp = atomicAdd(&m.spill, 1);
+  if (qp < a.qcap)
+    q[qp] = v;
+  else
+    atomicOr(a.err, DEV_ERR_OVERFLOW);
+}
+
+// Relaxes, at the priorities they were listed with (a vertex lowered since is
+// listed again; reading its distance first costs the trip more than the rare
+// repeat), the n vertices of near_[in]: improvements below U to near_[in ^ 1]
 // (count *n_out, the queue q when that is full), the others parked.  Four lanes
 // share a vertex, an edge each, J vertices of a lane in flight.
 template <int J>
@@ -371,11 +407,7 @@ __device__ __forceinline__ void mesh_relax_pass(const BqLoop &s, const BqArgs &a
             m.near_[in ^ 1][pos] = make_int4(v, p, db[j], de[j]);
           } else {
             m.full = 1;
-            const int32_t qp = atomicAdd(&m.spill, 1);
-            if (qp < a.qcap)
-              q[qp] = v;
-            else
-              atomicOr(a.err, DEV_ERR_OVERFLOW);
+            mesh_spill(a, m, mk.spill, q, v);
           }
         } else if (to == 1) {
           if (pos < kMeshLow) {
@@ -417,6 +449,7 @@ __device__ __forceinline__ void bq_mesh_session(BqLoop &s, const BqArgs &a, int3
   const int32_t mark_lo = -2 * session - 1, mark_hi = -2 * session - 2;  // below every pile tag
   const int32_t lo_tag = bq_lo_tag(s.g), hi_tag = bq_hi_tag(s.gh), next_tag = bq_lo_tag(s.g + 1);
   const int32_t lo_next = (s.g + 1) & 1, T = blockDim.x, lane = threadIdx.x & 31;
+  const BqMeshMarks mk{lo_tag, hi_tag, next_tag, mark_lo, mark_hi, bq_near_tag(0) + 2 * session - 1};
   int32_t *const q = s.in ? a.q1 : a.q0;
   int32_t nl = sctl[BQ_LO + (s.g & 1)];
   for (int32_t i = threadIdx.x; i < n; i += T) {
@@ -443,7 +476,6 @@ __device__ __forceinline__ void bq_mesh_session(BqLoop &s, const BqArgs &a, int3
     if (n > 0) {
       // ---- relax: near_[in] -> near_[in ^ 1], lo[L], hi
       int32_t *n_out = &m.n_near[in ^ 1];
-      const BqMeshMarks mk{lo_tag, hi_tag, next_tag, mark_lo, mark_hi};
       // a second vertex per lane only where the frontier has that many
       if (n <= T >> 2)
         mesh_relax_pass<1>(s, a, sctl, m, mk, n, in, L, U, n_out, q);
@@ -504,11 +536,7 @@ __device__ __forceinline__ void bq_mesh_session(BqLoop &s, const BqArgs &a, int3
             m.near_[in][pos] = x;
           } else {
             m.full = 1;
-            const int32_t qp = atomicAdd(&m.spill, 1);
-            if (qp < a.qcap)
-              q[qp] = x.x;
-            else
-              atomicOr(a.err, DEV_ERR_OVERFLOW);
+            mesh_spill(a, m, mk.spill, q, x.x);
           }
         }
       }
@@ -534,13 +562,9 @@ __device__ __forceinline__ void bq_mesh_session(BqLoop &s, const BqArgs &a, int3
     else
       atomicOr(a.err, DEV_ERR_OVERFLOW);
   }
-  const int32_t sp = (int32_t)min((int64_t)m.spill, a.qcap);
-  for (int32_t i = threadIdx.x; i < n; i += T) {
-    if (sp + i < a.qcap)
-      q[sp + i] = m.near_[in][i].x;
-    else
-      atomicOr(a.err, DEV_ERR_OVERFLOW);
-  }
+  for (int32_t i = threadIdx.x; i < n; i += T) mesh_spill(a, m, mk.spill, q, m.near_[in][i].x);
+  __syncthreads();
+  n = (int32_t)min((int64_t)m.spill, a.qcap);
   s.g++;
   s.phase = 0;
   s.hub = 0;
@@ -549,7 +573,7 @@ __device__ __forceinline__ void bq_mesh_session(BqLoop &s, const BqArgs &a, int3
     s.adv++;
   }
   if (threadIdx.x == 0) {
-    sctl[BQ_NEAR + (s.it + 2) % 3] = sp + n;
+    sctl[BQ_NEAR + (s.it + 2) % 3] = n;
     sctl[BQ_NEAR + s.it % 3] = sctl[BQ_NEAR + (s.it + 1) % 3] = 0;
     sctl[BQ_MIN + (s.it + 2) % 3] = cross;
     sctl[BQ_MIN + s.it % 3] = sctl[BQ_MIN + (s.it + 1) % 3] = INT_MAX;

@@ -117,6 +117,14 @@ struct BqSplitOut {
   int32_t *fill;         // optional count of entries sent to the low pile
   int32_t cap;
   bool dedup;            // two piles feed the low pile in this step: append once per vertex
+  Stage *lo_stage = nullptr, *hi_stage = nullptr;  // shared memory, or null: append directly
+
+  __device__ __forceinline__ void flush(int32_t *err) const {
+    if (!lo_stage) return;
+    stage_flush(lo_stage, lo, lo_cnt, cap, err);
+    if (hi) stage_flush(hi_stage, hi, hi_cnt, cap, err);
+    __syncthreads();
+  }
 };
 
 // Splits pile[0, n): stale entries (P < U) are dropped, the window
@@ -130,6 +138,7 @@ __device__ __forceinline__ void bq_pile_split(const int32_t *__restrict__ pile, 
                                               int32_t nparts) {
   const int32_t stride = nparts * blockDim.x;
   constexpr int kIn = 4;  // entries per thread in flight
+  int32_t fill = 0;
   for (int32_t i0 = rank * blockDim.x + threadIdx.x; i0 < n; i0 += kIn * stride) {
     int32_t vs[kIn], ps[kIn];
 #pragma unroll
@@ -148,21 +157,17 @@ __device__ __forceinline__ void bq_pile_split(const int32_t *__restrict__ pile, 
         } else {
           o.stamp[v] = o.lo_tag;
         }
-        const int32_t pos = agg_inc(o.lo_cnt);
-        if (pos < o.cap)
-          o.lo[pos] = v;
-        else
-          atomicOr(err, DEV_ERR_OVERFLOW);
-        if (o.fill) agg_inc(o.fill);
+        pile_append(o.lo_stage, o.lo, o.lo_cnt, o.cap, v, err);
+        ++fill;
       } else {
         o.stamp[v] = o.hi_tag;
-        const int32_t pos = agg_inc(o.hi_cnt);
-        if (pos < o.cap)
-          o.hi[pos] = v;
-        else
-          atomicOr(err, DEV_ERR_OVERFLOW);
+        pile_append(o.hi_stage, o.hi, o.hi_cnt, o.cap, v, err);
       }
     }
+  }
+  if (o.fill) {
+    fill = __reduce_add_sync(0xffffffffu, fill);
+    if ((threadIdx.x & 31) == 0 && fill) atomicAdd(o.fill, fill);
   }
 }
 

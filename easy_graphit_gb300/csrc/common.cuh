@@ -192,6 +192,23 @@ __device__ __forceinline__ void stage_make_room(const DOut &out, int32_t room) {
   }
 }
 
+// Appends v to a pile, through a CTA's stage when there is one.
+__device__ __forceinline__ void pile_append(Stage *st, int32_t *pile, int32_t *cnt, int32_t cap, int32_t v,
+                                            int32_t *err) {
+  if (st) {
+    const int32_t at = agg_inc(&st->n);
+    if (at < kStageCap) {
+      st->buf[at] = v;
+      return;
+    }
+  }
+  const int32_t pos = agg_inc(cnt);
+  if (pos < cap)
+    pile[pos] = v;
+  else
+    atomicOr(err, DEV_ERR_OVERFLOW);
+}
+
 // Far piles of the single-source delta-stepping queue (bucket_queue.cuh).  A
 // relaxation that lowers P[v] to p at or above the window's cutoff parks v on
 // the low pile (p below the horizon) or the high pile.  stamp[v] holds the tag
@@ -206,24 +223,35 @@ struct DFar {
   int32_t horizon;          // p < horizon -> low pile
   int32_t cap;              // entries a pile can hold (V)
   int32_t *err;
+  Stage *lo_stage, *hi_stage;  // shared memory, or null: append directly
+  // Mark of this step's frontier, or 0: improvements below the cutoff queue their
+  // vertex every time.  With it a vertex is queued once a step.  Such a vertex
+  // stays below every later cutoff and never parks again, so its stamp is free.
+  int32_t near_tag;
 
+  // claim: marks v for its pile; append, when the mark before it was another.
+  __device__ __forceinline__ int32_t tag_of(int32_t p) const { return p < horizon ? lo_tag : hi_tag; }
+  __device__ __forceinline__ int32_t claim(int32_t v, int32_t p) const { return atomicExch(stamp + v, tag_of(p)); }
   __device__ __forceinline__ void park(int32_t v, int32_t p) const {
-    const bool low = p < horizon;
-    const int32_t tag = low ? lo_tag : hi_tag;
-    if (atomicExch(stamp + v, tag) == tag) return;
-    if (low) {
-      const int32_t pos = agg_inc(lo_cnt);
-      if (pos < cap)
-        lo[pos] = v;
-      else
-        atomicOr(err, DEV_ERR_OVERFLOW);
-    } else {
-      const int32_t pos = agg_inc(hi_cnt);
-      if (pos < cap)
-        hi[pos] = v;
-      else
-        atomicOr(err, DEV_ERR_OVERFLOW);
-    }
+    if (claim(v, p) != tag_of(p)) append(v, p);
+  }
+  __device__ __forceinline__ void append(int32_t v, int32_t p) const {
+    if (p < horizon)
+      pile_append(lo_stage, lo, lo_cnt, cap, v, err);
+    else
+      pile_append(hi_stage, hi, hi_cnt, cap, v, err);
+  }
+  // Sends what the CTA staged (all of it, or when less than `room` is left); the
+  // whole CTA calls it, as stage_flush and stage_make_room.
+  __device__ __forceinline__ void flush() const {
+    if (!lo_stage) return;
+    stage_flush(lo_stage, lo, lo_cnt, cap, err);
+    stage_flush(hi_stage, hi, hi_cnt, cap, err);
+  }
+  __device__ __forceinline__ void make_room(int32_t room) const {
+    if (!lo_stage || (lo_stage->n <= kStageCap - room && hi_stage->n <= kStageCap - room)) return;
+    flush();
+    __syncthreads();
   }
 };
 

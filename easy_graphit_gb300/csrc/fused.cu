@@ -170,7 +170,7 @@ __device__ __forceinline__ void bq_solo(BqLoop &s, const BqArgs &a, BqStep st, i
       bq_mesh_session(s, a, sctl, *reinterpret_cast<BqMeshSmem *>(smem), ++*session, near_n, t0);
       steps |= 7;  // long enough to check the clock
     } else {
-      bq_step<LB>(s, a, st, sctl, 0, 1, smem, red);
+      bq_step<LB>(s, a, st, sctl, 0, 1, smem, red, nullptr);
       __syncthreads();
     }
     if ((steps & 7) == 7) {  // a read of the error word is a round trip
@@ -194,6 +194,9 @@ __global__ void __launch_bounds__(1024) k_sssp_bq(BqArgs a) {
   extern __shared__ int4 smem[];
   __shared__ int32_t red[33];
   __shared__ int32_t sctl[BQ_STOP];  // counts and minima of a one-CTA session
+  __shared__ Stage stages[3];        // appends of a step: frontier, low pile, high pile
+  if (threadIdx.x < 3) stages[threadIdx.x].n = 0;
+  __syncthreads();
   BqLoop s{1, 0, 0, 0, 0, bq_clamp((int64_t)a.width0 * a.delta), a.width0, 0, 0, 0, 0};
   int32_t *stop = a.b.ctl + BQ_STOP;
   int32_t session = 0;  // mesh sessions run (CTA 0)
@@ -225,7 +228,7 @@ __global__ void __launch_bounds__(1024) k_sssp_bq(BqArgs a) {
       for (int i = 0; i < kBqLoopInts; ++i) p[i] = pub[i];
       continue;
     }
-    bq_step<LB>(s, a, st, a.b.ctl, blockIdx.x, gridDim.x, smem, red);
+    bq_step<LB>(s, a, st, a.b.ctl, blockIdx.x, gridDim.x, smem, red, stages);
     clk.tick(stop, round, a.err);
     stop_on_overflow(stop, round, a.err);
     if (!grid_barrier(a.bar, gridDim.x, a.err, a.timeout_ns)) break;
@@ -494,7 +497,7 @@ __device__ __forceinline__ void do_fold(DoStat *s, const DoAcc &t) {
 // bfs.cpp's UDF (UBfs) that also notes the out-degree of each vertex it
 // reaches when the loop gathers statistics.
 struct UBfsNote {
-  static constexpr bool kWeight = false;
+  static constexpr bool kWeight = false, kPushes = true;
   int32_t *parent, *depth;
   const int32_t *off;
   DoAcc *acc;  // this thread's; null: no statistics
@@ -787,16 +790,19 @@ gg_status fused_bfs_do(gg_graph *g, const BfsDoPlan &p, int32_t n0, const VData 
   return GG_OK;
 }
 
-// Largest relax step the SSSP loop runs on one CTA, in frontier entries per
-// thread of the CTA (GG_BQ_SOLO_PER_THREAD overrides; 0 turns the one-CTA
-// mode off).  Pile steps take 8 times as many entries: one load and a
-// compare each.
+// Largest relax step the SSSP loop runs on one CTA: four frontier entries per
+// thread of the CTA (GG_BQ_SOLO_PER_THREAD overrides; 0 turns the one-CTA mode
+// off), and for the strategies that spread a list over threads at most 16 edges
+// per thread were every entry the graph's longest list -- a step of the whole GPU takes 9 us, and on a skewed graph CTA 0 alone
+// took 975 us for 1,844 vertices with hubs among them and 25 to 110 us for four to
+// forty (R-MAT of 250,000 vertices, TWCE: 1,860 us in all, 910 without).  Pile
+// steps take 32 entries per thread: one load and a compare each.
 static int32_t bq_solo_per_thread() {
   static const long env = [] {
     const char *e = getenv("GG_BQ_SOLO_PER_THREAD");
     return e ? atol(e) : -1L;
   }();
-  return env >= 0 ? (int32_t)env : 4;
+  return env >= 0 ? (int32_t)env : -1;
 }
 
 // Shared memory of the SSSP loop: the strategy's, or a mesh session's.
@@ -804,7 +810,8 @@ static size_t bq_smem(int lb, int cta, bool mesh) {
   return mesh ? std::max(lb_smem(lb, cta), sizeof(BqMeshSmem)) : lb_smem(lb, cta);
 }
 
-static BqArgs bq_args(gg_graph *g, gg_frontier *f, const BqBuffers &b, int32_t *dist, int32_t delta, int cta) {
+static BqArgs bq_args(gg_graph *g, gg_frontier *f, const BqBuffers &b, int32_t *dist, int32_t delta, int cta,
+                      int lb) {
   BqArgs a{};
   a.g = g->csr.view();
   a.g.nbuckets = 0;
@@ -818,8 +825,10 @@ static BqArgs bq_args(gg_graph *g, gg_frontier *f, const BqBuffers &b, int32_t *
   a.timeout_ns = barrier_timeout_ns();
   a.loop_limit_ns = loop_timeout_ns();
   a.delta = delta;
-  a.solo_max = bq_solo_per_thread() * cta;
+  const int32_t per_thread = bq_solo_per_thread();
+  a.solo_max = (per_thread >= 0 ? per_thread : 4) * cta;
   a.solo_pile_max = 8 * a.solo_max;
+  if (per_thread < 0 && g->max_degree > kMeshMaxDegree && lb != GG_LB_VERTEX_BASED) a.solo_max = std::min(a.solo_max, 16 * cta / g->max_degree);
   a.width0 = 16;
   a.hub_list = static_cast<int32_t *>(g->hubs.p);
   a.hub_cap = hub_capacity(g);
@@ -842,7 +851,7 @@ gg_status fused_sssp(gg_graph *g, const gg_schedule *s, int32_t n0, int32_t delt
   GG_TRY(graph_max_degree(g, &max_degree));  // kept with the graph
   const bool prepared = !iters;
   if (!prepared) GG_TRY(bq_start(pq->bq, n0, g->stream));
-  BqArgs a = bq_args(g, pq->frontier, pq->bq, vd.dist, delta, cta);
+  BqArgs a = bq_args(g, pq->frontier, pq->bq, vd.dist, delta, cta, s->load_balancing);
   const size_t sm = bq_smem(s->load_balancing, cta, a.mesh);
   switch (s->load_balancing) {
     case GG_LB_VERTEX_BASED: GG_TRY(coop_launch(g, prepared, k_sssp_bq<GG_LB_VERTEX_BASED>, cta, sm, a)); break;
@@ -940,7 +949,7 @@ gg_status fused_multi_enqueue(gg_graph *g, cudaStream_t st, bool sssp, const int
   GG_CUDA(cudaMemsetAsync(g->d_bar, 0, sizeof(uint32_t) * 2, st));
   if (sssp) {
     GG_TRY(bq_start(*bq, n, st));
-    BqArgs b = bq_args(g, f, *bq, out, delta, cta);
+    BqArgs b = bq_args(g, f, *bq, out, delta, cta, GG_LB_TWCE);
     void *args[] = {&b};
     note_launch();
     GG_CUDA(cudaLaunchCooperativeKernel(kernel, per_sm * g->sm_count, cta, args, smem, st));

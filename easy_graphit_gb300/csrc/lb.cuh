@@ -54,7 +54,10 @@ __device__ __forceinline__ void do_range(const DGraph &g, const F &f, const DOut
 }
 
 // ------------------------------------------------------------ VERTEX_BASED
-constexpr int kSerialInFlight = 4;
+// Edges a thread that walks a longer list alone has in flight (batched relax): a
+// hub's list is a chain of such batches (R-MAT of 250,000 vertices, 4 / 8 / 12 in
+// flight: 14.4 / 12.8 / 12.1 ms; 12 takes registers the other steps need).
+constexpr int kSerialInFlight = 8;
 // One thread per enumerated vertex, serial neighbour loop with the early exit
 // of operators.cpp:83-94.  Virtual CTA = blockDim.x vertices.
 template <class F>
@@ -63,7 +66,11 @@ __device__ __forceinline__ void lb_vertex(const DGraph &g, const Enum &en, int32
   const int32_t i = vcta * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int32_t s = en.at(i);
-  do_range<kSerialInFlight>(g, f, out, s, __ldg(g.off + s), __ldg(g.off + s + 1), 0, 1);
+  const int32_t b = __ldg(g.off + s), e = __ldg(g.off + s + 1);
+  if (e - b <= 4)
+    do_range(g, f, out, s, b, e, 0, 1);
+  else
+    do_range<kSerialInFlight>(g, f, out, s, b, e, 0, 1);
 }
 
 // ---------------------------------------------------------------------- WM
@@ -205,6 +212,14 @@ __device__ __forceinline__ void lb_twce(const DGraph &g, const Enum &en, int32_t
   __syncthreads();
 }
 
+// Between virtual CTAs: room in the stages of the output queue and, for a
+// functor that parks, of its piles.
+template <class F>
+__device__ __forceinline__ void lb_make_room(const F &f, const DOut &out) {
+  stage_make_room(out, kStageCap / 2);
+  if constexpr (lb_batch<F>::value) f.make_room(kStageCap / 2);
+}
+
 // TWCE over n vertices by CTA `rank` of `nparts`: whole
 // virtual CTAs in turn, or slices of them when there are fewer than CTAs.
 template <class F>
@@ -215,7 +230,7 @@ __device__ __forceinline__ void lb_twce_all(const DGraph &g, const Enum &en, int
   if (nv >= nparts) {
     for (int32_t v = rank; v < nv; v += nparts) {
       lb_twce(g, en, n, f, out, v, 0, 1, sm, hub);
-      stage_make_room(out, kStageCap / 2);
+      lb_make_room(f, out);
     }
   } else if (nv > 0) {
     const int32_t slices = nparts / nv;
@@ -240,7 +255,7 @@ __device__ __forceinline__ void lb_hubs(const DGraph &g, const HubList &hub, int
     lb_chunk(g, hub.list, f, out, c);
     if (out.stage) {
       __syncthreads();
-      stage_make_room(out, kStageCap / 2);
+      lb_make_room(f, out);
       __syncthreads();
     }
   }

@@ -4,77 +4,131 @@
 // parallel.
 #pragma once
 
+#include <type_traits>
+
 #include "engine.h"
 #include "lb.cuh"
 #include "udf.cuh"
 
 namespace gg {
 
+// A kernel's stages: appends to the output queue and, for the relax UDF, to the
+// far piles (Stage, common.cuh).  begin() before the work, end() after it, by the
+// whole CTA.  UDFs that track nothing have none.
+template <class F>
+struct KernelStages {
+  static constexpr int kStages = !F::kPushes ? 0 : (lb_batch<F>::value ? 3 : 1);
+  Stage st[kStages > 0 ? kStages : 1];
+  __device__ __forceinline__ void begin(F &f, DOut &out) {
+    if constexpr (kStages > 0) {
+      if (threadIdx.x < kStages) st[threadIdx.x].n = 0;
+      __syncthreads();
+      if (out.mode == OUT_SPARSE || out.mode == OUT_SPARSE_DEDUP) out.stage = &st[0];
+      if constexpr (kStages == 3) f.stage_parks(&st[1], &st[2]);
+    }
+  }
+  __device__ __forceinline__ void end(const F &f, const DOut &out) {
+    if constexpr (kStages > 0) {
+      if (out.stage) stage_flush(out);
+      f.flush();
+    }
+  }
+};
+template <class F>
+struct NoStages {
+  __device__ __forceinline__ void begin(F &, DOut &) {}
+  __device__ __forceinline__ void end(const F &, const DOut &) {}
+};
+// Shared memory only where there is something to stage.
+#define GG_STAGES(F, f, out)                                                       \
+  using Stages_ = std::conditional_t<F::kPushes, KernelStages<F>, NoStages<F>>;    \
+  __shared__ Stages_ stages_;                                                      \
+  stages_.begin(f, out)
+#define GG_STAGES_END(f, out) stages_.end(f, out)
+
 template <class F>
 __global__ void __launch_bounds__(1024) k_vertex(DGraph g, Enum en, F f, DOut out) {
+  GG_STAGES(F, f, out);
   const int32_t n = en.count();
   const int32_t nv = ceil_div(n, blockDim.x);
   for (int32_t v = blockIdx.x; v < nv; v += gridDim.x) lb_vertex(g, en, n, f, out, v);
+  GG_STAGES_END(f, out);
 }
 
 template <class F>
 __global__ void __launch_bounds__(1024) k_wm(DGraph g, Enum en, F f, DOut out) {
+  GG_STAGES(F, f, out);
   const int32_t n = en.count();
   const int32_t nv = ceil_div(n, blockDim.x >> 5);
   for (int32_t v = blockIdx.x; v < nv; v += gridDim.x) lb_wm(g, en, n, f, out, v);
+  GG_STAGES_END(f, out);
 }
 
 // One whole CTA per enumerated vertex (TWC large bin).
 template <class F>
 __global__ void __launch_bounds__(1024) k_cta(DGraph g, Enum en, F f, DOut out) {
+  GG_STAGES(F, f, out);
   const int32_t n = en.count();
   for (int32_t v = blockIdx.x; v < n; v += gridDim.x) {
     const int32_t s = en.at(v);
     do_range(g, f, out, s, __ldg(g.off + s), __ldg(g.off + s + 1), threadIdx.x, blockDim.x);
   }
+  GG_STAGES_END(f, out);
 }
 
 // TWCE, and with a hub list that takes every CTA part ETWC.
 template <class F>
 __global__ void __launch_bounds__(1024) k_twce(DGraph g, Enum en, F f, DOut out, HubList hub) {
+  GG_STAGES(F, f, out);
   extern __shared__ int4 smem_raw[];
   lb_twce_all(g, en, en.count(), f, out, blockIdx.x, gridDim.x, *reinterpret_cast<TwceSmem *>(smem_raw), hub);
+  GG_STAGES_END(f, out);
 }
 
 template <class F>
 __global__ void __launch_bounds__(1024)
     k_chunks(DGraph g, const int32_t *chunks, const int32_t *chunk_cnt, int32_t cap, F f, DOut out) {
+  GG_STAGES(F, f, out);
   const int32_t n = min(*(volatile const int32_t *)chunk_cnt, cap);
   for (int32_t v = blockIdx.x; v < n; v += gridDim.x) lb_chunk(g, chunks, f, out, v);
+  GG_STAGES_END(f, out);
 }
 
 template <class F>
 __global__ void __launch_bounds__(1024) k_cm(DGraph g, Enum en, F f, DOut out) {
+  GG_STAGES(F, f, out);
   extern __shared__ int4 smem_raw[];
   CmSmem &sm = *reinterpret_cast<CmSmem *>(smem_raw);
   const int32_t n = en.count();
   const int32_t nv = ceil_div(n, blockDim.x);
   for (int32_t v = blockIdx.x; v < nv; v += gridDim.x) lb_cm(g, en, n, f, out, v, sm);
+  GG_STAGES_END(f, out);
 }
 
 template <class F>
 __global__ void __launch_bounds__(1024)
     k_strict(DGraph g, Enum en, const int32_t *sum, F f, DOut out, int32_t per) {
+  GG_STAGES(F, f, out);
   const int32_t n = en.count();
   const int32_t nv = ceil_div(sum[n], per);
   for (int32_t v = blockIdx.x; v < nv; v += gridDim.x) lb_strict(g, en, n, sum, f, out, v, per);
+  GG_STAGES_END(f, out);
 }
 
 template <class F>
 __global__ void __launch_bounds__(1024) k_edge_only(DGraph g, F f, DOut out) {
+  GG_STAGES(F, f, out);
   lb_edge_only(g, f, out, (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
                (int64_t)gridDim.x * blockDim.x);
+  GG_STAGES_END(f, out);
 }
 
 template <class F>
 __global__ void __launch_bounds__(1024) k_edge_only_blocked(DGraph g, F f, DOut out) {
+  GG_STAGES(F, f, out);
   lb_edge_only_blocked(g, f, out, (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
                        (int64_t)gridDim.x * blockDim.x);
+  GG_STAGES_END(f, out);
 }
 
 // Helpers implemented in frontier.cu (not UDF-specific).

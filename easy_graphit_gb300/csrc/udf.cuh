@@ -17,7 +17,7 @@ __device__ __forceinline__ T vload(const T *p) {
 // CAS(&parent[dst], -1, src) (graphit.cpp:96-111) and the tracked parent
 // enqueues dst.  depth[dst] = level is written with it.
 struct UBfs {
-  static constexpr bool kWeight = false;
+  static constexpr bool kWeight = false, kPushes = true;
   int32_t *parent, *depth;
   int32_t level;
   __device__ __forceinline__ bool filter(int32_t v) const { return vload(parent + v) == -1; }
@@ -34,7 +34,7 @@ struct UBfs {
 // (when the queue keeps them), which is how the next bucket is found without
 // scanning every vertex.
 struct USssp {
-  static constexpr bool kWeight = true;
+  static constexpr bool kWeight = true, kPushes = true;
   static constexpr bool kBatch = true;  // push relax over a range: relax_range
   int32_t *dist;
   int32_t cutoff;
@@ -82,13 +82,25 @@ struct USssp {
           asm volatile("red.relaxed.gpu.global.min.s32 [%0], %1;" ::"l"(__cvta_generic_to_global(dist + d[j])),
                        "r"(np[j])
                        : "memory");
+      // The stamp exchanges of the batch go out together: their answers decide
+      // the appends, and one after the other they would be B round trips.
+      // A near vertex is claimed too where the loop marks its steps (near_tag):
+      // threads that lower one vertex together would each queue it, the copies be
+      // relaxed together and multiply.
+      int32_t was[B];
+#pragma unroll
+      for (int j = 0; j < B; ++j) {
+        const int32_t tag = np[j] < cutoff ? far.near_tag : far.tag_of(np[j]);
+        was[j] = prev[j] > np[j] && far.stamp && tag ? atomicExch(far.stamp + d[j], tag) : 0;
+      }
 #pragma unroll
       for (int j = 0; j < B; ++j) {
         if (prev[j] <= np[j]) continue;
-        if (np[j] < cutoff)
-          out.push(d[j]);
-        else if (far.stamp)
-          far.park(d[j], np[j]);
+        if (np[j] < cutoff) {
+          if (!far.near_tag || was[j] != far.near_tag) out.push(d[j]);
+        } else if (far.stamp && was[j] != far.tag_of(np[j])) {
+          far.append(d[j], np[j]);
+        }
       }
     }
   }
@@ -96,7 +108,7 @@ struct USssp {
 
 // pr.cpp:32-34: new_rank[dst] += contrib[src] (fp32 atomicAdd, writeSum).
 struct UPr {
-  static constexpr bool kWeight = false;
+  static constexpr bool kWeight = false, kPushes = false;
   const float *contrib;
   float *new_rank;
   __device__ __forceinline__ bool filter(int32_t) const { return true; }
@@ -111,7 +123,7 @@ struct UPr {
 // reference's access kind for ID[src_id] is left uninitialised,
 // graphit_types.h:374-383).
 struct UCc {
-  static constexpr bool kWeight = false;
+  static constexpr bool kWeight = false, kPushes = false;
   int32_t *ids, *updates;
   __device__ __forceinline__ bool filter(int32_t) const { return true; }
   __device__ __forceinline__ bool apply(int32_t s, int32_t d, int32_t) const {
@@ -129,7 +141,7 @@ struct UCc {
 // bc.cpp:34-40 forward: num_paths[dst] += num_paths[src] on unvisited dst; the
 // tracked num_paths enqueues dst (deduplicated: allow_dupes=false).
 struct UBcF {
-  static constexpr bool kWeight = false;
+  static constexpr bool kWeight = false, kPushes = true;
   double *sigma;
   const uint8_t *visited;
   __device__ __forceinline__ bool filter(int32_t v) const { return vload(visited + v) == 0; }
@@ -143,7 +155,7 @@ struct UBcF {
 // T = float is the reference's VertexData<float>; gg_bc accumulates in double.
 template <class T>
 struct UBcB {
-  static constexpr bool kWeight = false;
+  static constexpr bool kWeight = false, kPushes = false;
   T *dep;
   const uint8_t *visited;
   __device__ __forceinline__ bool filter(int32_t v) const { return vload(visited + v) == 0; }
@@ -171,6 +183,7 @@ struct batch_of<U, decltype(void(U::kBatch))> {
 template <class U, bool PULL>
 struct EdgeF {
   static constexpr bool kWeight = U::kWeight;
+  static constexpr bool kPushes = U::kPushes;  // whether apply ever tracks a vertex
   // push direction with a UDF that has a batched range relax (its to() filter
   // passes every vertex, so the range needs no per-edge destination test)
   static constexpr bool kBatch = !PULL && batch_of<U>::value;
@@ -188,6 +201,19 @@ struct EdgeF {
   __device__ __forceinline__ int32_t apply(int32_t s, int32_t d, int32_t w) const {
     if (PULL) return u.apply(d, s, w) ? s : -1;
     return u.apply(s, d, w) ? d : -1;
+  }
+  __device__ __forceinline__ void make_room(int32_t room) const {
+    if constexpr (kBatch) u.far.make_room(room);
+  }
+  __device__ __forceinline__ void flush() const {
+    if constexpr (kBatch) u.far.flush();
+  }
+  __device__ __forceinline__ void stage_parks(Stage *lo, Stage *hi) {
+    if constexpr (kBatch) {
+      if (!u.far.stamp) return;  // a plain apply parks nothing
+      u.far.lo_stage = lo;
+      u.far.hi_stage = hi;
+    }
   }
   // Only used when kBatch; the source filter (in_src) is checked by the caller.
   template <int B, class G, class Out>
