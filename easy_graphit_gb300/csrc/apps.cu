@@ -68,6 +68,17 @@ __global__ void k_reach(const int32_t *__restrict__ val, const int32_t *__restri
   }
 }
 
+// pr.cpp's vertex step between two edge passes (apps/pr.cpp:28-30, 36-41): the
+// update of one iteration and the contributions of the next, in one pass.
+__global__ void k_pr_step(VData d, const int32_t *__restrict__ off, int32_t V, float beta) {
+  for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
+    const float nr = beta + d.damping * d.new_rank[v];
+    d.old_rank[v] = nr;
+    d.new_rank[v] = 0.0f;
+    d.contrib[v] = nr / (float)(off[v + 1] - off[v]);  // a sink divides by 0, as in the reference
+  }
+}
+
 // The end of a fused single-source trial, in one launch: the reached vertices and
 // their out-degrees (val null: not wanted), then -- by the last block -- these
 // sums, the loop's counters and the status word into pinned host memory.  The sums
@@ -694,10 +705,16 @@ gg_status gg_pagerank(gg_graph *g, const gg_app_schedule *s, int32_t iters, floa
   GG_TRY(vertexset_apply_impl(g, nullptr, GG_VUDF_PR_RESET, vd));
   for (int32_t i = 0; i < iters; ++i) {
     const gg_schedule *sc = pick(s, V, V);
-    GG_TRY(vertexset_apply_impl(g, nullptr, GG_VUDF_PR_CONTRIB, vd));
+    if (i == 0) GG_TRY(vertexset_apply_impl(g, nullptr, GG_VUDF_PR_CONTRIB, vd));
     GG_TRY(edgeset_apply_impl(g, sc, GG_UDF_PR_ADD, GG_FILTER_NONE, nullptr, nullptr, true, vd,
                               INT_MAX, false));
-    GG_TRY(vertexset_apply_impl(g, nullptr, GG_VUDF_PR_UPDATE, vd));
+    if (i + 1 < iters) {
+      note_launch();
+      k_pr_step<<<g->sm_count * 8, 256, 0, g->stream>>>(vd, g->csr.off, V, (float)((1.0 - (double)damping) / V));
+      GG_CUDA(cudaGetLastError());
+    } else {
+      GG_TRY(vertexset_apply_impl(g, nullptr, GG_VUDF_PR_UPDATE, vd));
+    }
     if (st) st->iterations++;
     count_dir(st, sc);
   }

@@ -373,6 +373,59 @@ __device__ __forceinline__ void lb_strict(const DGraph &g, const Enum &en, int32
   }
 }
 
+// ---------------------------------------------------- EDGE_ONLY, run sums
+// Edges [e0, e1) for a functor that adds a term per edge to the enumerated end
+// (PageRank, pull): the edge list holds a vertex's edges in a row -- whole lists,
+// or their parts within a destination bucket -- so a warp sums the runs among 32
+// consecutive edges and adds one value a run.  An atomic per edge is what bound
+// this walk (1 M vertices, 15 M edges, four buckets: 142 us an iteration at 61 %
+// of the L2's rate; now 56).  Four groups of 32 edges are in flight.
+template <class F, class = void>
+struct lb_run_sums {
+  static constexpr bool value = false;
+};
+template <class F>
+struct lb_run_sums<F, decltype(void(F::kRunSums))> {
+  static constexpr bool value = F::kRunSums;
+};
+template <class F>
+__device__ __forceinline__ void lb_edge_runs(const DGraph &g, const F &f, int64_t e0, int64_t e1, int64_t r,
+                                             int64_t width) {
+  constexpr int kIn = 4;
+  const int32_t lane = threadIdx.x & 31;
+  for (int64_t base = e0 + (r >> 5) * (32 * kIn); base < e1; base += (width >> 5) * (32 * kIn)) {
+    int32_t s[kIn], d[kIn];
+    float x[kIn];
+    bool ok[kIn];
+#pragma unroll
+    for (int j = 0; j < kIn; ++j) {
+      const int64_t k = base + j * 32 + lane;
+      s[j] = k < e1 ? __ldg(g.src + k) : -1;
+      d[j] = k < e1 ? __ldg(g.dst + k) : -1;
+    }
+#pragma unroll
+    for (int j = 0; j < kIn; ++j) {
+      ok[j] = d[j] >= 0 && f.src_ok(s[j]) && f.dst_ok(d[j]);
+      x[j] = ok[j] ? f.term(d[j]) : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < kIn; ++j) {
+      const int32_t before = __shfl_up_sync(0xffffffffu, s[j], 1);  // by all lanes, lane 0 too
+      const bool head = lane == 0 || before != s[j];
+      const uint32_t heads = __ballot_sync(0xffffffffu, head), oks = __ballot_sync(0xffffffffu, ok[j]);
+      const uint32_t after = lane == 31 ? 0u : heads >> (lane + 1);
+      const int32_t end = after ? lane + __ffs(after) : 32;  // first lane past this one's run
+#pragma unroll
+      for (int i = 1; i < 32; i <<= 1) {
+        const float o = __shfl_down_sync(0xffffffffu, x[j], i);
+        if (lane + i < end) x[j] += o;
+      }
+      const uint32_t run = (end == 32 ? ~0u : (1u << end) - 1u) & ~((1u << lane) - 1u);
+      if (head && (oks & run)) f.add(s[j], x[j]);
+    }
+  }
+}
+
 // --------------------------------------------------------------- EDGE_ONLY
 // Thread per COO edge over every edge of the graph (operators.cpp:175-200);
 // both endpoints go through the filters.  `r`/`width` index the calling
@@ -380,6 +433,10 @@ __device__ __forceinline__ void lb_strict(const DGraph &g, const Enum &en, int32
 template <class F>
 __device__ __forceinline__ void lb_edge_only(const DGraph &g, const F &f, const DOut &out,
                                              int64_t r, int64_t width) {
+  if constexpr (lb_run_sums<F>::value) {
+    lb_edge_runs(g, f, 0, g.E, r, width);
+    return;
+  }
   for (int64_t k = r; k < g.E; k += width) {
     const int32_t s = __ldg(g.src + k);
     if (!f.src_ok(s)) continue;
@@ -394,8 +451,13 @@ template <class F>
 __device__ __forceinline__ void lb_edge_only_blocked(const DGraph &g, const F &f, const DOut &out,
                                                      int64_t r, int64_t width) {
   for (int32_t b = 0; b < g.nbuckets; ++b) {
-    const int32_t e1 = __ldg(g.bucket + b + 1);
-    for (int64_t k = __ldg(g.bucket + b) + r; k < e1; k += width) {
+    const int32_t e0 = __ldg(g.bucket + b), e1 = __ldg(g.bucket + b + 1);
+    if constexpr (lb_run_sums<F>::value) {
+      lb_edge_runs(g, f, e0, e1, r, width);
+      __syncthreads();
+      continue;
+    }
+    for (int64_t k = e0 + r; k < e1; k += width) {
       const int32_t s = __ldg(g.src + k);
       if (!f.src_ok(s)) continue;
       do_edge(g, f, out, s, (int32_t)k);

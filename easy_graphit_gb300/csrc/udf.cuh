@@ -109,8 +109,11 @@ struct USssp {
 // pr.cpp:32-34: new_rank[dst] += contrib[src] (fp32 atomicAdd, writeSum).
 struct UPr {
   static constexpr bool kWeight = false, kPushes = false;
+  static constexpr bool kSums = true;  // apply adds term(s) to the target: runs of one target can be summed first
   const float *contrib;
   float *new_rank;
+  __device__ __forceinline__ float term(int32_t s) const { return __ldg(contrib + s); }
+  __device__ __forceinline__ void add(int32_t d, float x) const { atomicAdd(new_rank + d, x); }
   __device__ __forceinline__ bool filter(int32_t) const { return true; }
   __device__ __forceinline__ bool apply(int32_t s, int32_t d, int32_t) const {
     atomicAdd(new_rank + d, __ldg(contrib + s));
@@ -180,8 +183,22 @@ struct batch_of<U, decltype(void(U::kBatch))> {
   static constexpr bool value = U::kBatch;
 };
 
+template <class U, class = void>
+struct sums_of {
+  static constexpr bool value = false;
+};
+template <class U>
+struct sums_of<U, decltype(void(U::kSums))> {
+  static constexpr bool value = U::kSums;
+};
+
 template <class U, bool PULL>
 struct EdgeF {
+  // pull direction with a UDF that sums: the edges of an enumerated vertex, in a
+  // row in the edge list, add to that vertex
+  static constexpr bool kRunSums = PULL && sums_of<U>::value;
+  __device__ __forceinline__ float term(int32_t d) const { return u.term(d); }
+  __device__ __forceinline__ void add(int32_t s, float x) const { u.add(s, x); }
   static constexpr bool kWeight = U::kWeight;
   static constexpr bool kPushes = U::kPushes;  // whether apply ever tracks a vertex
   // push direction with a UDF that has a batched range relax (its to() filter
