@@ -11,8 +11,8 @@
 //    next level's masks and depths;
 //  * bottom-up (frontier larger than V / bu_div): groups of 8 lanes take the
 //    vertices some still-expanding source has not reached and OR the level
-//    masks of their in-neighbours, 8 at a time, stopping as soon as every such
-//    source is found; no atomics.
+//    masks of their in-neighbours, 32 at a time, stopping as soon as every such
+//    source is found, a CTA the long lists; no atomics in global memory.
 // Level masks rotate through three arrays and queues through three buffers:
 // the masks of level L-1 are cleared (from its queue) while level L publishes,
 // so a bottom-up scan never reads a stale mask.
@@ -79,10 +79,163 @@ __device__ __forceinline__ void ms_fold(const MsAcc &t, unsigned long long *s_ac
   }
 }
 
-__global__ void __launch_bounds__(512) k_msbfs(DGraph g, MsBfsState st) {
+// A bottom-up level: every vertex that some still-expanding source wants ORs the
+// level masks of its in-neighbours and stops when each such source is found.  A
+// lane per vertex reads the masks (coalesced) and drops vertices nobody wants or
+// without in-edges; 8-lane groups walk the lists, 32 in-neighbours in flight each,
+// four vertices of a warp at a time; lists longer than kMsLong are set aside for
+// the whole CTA.  With a group per vertex and 8 in flight, a hub that one source
+// does not reach was walked alone for 2.4 ms, whatever the level held (1 M
+// vertices; a level that chose bottom-up with such a hub in it: 3.2 ms of 4.9).
+constexpr int32_t kMsLong = 512;
+constexpr int32_t kMsLongMax = 256;  // set aside per CTA; more are walked by groups
+struct MsLong {
+  int32_t n;
+  uint32_t found[2];
+  int32_t v[kMsLongMax];
+};
+__device__ __forceinline__ uint64_t ms_shfl(uint64_t x, int32_t l) {
+  return __shfl_sync(0xffffffffu, (unsigned long long)x, l & 31);
+}
+__device__ __forceinline__ void ms_bottom_up(const MsBfsState &st, int32_t L, const uint64_t *frc, uint64_t *frn,
+                                             const DOut &out, MsAcc &acc, MsLong &lg) {
+  const int32_t lane = threadIdx.x & 31, sub = lane & 7, gi = lane >> 3;
+  const uint32_t gmask = 0xFFu << (gi * 8);
+  const uint64_t act = *(volatile unsigned long long *)(st.actm + L % 3);
+  if (threadIdx.x == 0) {
+    lg.n = 0;
+    lg.found[0] = lg.found[1] = 0u;
+  }
+  __syncthreads();
+  int32_t since = 0;  // vertices the CTA can have staged since there was room
+  for (int64_t first = (int64_t)blockIdx.x * blockDim.x; first < st.V; first += (int64_t)gridDim.x * blockDim.x) {
+    if (since + (int32_t)blockDim.x > kStageCap / 2) {
+      __syncthreads();
+      stage_make_room(out, kStageCap / 2 + (int32_t)blockDim.x);
+      __syncthreads();
+      since = 0;
+    }
+    since += (int32_t)blockDim.x;
+    const int64_t v64 = first + threadIdx.x;
+    const int32_t v = (int32_t)v64;
+    uint64_t sv = 0, want = 0, found = 0;
+    int32_t kb = 0, ke = 0;
+    if (v64 < st.V) {
+      sv = __ldcg(st.seen + v);
+      want = act & ~sv;
+      if (want) {
+        kb = __ldg(st.toff + v);
+        ke = __ldg(st.toff + v + 1);
+      }
+    }
+    bool mine_here = want != 0 && ke > kb;
+    if (mine_here && ke - kb > kMsLong) {
+      const int32_t at = agg_inc(&lg.n);
+      if (at < kMsLongMax) {
+        lg.v[at] = v;
+        mine_here = false;
+      }
+    }
+    __syncwarp();
+    uint32_t open = __ballot_sync(0xffffffffu, mine_here);
+    while (open) {
+      int32_t l[4];  // the next four vertices, a group each (-1: none)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        l[j] = __ffs(open) - 1;
+        open &= open - 1;
+      }
+      const int32_t mine = gi == 0 ? l[0] : (gi == 1 ? l[1] : (gi == 2 ? l[2] : l[3]));
+      const uint64_t w = ms_shfl(want, mine);
+      const int32_t b = __shfl_sync(0xffffffffu, kb, mine & 31), e = __shfl_sync(0xffffffffu, ke, mine & 31);
+      uint64_t f = 0;
+      if (mine >= 0)
+        for (int32_t k0 = b; k0 < e; k0 += 32) {
+          int32_t u[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) u[j] = k0 + 8 * j + sub < e ? __ldg(st.tsrc + k0 + 8 * j + sub) : -1;
+          uint64_t m = 0;
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (u[j] >= 0) m |= __ldcg(frc + u[j]);
+          m &= w;
+          m |= __shfl_xor_sync(gmask, (unsigned long long)m, 1);
+          m |= __shfl_xor_sync(gmask, (unsigned long long)m, 2);
+          m |= __shfl_xor_sync(gmask, (unsigned long long)m, 4);
+          f |= m;
+          if (f == w) break;
+        }
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint64_t h = ms_shfl(f, j * 8);
+        if (lane == l[j]) found = h;
+      }
+    }
+    if (found) {
+      st.seen[v] = sv | found;
+      frn[v] = found;
+      out.sparse(v);
+      acc.note(st, v, found);
+    }
+    if (!st.depth) continue;
+    // the warp's rows of one source are consecutive words: a store per source
+    uint32_t any[2] = {__reduce_or_sync(0xffffffffu, (uint32_t)found),
+                       __reduce_or_sync(0xffffffffu, (uint32_t)(found >> 32))};
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      for (uint32_t bits = any[h]; bits; bits &= bits - 1) {
+        const int32_t s = 32 * h + __ffs(bits) - 1;
+        if ((found >> s) & 1) st.depth[(int64_t)s * st.depth_stride + v] = L + 1;
+      }
+  }
+  __syncthreads();
+  const int32_t nl = min(lg.n, kMsLongMax);
+  for (int32_t i = 0; i < nl; ++i) {
+    const int32_t v = lg.v[i];
+    const uint64_t sv = __ldcg(st.seen + v), want = act & ~sv;
+    const int32_t kb = __ldg(st.toff + v), ke = __ldg(st.toff + v + 1), T = blockDim.x;
+    uint64_t found = 0;
+    for (int32_t k0 = kb; k0 < ke; k0 += 4 * T) {
+      int32_t u[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int64_t k = (int64_t)k0 + j * T + threadIdx.x;
+        u[j] = k < ke ? __ldg(st.tsrc + k) : -1;
+      }
+      uint64_t m = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (u[j] >= 0) m |= __ldcg(frc + u[j]);
+      m &= want;
+      const uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)m), hi = __reduce_or_sync(0xffffffffu, (uint32_t)(m >> 32));
+      if (lane == 0 && lo) atomicOr(&lg.found[0], lo);
+      if (lane == 0 && hi) atomicOr(&lg.found[1], hi);
+      __syncthreads();
+      found = (uint64_t)lg.found[1] << 32 | lg.found[0];
+      __syncthreads();
+      if (found == want || (int64_t)k0 + 4 * T >= ke) break;
+    }
+    if (threadIdx.x == 0) {
+      lg.found[0] = lg.found[1] = 0u;
+      if (found) {
+        st.seen[v] = sv | found;
+        frn[v] = found;
+        out.sparse(v);
+        acc.note(st, v, found);
+      }
+    }
+    if (st.depth && threadIdx.x < kMsBfsWidth && ((found >> threadIdx.x) & 1))
+      st.depth[(int64_t)threadIdx.x * st.depth_stride + v] = L + 1;
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(512, 3) k_msbfs(DGraph g, MsBfsState st) {
   extern __shared__ int4 smem[];
   __shared__ unsigned long long s_act;
   __shared__ unsigned long long s_stat[3];
+  __shared__ MsLong long_;
   __shared__ Stage stage;
   if (threadIdx.x == 0) stage.n = 0;  // the first level's barrier comes before any append
   const int32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -152,36 +305,8 @@ __global__ void __launch_bounds__(512) k_msbfs(DGraph g, MsBfsState st) {
       const Enum en{ms_q(st, L), nullptr, n};
       lb_twce_all(g, en, n, f, out, blockIdx.x, gridDim.x, *reinterpret_cast<TwceSmem *>(smem), hub);
     } else {
-      // bottom-up: 8-lane groups over the vertices still wanted by some source
       ++bu_levels;
-      const uint64_t act = *(volatile unsigned long long *)(st.actm + L % 3);
-      const int32_t sub = lane & 7;
-      const uint32_t gmask = 0xFFu << (lane & ~7);
-      for (int32_t v = tid >> 3; v < st.V; v += nthreads >> 3) {
-        const uint64_t sv = __ldcg(st.seen + v);
-        const uint64_t want = act & ~sv;
-        if (!want) continue;
-        const int32_t kb = __ldg(st.toff + v), ke = __ldg(st.toff + v + 1);
-        uint64_t found = 0;
-        for (int32_t k0 = kb; k0 < ke; k0 += 8) {
-          uint64_t m = 0;
-          if (k0 + sub < ke) m = __ldcg(frc + __ldg(st.tsrc + k0 + sub)) & want;
-          m |= __shfl_xor_sync(gmask, m, 1);
-          m |= __shfl_xor_sync(gmask, m, 2);
-          m |= __shfl_xor_sync(gmask, m, 4);
-          found |= m;
-          if (found == want) break;
-        }
-        if (found) {
-          if (sub == 0) {
-            st.seen[v] = sv | found;
-            frn[v] = found;
-            out.sparse(v);
-            acc.note(st, v, found);
-          }
-          ms_depths(st, v, found, L + 1, sub, 8);
-        }
-      }
+      ms_bottom_up(st, L, frc, frn, out, acc, long_);
     }
     stage_flush(out);
     if (!grid_barrier(st.bar, gridDim.x, st.err, st.timeout_ns)) break;
