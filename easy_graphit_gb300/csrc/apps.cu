@@ -804,6 +804,23 @@ gg_status gg_bc(gg_graph *g, const gg_app_schedule *s, int32_t src, float *dep_o
   GG_TRY(app_array(g, 5, V, &dep));
   GG_TRY(app_array(g, 3, V, &dep64));
   GG_TRY(app_array(g, 7, V, &visited));
+  if (s->fuse && s->kind == GG_SCHED_SIMPLE && fused_supported(&s->s1)) {
+    int32_t *depth = nullptr, *lev = nullptr, *loff = nullptr;
+    GG_TRY(app_array(g, 0, V, &depth));
+    GG_TRY(app_array(g, 1, V, &lev));
+    GG_TRY(app_array(g, 2, (size_t)V + 2, &loff));
+    Trial t(g);
+    GG_TRY(fused_bc(g, &s->s1, src, depth, lev, loff, sigma, dep64, dep));
+    GG_TRY(end_trial(t, "bc", depth, g->d_misc + 44, st,
+                     {{reinterpret_cast<int32_t *>(dep_out), reinterpret_cast<const int32_t *>(dep)}}));
+    if (st) {
+      st->iterations = g->h_out->stats[0];
+      st->push_iterations = 2 * st->iterations - 1;  // forward, and backward from every level but the source's
+      st->edges_traversed *= 2;
+      st->fused = 1;
+    }
+    return GG_OK;
+  }
   gg_frontier *f = nullptr;
   GG_TRY(app_frontier(g, &f));
   if (!g->app_list) GG_TRY(gg_frontier_list_create(g, &g->app_list));

@@ -263,6 +263,13 @@ struct BfsDoPlan {
 };
 gg_status fused_bfs_do(gg_graph *g, const BfsDoPlan &p, int32_t n0, const VData &vd, gg_frontier *f,
                        int32_t *iters, int32_t *pulls);
+// CTAs of a persistent loop: the resident ones, fewer on a graph that has no work
+// for them.
+int loop_grid(const gg_graph *g, int per_sm, int cta);
+// Single-source BC in one launch (fused_bc.cu), launched only; depth, lev: V ints,
+// loff: V + 2; stats (levels) at d_misc + 44.
+gg_status fused_bc(gg_graph *g, const gg_schedule *s, int32_t src, int32_t *depth, int32_t *lev, int32_t *loff,
+                   double *sigma, double *dep64, float *out);
 gg_status fused_sssp(gg_graph *g, const gg_schedule *s, int32_t n0, int32_t delta, const VData &vd,
                      gg_pq *pq, int32_t *iters, int64_t *advances, bool *ran);
 // Bucket-queue buffers for V vertices (pool memory on the graph's stream), their

@@ -259,6 +259,14 @@ gg_status bq_start(const BqBuffers &b, int32_t n0, cudaStream_t st) {
   return GG_OK;
 }
 
+// A small graph takes fewer CTAs: 8 lanes for every vertex or a thread for every
+// edge, whichever is more.  What the others would do is wait (a barrier of 41 CTAs
+// takes 1.3 us, of 608 2.2).
+int loop_grid(const gg_graph *g, int per_sm, int cta) {
+  const int64_t want = std::max(ceil_div((int64_t)g->csr.V * kStage1, cta), ceil_div((int64_t)g->csr.E, cta));
+  return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)per_sm * g->sm_count, want));
+}
+
 template <class K, class A, class... More>
 static gg_status coop_launch(gg_graph *g, bool prepared, K kernel, int cta, size_t smem, A &a, More &...more) {
   int per_sm = 0;
@@ -266,11 +274,7 @@ static gg_status coop_launch(gg_graph *g, bool prepared, K kernel, int cta, size
     GG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   GG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, cta, smem));
   if (per_sm < 1) return set_error(GG_ERR_UNSUPPORTED, "fused kernel does not fit on an SM");
-  // A small graph takes fewer CTAs: 8 lanes for every vertex or a thread for
-  // every edge, whichever is more.  What the others would do is wait (a barrier of
-  // 41 CTAs takes 1.3 us, of 608 2.2).
-  const int64_t want = std::max(ceil_div((int64_t)g->csr.V * kStage1, cta), ceil_div((int64_t)g->csr.E, cta));
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(per_sm * g->sm_count, want));
+  const int grid = loop_grid(g, per_sm, cta);
   if (!prepared) GG_CUDA(cudaMemsetAsync(g->d_bar, 0, sizeof(uint32_t) * 2, g->stream));
   void *args[] = {&a, &more...};
   GG_CUDA(cudaEventRecord(g->ev2, g->stream));
