@@ -281,6 +281,33 @@ __device__ __forceinline__ void mesh_relax(const MeshView &mv, const MeshSink &s
   }
 }
 
+// The same by four lanes a vertex, an edge each (lane `sub` takes b + sub, b + sub +
+// 4, ...): steps of few vertices, the common ones, are bound by the chain of one
+// thread's loads and appends, four edges' worth when a thread has the vertex alone
+// (50 vertices a step: 6,200 cycles of 11,000; 32 sources on a 500 x 501 grid at delta
+// 32: 34.6 -> 26.1 ms, on 2048^2 198 -> 161).  Steps of more vertices than a quarter
+// of the CTA keep a thread each.  The check reads the distance
+// once per lane, with the edge.
+__device__ __forceinline__ void mesh_relax_lanes(const MeshView &mv, const MeshSink &s, int32_t v, int32_t p, int32_t b,
+                                                 int32_t e, bool check, int32_t sub, int32_t &smin) {
+  for (int32_t k = b + sub; k < e; k += 4) {
+    const int32_t now = check ? __ldcg(mv.dist + v) : p;
+    const int32_t d = __ldg(mv.dst + k), w = __ldg(mv.w + k);
+    const int32_t q = min(p, now);
+    if (q < s.lo) return;
+    const int32_t np = q + w;
+    const int32_t prev = __ldcg(mv.dist + d), st = __ldcg(mv.stamp + d);
+    const int32_t db = __ldg(mv.off + d), de = __ldg(mv.off + d + 1);
+    if (prev <= np) continue;
+    asm volatile("red.relaxed.gpu.global.min.s32 [%0], %1;" ::"l"(__cvta_generic_to_global(mv.dist + d)), "r"(np)
+                 : "memory");
+    if (np < s.cutoff)
+      mesh_list_push(mv, s, d, np, db, de);
+    else
+      mesh_park<false>(mv, s, d, np, db, de, st, smin);
+  }
+}
+
 // Warp-then-block folds of per-thread values into shared words.
 __device__ __forceinline__ void mesh_fold_min(int32_t v, int32_t *dst) {
   v = __reduce_min_sync(0xffffffffu, v);
@@ -577,7 +604,12 @@ __global__ void __launch_bounds__(kMeshThreads) k_sssp_cta(CtaSsspArgs c) {
         // the first block-width of entries is relaxed by the thread that reads
         // it; the rest goes to the relax list (even shares in the first round)
         if (ns > T) mesh_scan_slot(mv, s, slot + T, ns - T);
-        if ((int32_t)threadIdx.x < ns) {
+        if (ns <= T / 4) {
+          if ((int32_t)threadIdx.x >> 2 < ns) {
+            const int4 x = __ldcg(slot + (threadIdx.x >> 2));
+            mesh_relax_lanes(mv, s, x.x, x.y, x.z, x.w, true, threadIdx.x & 3, smin);
+          }
+        } else if ((int32_t)threadIdx.x < ns) {
           const int4 x = __ldcg(slot + threadIdx.x);
           mesh_relax(mv, s, x.x, x.y, x.z, x.w, true, smin);
         }
@@ -611,9 +643,16 @@ __global__ void __launch_bounds__(kMeshThreads) k_sssp_cta(CtaSsspArgs c) {
       const int4 *lin = lists + ((r - 1) & 1) * kMeshList;
       s.list = lists + (r & 1) * kMeshList;
       s.list_cnt = &C.list_cnt[r % 3];
-      for (int32_t i = threadIdx.x; i < nl; i += blockDim.x) {
-        const int4 x = lin[i];
-        mesh_relax(mv, s, x.x, x.y, x.z, x.w < 0 ? ~x.w : x.w, x.w < 0, smin);
+      if (nl <= (int32_t)blockDim.x / 4) {
+        if ((int32_t)threadIdx.x >> 2 < nl) {
+          const int4 x = lin[threadIdx.x >> 2];
+          mesh_relax_lanes(mv, s, x.x, x.y, x.z, x.w < 0 ? ~x.w : x.w, x.w < 0, threadIdx.x & 3, smin);
+        }
+      } else {
+        for (int32_t i = threadIdx.x; i < nl; i += blockDim.x) {
+          const int4 x = lin[i];
+          mesh_relax(mv, s, x.x, x.y, x.z, x.w < 0 ? ~x.w : x.w, x.w < 0, smin);
+        }
       }
       mesh_fold_min(smin, &C.srec);
       smin = INT_MAX;
