@@ -1,19 +1,25 @@
-// PageRank pull iteration for PULL + TWC schedules: the in-degree bins of the
-// transposed graph are built once per call (thread / warp / tiles of a CTA per
-// vertex, the TWC binning of graph.h:48-54 applied to the pull gather), and
-// every iteration is one gather per bin that fuses pr.cpp's three steps
+// PageRank pull iteration for PULL + TWC schedules: the vertices fall into three
+// classes by in-degree (thread / warp / tiles of a CTA per vertex, the TWC binning
+// of graph.h:48-54 applied to the pull gather), and every iteration is one launch
+// that fuses pr.cpp's three steps
 //   contrib[u] = old[u] / outdeg[u];   new[v] = sum contrib[u];
 //   old[v] = (1-d)/V + d * new[v]
 // (apps/pr.cpp:28-41).  Each vertex's sum is formed in a fixed order -- by its
 // owner, or for hubs from per-tile partial sums added in tile order -- so there
-// are no atomics and results are bit-identical across runs.  The next
+// are no float atomics and results are bit-identical across runs.  The next
 // iteration's contributions go to the other half of a double buffer.
 //
-// The gathers are latency-bound (contrib is L2-resident, its reads random), so
-// every lane keeps four independent contrib loads in flight, and the iteration
-// runs on the degree-ordered copy of the graph (relabel.cu): the contributions
-// of the high-degree vertices, read by most in-edges, share cache lines.  Ranks
+// The iteration runs on the degree-ordered copy of the graph (relabel.cu): the
+// contributions of the high-degree vertices, read by most in-edges, share cache
+// lines, and the classes are ranges of ids -- that order goes by floor(log2(degree +
+// 1)), so a boundary at 2^k - 1 is found by bisection and no bins are built.  Ranks
 // come back to the caller's ids at the end.
+//
+// What bounds the gathers is the L1's rate of scattered sectors (74 % of it in the
+// warp class), so every lane keeps four contrib loads in flight and the classes
+// run side by side: in launches of their own they left its tails empty three times
+// an iteration (directed R-MAT 22, an iteration: 49 + 142 + 31 + 5 us in four
+// launches, now 183 in one).
 #include <algorithm>
 #include <vector>
 
@@ -21,9 +27,11 @@
 
 namespace gg {
 
-constexpr int32_t kPrSmallMax = 32;   // in-degree < 32: one thread
-constexpr int32_t kPrMidMax = 4096;   // < 4096: one warp; else tiles of kPrTile edges
-constexpr int32_t kPrTile = 8192;     // in-edges per CTA tile of a hub
+constexpr int32_t kPrSmallMax = 31;   // in-degree < 31: one thread
+constexpr int32_t kPrMidMax = 4095;   // < 4095: one warp; else tiles of kPrTile edges
+constexpr int32_t kPrTile = 4096;     // in-edges per CTA tile of a hub: 16 a thread
+constexpr int32_t kPrThreads = 256;
+constexpr int32_t kPrMidPer = 4;      // vertices a warp of the middle class takes
 
 struct PrArgs {
   const int32_t *toff, *tsrc;   // CSC
@@ -56,76 +64,78 @@ __device__ __forceinline__ float pr_gather(const PrArgs &a, int32_t k0, int32_t 
   return (s0 + s1) + (s2 + s3);
 }
 
-__global__ void k_pr_small(PrArgs a, const int32_t *__restrict__ bin, int32_t n) {
-  for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int32_t v = bin[i];
-    pr_finish(a, v, pr_gather(a, __ldg(a.toff + v), __ldg(a.toff + v + 1), 1));
-  }
-}
+// One iteration.  Hubs are vertices [0, nh), their tiles in vertex order: tile t
+// covers in-edges [tile_k[t], + kPrTile) of tile_v[t], hub v owns tiles [first[v],
+// first[v + 1]).  The middle class is [nh, mid), the rest single threads'.  Blocks
+// come in that order, the longest work first.
+struct PrIter {
+  PrArgs a;
+  const int32_t *first, *tile_v, *tile_k;
+  double *partial;  // [ntiles]
+  int32_t *done;    // [nh] tiles of a hub summed so far; zero between iterations
+  int32_t ntiles, nh, mid, V, mid_blocks;
+};
 
-__global__ void k_pr_mid(PrArgs a, const int32_t *__restrict__ bin, int32_t n) {
-  const int32_t lane = threadIdx.x & 31;
-  const int32_t w0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-  for (int32_t i = w0; i < n; i += nw) {
-    const int32_t v = bin[i];
-    float s = pr_gather(a, __ldg(a.toff + v) + lane, __ldg(a.toff + v + 1), 32);
+__global__ void __launch_bounds__(kPrThreads) k_pr_iter(PrIter p) {
+  const PrArgs &a = p.a;
+  const int32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int32_t b = (int32_t)blockIdx.x;
+  if (b < p.ntiles) {
+    __shared__ float part[kPrThreads / 32];
+    const int32_t v = p.tile_v[b];
+    const int32_t kb = p.tile_k[b], ke = min(kb + kPrTile, __ldg(a.toff + v + 1));
+    float s = pr_gather(a, kb + (int32_t)threadIdx.x, ke, kPrThreads);
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-    if (lane == 0) pr_finish(a, v, s);
-  }
-}
-
-// One CTA per hub tile: partial[t] = sum over the tile's in-edges.
-__global__ void __launch_bounds__(512) k_pr_tile(PrArgs a, const int32_t *__restrict__ tile_v,
-                                                 const int32_t *__restrict__ tile_k, int32_t ntiles,
-                                                 float *__restrict__ partial) {
-  __shared__ float part[32];
-  for (int32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int32_t v = tile_v[t];
-    const int32_t kb = tile_k[t], ke = min(kb + kPrTile, __ldg(a.toff + v + 1));
-    float s = pr_gather(a, kb + (int32_t)threadIdx.x, ke, (int32_t)blockDim.x);
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    if (lane == 0) part[wid] = s;
     __syncthreads();
-    if (threadIdx.x < 32) {
-      s = threadIdx.x < (blockDim.x >> 5) ? part[threadIdx.x] : 0.f;
+    if (threadIdx.x != 0) return;
+    // the warps' and the tiles' sums are few: added in fp64, they round once
+    double sum = 0.0;
+    for (int w = 0; w < kPrThreads / 32; ++w) sum += (double)part[w];
+    const int32_t t0 = p.first[v], t1 = p.first[v + 1];
+    p.partial[b] = sum;
+    __threadfence();
+    if (atomicAdd(p.done + v, 1) != t1 - t0 - 1) return;
+    __threadfence();  // the hub's last tile adds them all, in tile order
+    sum = 0.0;
+    for (int32_t t = t0; t < t1; ++t) sum += __ldcg(p.partial + t);
+    p.done[v] = 0;
+    pr_finish(a, v, (float)sum);
+    return;
+  }
+  b -= p.ntiles;
+  if (b < p.mid_blocks) {
+    const int32_t v0 = p.nh + (b * (kPrThreads / 32) + wid) * kPrMidPer, v1 = min(v0 + kPrMidPer, p.mid);
+    for (int32_t v = v0; v < v1; ++v) {
+      float s = pr_gather(a, __ldg(a.toff + v) + lane, __ldg(a.toff + v + 1), 32);
 #pragma unroll
       for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-      if (threadIdx.x == 0) partial[t] = s;
+      if (lane == 0) pr_finish(a, v, s);
     }
-    __syncthreads();
+    return;
   }
+  b -= p.mid_blocks;
+  const int64_t v = (int64_t)p.mid + (int64_t)b * kPrThreads + threadIdx.x;
+  if (v < p.V) pr_finish(a, (int32_t)v, pr_gather(a, __ldg(a.toff + v), __ldg(a.toff + v + 1), 1));
 }
 
-// Hub i owns tiles [first[i], first[i+1]): their partial sums in tile order.
-__global__ void k_pr_hub_finish(PrArgs a, const int32_t *__restrict__ hubs, const int32_t *__restrict__ first,
-                                int32_t nhubs, const float *__restrict__ partial) {
-  for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nhubs; i += gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int32_t t = first[i]; t < first[i + 1]; ++t) s += partial[t];
-    pr_finish(a, hubs[i], s);
-  }
-}
-
-__global__ void k_pr_bin(const int32_t *__restrict__ toff, int32_t V, int32_t *__restrict__ bins, int32_t *cnt) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  const int64_t end = (V + stride - 1) / stride * stride;  // whole warps iterate together
-  for (int64_t v = blockIdx.x * blockDim.x + threadIdx.x; v < end; v += stride) {
-    int32_t d = -1;
-    if (v < V) d = toff[v + 1] - toff[v];
-    const int which = d < 0 ? -1 : (d < kPrSmallMax ? 0 : (d < kPrMidMax ? 1 : 2));
-    for (int b = 0; b < 3; ++b) {
-      const bool p = which == b;
-      const uint32_t m = __ballot_sync(0xffffffffu, p);
-      if (!m) continue;
-      const int32_t lane = threadIdx.x & 31;
-      int32_t base = 0;
-      if (lane == 0) base = atomicAdd(cnt + b, __popc(m));
-      base = __shfl_sync(0xffffffffu, base, 0);
-      if (p) bins[(int64_t)b * V + base + __popc(m & ((1u << lane) - 1))] = (int32_t)v;
+// bounds[i] = first vertex whose in-degree class lies below the i-th boundary
+// (in-degrees fall from class to class; a thread bisects for each).
+__global__ void k_pr_bounds(const int32_t *__restrict__ toff, int32_t V, int32_t *__restrict__ bounds) {
+  if (threadIdx.x >= 2) return;
+  const int32_t least = threadIdx.x == 0 ? kPrMidMax : kPrSmallMax;
+  int32_t lo = 0, len = V;
+  while (len > 0) {
+    const int32_t half = len >> 1, v = lo + half;
+    if (__ldg(toff + v + 1) - __ldg(toff + v) >= least) {
+      lo = v + 1;
+      len -= half + 1;
+    } else {
+      len = half;
     }
   }
+  bounds[threadIdx.x] = lo;
 }
 
 __global__ void k_pr_unperm(const float *__restrict__ rank_new, const int32_t *__restrict__ perm, int32_t V,
@@ -141,83 +151,54 @@ __global__ void k_pr_init(const int32_t *__restrict__ off, int32_t V, float inv_
   }
 }
 
-__global__ void k_pr_hub_bounds(const int32_t *__restrict__ toff, const int32_t *__restrict__ hubs, int32_t nh,
-                                int32_t *__restrict__ bounds) {
-  for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nh; i += gridDim.x * blockDim.x) {
-    bounds[2 * i] = toff[hubs[i]];
-    bounds[2 * i + 1] = toff[hubs[i] + 1];
-  }
-}
-
-// In-degree bins of the transposed graph (in the TWC-bin scratch slot: no
-// load-balancing strategy runs during the PageRank loop) and the tiles of the
-// hub bin: tile t covers in-edges [tile_k[t], tile_k[t] + kPrTile) of tile_v[t].
-struct PrPlan {
-  int32_t *bins = nullptr;
-  int32_t cnt[3] = {0, 0, 0};
-  int32_t *hubs = nullptr, *first = nullptr, *tile_v = nullptr, *tile_k = nullptr;
-  float *partial = nullptr;
-  int32_t ntiles = 0;
-};
-
-static gg_status pr_plan(gg_graph *g, const GraphStore &t, PrPlan *P) {
+// The classes' ranges and the hubs' tiles.  Hubs are few: their tile list is laid
+// out on the host.
+static gg_status pr_plan(gg_graph *g, const GraphStore &t, PrIter *P) {
   const int32_t V = g->csr.V;
+  cudaStream_t st = g->stream;
   void *p = nullptr;
-  GG_TRY(scratch_get(g, 1, sizeof(int32_t) * (3 * (size_t)V + 16), &p));
-  P->bins = (int32_t *)p;
-  int32_t *cnt = P->bins + 3 * (size_t)V + 4;
-  GG_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * 3, g->stream));
+  GG_TRY(scratch_get(g, 3, sizeof(int32_t) * 2, &p));
   note_launch();
-  k_pr_bin<<<g->sm_count * 8, 256, 0, g->stream>>>(t.off, V, P->bins, cnt);
+  k_pr_bounds<<<1, 32, 0, st>>>(t.off, V, (int32_t *)p);
   GG_CUDA(cudaGetLastError());
-  GG_CUDA(cudaMemcpyAsync(P->cnt, cnt, sizeof(int32_t) * 3, cudaMemcpyDeviceToHost, g->stream));
-  GG_CUDA(cudaStreamSynchronize(g->stream));
-  const int32_t nh = P->cnt[2];
+  int32_t bounds[2];
+  GG_CUDA(cudaMemcpyAsync(bounds, p, sizeof(bounds), cudaMemcpyDeviceToHost, st));
+  GG_CUDA(cudaStreamSynchronize(st));
+  const int32_t nh = bounds[0];
+  P->nh = nh;
+  P->mid = bounds[1];
+  P->V = V;
+  P->mid_blocks = ceil_div(bounds[1] - nh, kPrThreads / 32 * kPrMidPer);
+  P->ntiles = 0;
   if (nh == 0) return GG_OK;
-  // hubs are few: their tile list is laid out on the host, in vertex order
-  std::vector<int32_t> hubs(nh), lo(nh), hi(nh);
-  GG_CUDA(cudaMemcpy(hubs.data(), P->bins + 2 * (size_t)V, sizeof(int32_t) * nh, cudaMemcpyDeviceToHost));
-  std::sort(hubs.begin(), hubs.end());
-  {  // in-list bounds of the hubs, gathered on the device
-    GG_TRY(scratch_get(g, 3, sizeof(int32_t) * 3 * (size_t)nh, &p));
-    int32_t *hd = (int32_t *)p, *bounds = hd + nh;
-    GG_CUDA(cudaMemcpyAsync(hd, hubs.data(), sizeof(int32_t) * nh, cudaMemcpyHostToDevice, g->stream));
-    note_launch();
-    k_pr_hub_bounds<<<std::max(1, std::min(ceil_div(nh, 256), g->sm_count)), 256, 0, g->stream>>>(t.off, hd, nh,
-                                                                                                   bounds);
-    GG_CUDA(cudaGetLastError());
-    std::vector<int32_t> b2(2 * (size_t)nh);
-    GG_CUDA(cudaMemcpyAsync(b2.data(), bounds, sizeof(int32_t) * b2.size(), cudaMemcpyDeviceToHost, g->stream));
-    GG_CUDA(cudaStreamSynchronize(g->stream));
-    for (int32_t i = 0; i < nh; ++i) {
-      lo[i] = b2[2 * (size_t)i];
-      hi[i] = b2[2 * (size_t)i + 1];
+  std::vector<int32_t> off(nh + 1), plan(nh + 1, 0), tv, tk;
+  GG_CUDA(cudaMemcpyAsync(off.data(), t.off, sizeof(int32_t) * off.size(), cudaMemcpyDeviceToHost, st));
+  GG_CUDA(cudaStreamSynchronize(st));
+  for (int32_t v = 0; v < nh; ++v) {
+    plan[v] = (int32_t)tv.size();
+    for (int64_t k = off[v]; k < off[v + 1]; k += kPrTile) {
+      tv.push_back(v);
+      tk.push_back((int32_t)k);
     }
   }
-  std::vector<int32_t> tv, tk, first(nh + 1, 0);
-  for (int32_t i = 0; i < nh; ++i) {
-    first[i] = (int32_t)tv.size();
-    for (int32_t k = lo[i]; k < hi[i]; k += kPrTile) {
-      tv.push_back(hubs[i]);
-      tk.push_back(k);
-    }
-  }
-  first[nh] = (int32_t)tv.size();
-  P->ntiles = (int32_t)tv.size();
-  // layout: hubs[nh] first[nh+1] tile_v[ntiles] tile_k[ntiles] partial[ntiles]
-  const size_t words = (size_t)nh + first.size() + 3 * tv.size();
-  GG_TRY(scratch_get(g, 2, sizeof(int32_t) * words, &p));
-  P->hubs = (int32_t *)p;
-  P->first = P->hubs + nh;
-  P->tile_v = P->first + first.size();
-  P->tile_k = P->tile_v + tv.size();
-  P->partial = reinterpret_cast<float *>(P->tile_k + tv.size());
-  GG_CUDA(cudaMemcpyAsync(P->hubs, hubs.data(), sizeof(int32_t) * nh, cudaMemcpyHostToDevice, g->stream));
-  GG_CUDA(cudaMemcpyAsync(P->first, first.data(), sizeof(int32_t) * first.size(), cudaMemcpyHostToDevice,
-                          g->stream));
-  GG_CUDA(cudaMemcpyAsync(P->tile_v, tv.data(), sizeof(int32_t) * tv.size(), cudaMemcpyHostToDevice, g->stream));
-  GG_CUDA(cudaMemcpyAsync(P->tile_k, tk.data(), sizeof(int32_t) * tk.size(), cudaMemcpyHostToDevice, g->stream));
-  GG_CUDA(cudaStreamSynchronize(g->stream));  // the host vectors go out of scope
+  const int32_t ntiles = (int32_t)tv.size();
+  plan[nh] = ntiles;
+  plan.insert(plan.end(), tv.begin(), tv.end());
+  plan.insert(plan.end(), tk.begin(), tk.end());
+  // layout: first[nh + 1] tile_v[ntiles] tile_k[ntiles], partial[ntiles] on an
+  // 8-byte boundary, done[nh]
+  const size_t words = (plan.size() + 1) / 2 * 2;
+  GG_TRY(scratch_get(g, 2, sizeof(int32_t) * (words + 2 * (size_t)ntiles + (size_t)nh), &p));
+  int32_t *d = (int32_t *)p;
+  GG_CUDA(cudaMemcpyAsync(d, plan.data(), sizeof(int32_t) * plan.size(), cudaMemcpyHostToDevice, st));
+  P->first = d;
+  P->tile_v = d + nh + 1;
+  P->tile_k = P->tile_v + ntiles;
+  P->partial = reinterpret_cast<double *>(d + words);
+  P->done = d + words + 2 * (size_t)ntiles;
+  P->ntiles = ntiles;
+  GG_CUDA(cudaMemsetAsync(P->done, 0, sizeof(int32_t) * (size_t)nh, st));
+  GG_CUDA(cudaStreamSynchronize(st));  // the host vector goes out of scope
   return GG_OK;
 }
 
@@ -228,38 +209,25 @@ gg_status pagerank_pull_twc(gg_graph *g, int32_t iters, float damping, float *ra
   const GraphStore &t = g->symmetric ? g->rel->g : g->rel->csc;  // in-lists in new ids
   float *rank = nullptr;  // ranks in new ids
   GG_TRY(scratch_get_app(g, 4, sizeof(float) * std::max(V, 1), (void **)&rank));
-  PrPlan P;
+  PrIter P{};
   GG_TRY(pr_plan(g, t, &P));
   cudaStream_t st = g->stream;
   const float inv_v = (float)(1.0 / V);
   note_launch();
   k_pr_init<<<g->sm_count * 8, 256, 0, st>>>(g->rel->g.off, V, inv_v, rank, contrib2);
-  PrArgs a{};
+  PrArgs &a = P.a;
   a.toff = t.off;
   a.tsrc = t.dst;
   a.off = g->rel->g.off;  // out-degrees in new ids
   a.rank = rank;
   a.beta = (float)((1.0 - (double)damping) / V);  // pr.cpp:37
   a.damp = damping;
-  const int32_t nh = P.cnt[2];
+  const int blocks = std::max(1, P.ntiles + P.mid_blocks + ceil_div(V - P.mid, kPrThreads));
   for (int32_t it = 0; it < iters; ++it) {
     a.contrib = contrib2 + (size_t)(it & 1) * V;
     a.contrib_next = contrib2 + (size_t)((it + 1) & 1) * V;
-    if (P.cnt[0]) {
-      note_launch();
-      k_pr_small<<<g->sm_count * 8, 256, 0, st>>>(a, P.bins, P.cnt[0]);
-    }
-    if (P.cnt[1]) {
-      note_launch();
-      k_pr_mid<<<g->sm_count * 8, 256, 0, st>>>(a, P.bins + V, P.cnt[1]);
-    }
-    if (nh) {
-      note_launch();
-      k_pr_tile<<<std::min(P.ntiles, g->sm_count * 4), 512, 0, st>>>(a, P.tile_v, P.tile_k, P.ntiles, P.partial);
-      note_launch();
-      k_pr_hub_finish<<<std::max(1, std::min(ceil_div(nh, 128), g->sm_count)), 128, 0, st>>>(a, P.hubs, P.first,
-                                                                                               nh, P.partial);
-    }
+    note_launch();
+    k_pr_iter<<<blocks, kPrThreads, 0, st>>>(P);
   }
   note_launch();
   k_pr_unperm<<<g->sm_count * 8, 256, 0, st>>>(rank, g->rel->perm, V, rank_out);
