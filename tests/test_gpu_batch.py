@@ -357,6 +357,33 @@ def test_sssp_batch_light_and_heavy_edges(delta):
     g.close()
 
 
+@pytest.mark.parametrize("delta", [1, 50, 100000])
+@pytest.mark.parametrize("edge_parallel_max", [-1, 6])
+def test_sssp_batch_remainders_of_an_edge_group(delta, edge_parallel_max):
+    """Lists of 1 to 70 edges, every remainder of a group of 32 and of its quads,
+    active for all 32 sources at once and improving for all, some or none."""
+    from easy_graphit_gb300 import set_batch_tuning
+    rng = np.random.default_rng(17)
+    u, v = [], []
+    for d in range(1, 71):                     # vertex 31 + d: d edges
+        u += [31 + d] * d
+        v += list(rng.choice(np.arange(102, 260), d, replace=False))
+    for s in range(32):                        # every source reaches every such list
+        u += [s] * 70
+        v += list(range(32, 102))
+    u += list(range(102, 260))                 # and the targets lead back into them
+    v += list(rng.integers(32, 102, 158))
+    w = rng.integers(1, 200, len(u)).astype(np.int32)
+    hg = HostGraph.from_edges(260, np.array(u, np.int32), np.array(v, np.int32), w)
+    g = GraphT(hg)
+    off, dst, ww = np.array(hg.offsets), np.array(hg.dst), np.array(hg.weights)
+    set_batch_tuning(g, "sssp", chunk=64, edge_parallel_max=edge_parallel_max)
+    dist, _ = sssp_batch(g, list(range(32)), delta)
+    for s in range(32):
+        np.testing.assert_array_equal(dist[s], oracle.sssp_dijkstra(off, dst, ww, s), err_msg=f"source {s}")
+    g.close()
+
+
 @pytest.mark.parametrize("delta", [1, 32, 1000])
 def test_sssp_one_cta_per_source_forced_on_a_graph_with_hubs(delta):
     """The per-source form (one CTA per source, bucket ring) forced onto a
