@@ -125,10 +125,6 @@ __device__ __forceinline__ BqStep bq_decide(const BqLoop &s, const int32_t *ctl,
   return nh > 0 ? BqStep{BQ_HIMIN, nh, 0} : BqStep{BQ_DONE, 0, 0};
 }
 
-// Mark of the vertices relax step `step` queues (the last step's for its hubs);
-// a mesh session's queue marks lie between them.
-__device__ __forceinline__ int32_t bq_near_tag(int32_t step) { return INT_MIN + 2 + 2 * step; }
-
 // One step, CTA `rank` of `nparts` taking its share.
 // `ctl` holds the control words: global memory in grid mode, CTA 0's shared
 // copy in a one-CTA session.  `stages`: three in shared memory, empty.
@@ -275,17 +271,17 @@ __device__ __forceinline__ void bq_step(BqLoop &s, const BqArgs &a, const BqStep
 // kMeshMaxDegree): the same rule and the same counts, with the frontier and the
 // low pile in shared memory.  A bucket is bound by its dependent L2 round trips.
 // In bq_step's form an advance is two steps (minimum, split) and a relax reads
-// queue, offsets, edges, targets and answers of the stamp exchanges one after the
+// queue, offsets, edges, targets and answers of the stamp claims one after the
 // other, 15 to 20 trips and as many barriers a bucket; here
 //  * an advance reads the pile's priorities once (one trip), reduces them and
 //    splits the pile from shared memory;
 //  * a relax has two trips: a vertex's edges, then the targets' distances,
 //    stamps and edge ranges together; what it queues carries priority and edge
 //    range.  Four lanes share a vertex, an edge each;
-//  * a park decides by the stamp it read and marks the vertex with a plain
-//    store: a vertex parked twice in one round may be listed twice, which the
-//    exchange at the end of the session undoes: the piles and the queue in
-//    global memory get a vertex once.
+//  * a park decides by the stamp it read and raises the stamp without waiting
+//    for the answer: a vertex parked twice in one round may be listed twice,
+//    which the claims at the end of the session undo: the piles and the queue
+//    in global memory get a vertex once.
 // An entry that an advance takes or finds settled can never be parked again
 // (its distance stays below every later cutoff), so a session needs one mark.
 // 700 x 501 grid, delta 128 (1,344 buckets, 3 relaxes each): 24-29 -> 12.9 ms;
@@ -319,13 +315,12 @@ __device__ __forceinline__ int32_t mesh_places(int32_t to, int32_t *cnt) {
 
 // Buffered high parks to the high pile of generation gh; the whole CTA calls it
 // between barriers.
-__device__ __forceinline__ void mesh_flush_high(const BqLoop &s, const BqArgs &a, int32_t *sctl, BqMeshSmem &m,
-                                                int32_t mark_lo) {
-  const int32_t n = min(m.n_hi, kMeshHigh), tag = bq_hi_tag(s.gh), lo_tag = bq_lo_tag(s.g);
+__device__ __forceinline__ void mesh_flush_high(const BqLoop &s, const BqArgs &a, int32_t *sctl, BqMeshSmem &m) {
+  const int32_t n = min(m.n_hi, kMeshHigh);
+  const uint32_t tag = bq_hi_tag(s.gh);
   for (int32_t i = threadIdx.x; i < n; i += blockDim.x) {
-    const int32_t v = m.hi[i], t = __ldcg(a.b.stamp + v);
-    if (t == mark_lo || t == lo_tag || t == bq_lo_tag(s.g + 1)) continue;  // since parked lower
-    if (atomicExch(a.b.stamp + v, tag) == tag) continue;
+    const int32_t v = m.hi[i];
+    if (stamp_claim(a.b.stamp, v, tag) >= tag) continue;  // listed, or since parked lower
     const int32_t pos = agg_inc(sctl + BQ_HI + (s.gh & 1));
     if (pos < a.b.V)
       a.b.hi[s.gh & 1][pos] = v;
@@ -336,14 +331,12 @@ __device__ __forceinline__ void mesh_flush_high(const BqLoop &s, const BqArgs &a
   if (threadIdx.x == 0) m.n_hi = 0;
 }
 
-struct BqMeshMarks {
-  int32_t lo_tag, hi_tag, next_tag, mark_lo, mark_hi, spill;
-};
-
-// A window vertex to the frontier queue in global memory, once a session: it is
-// below the cutoff and never parks again, so its stamp is free to say so.
-__device__ __forceinline__ void mesh_spill(const BqArgs &a, BqMeshSmem &m, int32_t tag, int32_t *q, int32_t v) {
-  if (atomicExch(a.b.stamp + v, tag) == tag) return;
+// A window vertex to the frontier queue in global memory, once a session: `step`
+// is the relax step that will read the queue.  A session spills in its last round
+// only, so that step is the same for all of its spills.
+__device__ __forceinline__ void mesh_spill(const BqArgs &a, BqMeshSmem &m, int32_t step, int32_t *q, int32_t v) {
+  const uint32_t tag = bq_spill_tag(step);
+  if (stamp_claim(a.b.stamp, v, tag) >= tag) return;
   const int32_t qp = atomicAdd(&m.spill, 1);
   if (qp < a.qcap)
     q[qp] = v;
@@ -358,16 +351,20 @@ __device__ __forceinline__ void mesh_spill(const BqArgs &a, BqMeshSmem &m, int32
 // share a vertex, an edge each, J vertices of a lane in flight.
 template <int J>
 __device__ __forceinline__ void mesh_relax_pass(const BqLoop &s, const BqArgs &a, int32_t *sctl, BqMeshSmem &m,
-                                                const BqMeshMarks &mk, int32_t n, int32_t in, int32_t L, int32_t U,
+                                                int32_t n, int32_t in, int32_t L, int32_t U,
                                                 int32_t *n_out, int32_t *q) {
   const int32_t per = blockDim.x >> 2, lane = threadIdx.x & 31, lo_next = (s.g + 1) & 1;
+  const uint32_t lo_tag = bq_lo_tag(s.g), lo_mark = bq_lo_mark(s.g), next_tag = bq_lo_tag(s.g + 1);
+  const uint32_t hi_mark = bq_hi_mark(s.gh), hi_tag = bq_hi_tag(s.gh);
+  uint32_t *const stamps = reinterpret_cast<uint32_t *>(a.b.stamp);
   int32_t *cnt = lane == 0 ? n_out : (lane == 1 ? &m.n_lo[L] : &m.n_hi);
   // a warp without a vertex leaves at once: in a round of a few vertices the
   // others' empty instructions would cost more than the loads
   for (int32_t w0 = (threadIdx.x & ~31) >> 2; w0 < n; w0 += J * per) {
     bool more = true;
     for (int32_t hop = threadIdx.x & 3; more; hop += 4) {
-      int32_t d[J], np[J], prev[J], st[J], db[J], de[J];
+      int32_t d[J], np[J], prev[J], db[J], de[J];
+      uint32_t st[J];
       more = false;
 #pragma unroll
       for (int j = 0; j < J; ++j) {
@@ -383,7 +380,7 @@ __device__ __forceinline__ void mesh_relax_pass(const BqLoop &s, const BqArgs &a
       for (int j = 0; j < J; ++j) {
         const bool ok = d[j] >= 0;
         prev[j] = ok ? __ldcg(a.dist + d[j]) : INT_MIN;
-        st[j] = ok ? __ldcg(a.b.stamp + d[j]) : 0;
+        st[j] = ok ? __ldcg(stamps + d[j]) : 0u;
         db[j] = ok ? __ldg(a.g.off + d[j]) : 0;
         de[j] = ok ? __ldg(a.g.off + d[j] + 1) : 0;
       }
@@ -397,9 +394,9 @@ __device__ __forceinline__ void mesh_relax_pass(const BqLoop &s, const BqArgs &a
           if (p < U)
             to = 0;
           else if (p < s.hz)
-            to = st[j] == mk.lo_tag || st[j] == mk.mark_lo || st[j] == mk.next_tag ? -1 : 1;
+            to = st[j] >= lo_tag ? -1 : 1;
           else
-            to = st[j] == mk.hi_tag || st[j] == mk.mark_hi ? -1 : 2;
+            to = st[j] >= hi_mark ? -1 : 2;
         }
         const int32_t pos = mesh_places(to, cnt);
         if (to == 0) {
@@ -407,15 +404,15 @@ __device__ __forceinline__ void mesh_relax_pass(const BqLoop &s, const BqArgs &a
             m.near_[in ^ 1][pos] = make_int4(v, p, db[j], de[j]);
           } else {
             m.full = 1;
-            mesh_spill(a, m, mk.spill, q, v);
+            mesh_spill(a, m, s.relax + 1, q, v);
           }
         } else if (to == 1) {
           if (pos < kMeshLow) {
-            a.b.stamp[v] = mk.mark_lo;
+            atomicMax(stamps + v, lo_mark);
             m.lo[L][pos] = make_int4(v, p, db[j], de[j]);
           } else {
             m.full = 1;
-            if (atomicExch(a.b.stamp + v, mk.next_tag) != mk.next_tag) {
+            if (stamp_claim(a.b.stamp, v, next_tag) < next_tag) {
               const int32_t gp = atomicAdd(sctl + BQ_LO + lo_next, 1);
               if (gp < a.b.V)
                 a.b.lo[lo_next][gp] = v;
@@ -425,9 +422,9 @@ __device__ __forceinline__ void mesh_relax_pass(const BqLoop &s, const BqArgs &a
           }
         } else if (to == 2) {
           if (pos < kMeshHigh) {
-            a.b.stamp[v] = mk.mark_hi;
+            atomicMax(stamps + v, hi_mark);
             m.hi[pos] = v;
-          } else if (atomicExch(a.b.stamp + v, mk.hi_tag) != mk.hi_tag) {
+          } else if (stamp_claim(a.b.stamp, v, hi_tag) < hi_tag) {
             const int32_t gp = atomicAdd(sctl + BQ_HI + (s.gh & 1), 1);
             if (gp < a.b.V)
               a.b.hi[s.gh & 1][gp] = v;
@@ -441,15 +438,12 @@ __device__ __forceinline__ void mesh_relax_pass(const BqLoop &s, const BqArgs &a
   }
 }
 
-// Runs relaxes and advances while they fit; `session` numbers the sessions of
-// the run (its marks).  On return the loop state and control words are as after
-// a bq_step, ready for bq_decide.
+// Runs relaxes and advances while they fit.  On return the loop state and control
+// words are as after a bq_step, ready for bq_decide.
 __device__ __forceinline__ void bq_mesh_session(BqLoop &s, const BqArgs &a, int32_t *sctl, BqMeshSmem &m,
-                                                int32_t session, int32_t n, uint64_t t0) {
-  const int32_t mark_lo = -2 * session - 1, mark_hi = -2 * session - 2;  // below every pile tag
-  const int32_t lo_tag = bq_lo_tag(s.g), hi_tag = bq_hi_tag(s.gh), next_tag = bq_lo_tag(s.g + 1);
+                                                int32_t n, uint64_t t0) {
+  const uint32_t next_tag = bq_lo_tag(s.g + 1);
   const int32_t lo_next = (s.g + 1) & 1, T = blockDim.x, lane = threadIdx.x & 31;
-  const BqMeshMarks mk{lo_tag, hi_tag, next_tag, mark_lo, mark_hi, bq_near_tag(0) + 2 * session - 1};
   int32_t *const q = s.in ? a.q1 : a.q0;
   int32_t nl = sctl[BQ_LO + (s.g & 1)];
   for (int32_t i = threadIdx.x; i < n; i += T) {
@@ -478,9 +472,9 @@ __device__ __forceinline__ void bq_mesh_session(BqLoop &s, const BqArgs &a, int3
       int32_t *n_out = &m.n_near[in ^ 1];
       // a second vertex per lane only where the frontier has that many
       if (n <= T >> 2)
-        mesh_relax_pass<1>(s, a, sctl, m, mk, n, in, L, U, n_out, q);
+        mesh_relax_pass<1>(s, a, sctl, m, n, in, L, U, n_out, q);
       else
-        mesh_relax_pass<2>(s, a, sctl, m, mk, n, in, L, U, n_out, q);
+        mesh_relax_pass<2>(s, a, sctl, m, n, in, L, U, n_out, q);
       s.relax++;
       if (threadIdx.x == 0 && (round & 15) == 0)  // the session's time slice, and overflows
         m.quit = globaltimer_ns() - t0 > kSoloSliceNs || (*(volatile int32_t *)a.err & DEV_ERR_OVERFLOW) != 0;
@@ -491,7 +485,7 @@ __device__ __forceinline__ void bq_mesh_session(BqLoop &s, const BqArgs &a, int3
       const bool flush = m.n_hi > kMeshHigh / 2;
       __syncthreads();
       if (threadIdx.x == 0) m.n_near[in ^ 1] = 0;
-      if (flush) mesh_flush_high(s, a, sctl, m, mark_lo);
+      if (flush) mesh_flush_high(s, a, sctl, m);
       if (leave) break;
     } else {
       // ---- advance: the exact minimum of the live entries, then the split
@@ -536,7 +530,7 @@ __device__ __forceinline__ void bq_mesh_session(BqLoop &s, const BqArgs &a, int3
             m.near_[in][pos] = x;
           } else {
             m.full = 1;
-            mesh_spill(a, m, mk.spill, q, x.x);
+            mesh_spill(a, m, s.relax, q, x.x);
           }
         }
       }
@@ -551,18 +545,18 @@ __device__ __forceinline__ void bq_mesh_session(BqLoop &s, const BqArgs &a, int3
   }
   // ---- back to the queues and piles in global memory, a vertex once per pile
   __syncthreads();
-  mesh_flush_high(s, a, sctl, m, mark_lo);
+  mesh_flush_high(s, a, sctl, m);
   nl = min(m.n_lo[L], kMeshLow);
   for (int32_t i = threadIdx.x; i < nl; i += T) {
     const int32_t v = m.lo[L][i].x;
-    if (atomicExch(a.b.stamp + v, next_tag) == next_tag) continue;
+    if (stamp_claim(a.b.stamp, v, next_tag) >= next_tag) continue;
     const int32_t pos = agg_inc(sctl + BQ_LO + lo_next);
     if (pos < a.b.V)
       a.b.lo[lo_next][pos] = v;
     else
       atomicOr(a.err, DEV_ERR_OVERFLOW);
   }
-  for (int32_t i = threadIdx.x; i < n; i += T) mesh_spill(a, m, mk.spill, q, m.near_[in][i].x);
+  for (int32_t i = threadIdx.x; i < n; i += T) mesh_spill(a, m, s.relax, q, m.near_[in][i].x);
   __syncthreads();
   n = (int32_t)min((int64_t)m.spill, a.qcap);
   s.g++;

@@ -10,9 +10,9 @@
 // the window's cutoff got that priority from a relaxation at or above the
 // cutoff of its own time (cutoffs only grow), and such a relaxation parks it
 // (DFar::park).  Parking goes to the low pile when the priority is below the
-// horizon and to the high pile otherwise; the tag in stamp[v] keeps a vertex
-// listed at most once per pile generation, so a pile never holds more than V
-// entries.  An entry whose vertex has since dropped below the cutoff was
+// horizon and to the high pile otherwise; stamp[v] keeps a vertex listed at most
+// once per pile generation, so a pile never holds more than V entries (the order
+// of stamps below).  An entry whose vertex has since dropped below the cutoff was
 // queued at that time and is stale; an advance skips it.
 //
 // An advance takes the exact minimum over the low pile (bq_pile_min): every
@@ -21,7 +21,7 @@
 // frontier and the rest to the next low-pile generation.  A window that
 // reaches past the horizon also splits the high pile, with a new horizon
 // above the window: a vertex parked high and later low sits on both piles
-// then, so appends to the low pile exchange the tag and keep one copy.  When
+// then, so appends to the low pile claim the stamp and keep one copy.  When
 // the low pile holds no live entry the high pile is scanned instead (a
 // refill): its minimum starts the window, the new horizon is set a few buckets
 // above it, and the split sends window entries to the frontier, entries below
@@ -34,10 +34,26 @@
 
 namespace gg {
 
-// Pile tags: even for low-pile generations, odd for high ones; 0 = never
-// parked (stamps are cleared at the start of every run).
-__host__ __device__ __forceinline__ int32_t bq_lo_tag(int32_t gen) { return 2 * gen + 2; }
-__host__ __device__ __forceinline__ int32_t bq_hi_tag(int32_t gen) { return 2 * gen + 1; }
+// Stamps.  Threads of one step decide from distances they read before the others'
+// updates, so one may queue a vertex while another, on an older distance, parks
+// it, in any order.  A stamp therefore only grows: a claim is an atomicMax
+// (stamp_claim) and appends when it raised the stamp.  In rising order:
+//   0                    never parked (stamps are cleared at the start of every run)
+//   hi_mark, hi_tag      buffered for / on the high pile of a generation
+//   lo_tag, lo_mark      on the low pile of a generation / in the list of the mesh
+//                        session that works on it (bq_loop.cuh)
+//   spill_tag, near_tag  queued by a mesh session before / by a relax step
+// What a later claim is refused for is always the older decision: a vertex below the
+// cutoff stays below every later one, and one below the horizon, which only grows too,
+// never goes high again.  With exchanged tags a park after a near claim found another
+// tag and appended again, several times a step where many threads lower one vertex
+// (complete graph of 400 vertices, weights to 255, delta 32: more than V entries).
+__host__ __device__ __forceinline__ uint32_t bq_hi_tag(int32_t gen) { return 2u * (uint32_t)gen + 2u; }
+__host__ __device__ __forceinline__ uint32_t bq_hi_mark(int32_t gen) { return bq_hi_tag(gen) - 1u; }
+__host__ __device__ __forceinline__ uint32_t bq_lo_tag(int32_t gen) { return (1u << 30) + 2u * (uint32_t)gen; }
+__host__ __device__ __forceinline__ uint32_t bq_lo_mark(int32_t gen) { return bq_lo_tag(gen) + 1u; }
+__host__ __device__ __forceinline__ uint32_t bq_near_tag(int32_t step) { return (1u << 31) + 2u + 2u * (uint32_t)step; }
+__host__ __device__ __forceinline__ uint32_t bq_spill_tag(int32_t next_step) { return bq_near_tag(next_step) - 1u; }
 
 __host__ __device__ __forceinline__ int32_t bq_clamp(int64_t x) {
   return x >= (int64_t)INT_MAX ? INT_MAX : (int32_t)x;
@@ -110,9 +126,9 @@ __device__ __forceinline__ void bq_pile_min(const int32_t *__restrict__ pile, in
 struct BqSplitOut {
   int32_t *stamp;
   int32_t *lo, *lo_cnt;
-  int32_t lo_tag;
+  uint32_t lo_tag;
   int32_t *hi, *hi_cnt;  // null: everything goes to the low pile
-  int32_t hi_tag;
+  uint32_t hi_tag;
   int32_t horizon;
   int32_t *fill;         // optional count of entries sent to the low pile
   int32_t cap;
@@ -153,14 +169,14 @@ __device__ __forceinline__ void bq_pile_split(const int32_t *__restrict__ pile, 
         front.sparse(v);
       } else if (!o.hi || p < o.horizon) {
         if (o.dedup) {
-          if (atomicExch(o.stamp + v, o.lo_tag) == o.lo_tag) continue;
+          if (stamp_claim(o.stamp, v, o.lo_tag) >= o.lo_tag) continue;
         } else {
-          o.stamp[v] = o.lo_tag;
+          o.stamp[v] = (int32_t)o.lo_tag;
         }
         pile_append(o.lo_stage, o.lo, o.lo_cnt, o.cap, v, err);
         ++fill;
       } else {
-        o.stamp[v] = o.hi_tag;
+        o.stamp[v] = (int32_t)o.hi_tag;
         pile_append(o.hi_stage, o.hi, o.hi_cnt, o.cap, v, err);
       }
     }

@@ -209,31 +209,36 @@ __device__ __forceinline__ void pile_append(Stage *st, int32_t *pile, int32_t *c
     atomicOr(err, DEV_ERR_OVERFLOW);
 }
 
+// Raises v's stamp to `tag` and returns what it was: v is this caller's to append
+// when that was below the tag.
+__device__ __forceinline__ uint32_t stamp_claim(int32_t *stamp, int32_t v, uint32_t tag) {
+  return atomicMax(reinterpret_cast<uint32_t *>(stamp) + v, tag);
+}
+
 // Far piles of the single-source delta-stepping queue (bucket_queue.cuh).  A
 // relaxation that lowers P[v] to p at or above the window's cutoff parks v on
 // the low pile (p below the horizon) or the high pile.  stamp[v] holds the tag
 // of the pile generation that already lists v, so each vertex is listed at most
-// once per pile: the exchange that writes the tag decides who appends.  With
-// stamp == nullptr nothing is parked (a plain edgeset.apply of the relax UDF).
+// once per pile: the claim that raises the stamp to the tag decides who appends
+// (the order of tags is in bucket_queue.cuh).  With stamp == nullptr nothing is
+// parked (a plain edgeset.apply of the relax UDF).
 struct DFar {
   int32_t *stamp;           // [V]
   int32_t *lo, *lo_cnt;     // low pile of the current generation and its count
   int32_t *hi, *hi_cnt;     // high pile of the current generation and its count
-  int32_t lo_tag, hi_tag;
+  uint32_t lo_tag, hi_tag;
   int32_t horizon;          // p < horizon -> low pile
   int32_t cap;              // entries a pile can hold (V)
   int32_t *err;
   Stage *lo_stage, *hi_stage;  // shared memory, or null: append directly
   // Mark of this step's frontier, or 0: improvements below the cutoff queue their
-  // vertex every time.  With it a vertex is queued once a step.  Such a vertex
-  // stays below every later cutoff and never parks again, so its stamp is free.
-  int32_t near_tag;
+  // vertex every time.  With it a vertex is queued once a step, and a park that
+  // another thread of the step decided on an older distance is refused.
+  uint32_t near_tag;
 
-  // claim: marks v for its pile; append, when the mark before it was another.
-  __device__ __forceinline__ int32_t tag_of(int32_t p) const { return p < horizon ? lo_tag : hi_tag; }
-  __device__ __forceinline__ int32_t claim(int32_t v, int32_t p) const { return atomicExch(stamp + v, tag_of(p)); }
+  __device__ __forceinline__ uint32_t tag_of(int32_t p) const { return p < horizon ? lo_tag : hi_tag; }
   __device__ __forceinline__ void park(int32_t v, int32_t p) const {
-    if (claim(v, p) != tag_of(p)) append(v, p);
+    if (stamp_claim(stamp, v, tag_of(p)) < tag_of(p)) append(v, p);
   }
   __device__ __forceinline__ void append(int32_t v, int32_t p) const {
     if (p < horizon)

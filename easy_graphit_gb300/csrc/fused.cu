@@ -158,7 +158,7 @@ __device__ __forceinline__ void bq_publish(const BqLoop &s, int32_t *ctl) {
 // global memory at its end.  The whole CTA calls it.
 template <int LB>
 __device__ __forceinline__ void bq_solo(BqLoop &s, const BqArgs &a, BqStep st, int4 *smem, int32_t *red,
-                                        int32_t *flag, int32_t *sctl, int32_t *session) {
+                                        int32_t *flag, int32_t *sctl) {
   for (int i = threadIdx.x; i < BQ_STOP; i += blockDim.x) sctl[i] = __ldcg(a.b.ctl + i);
   uint64_t t0 = 0;
   if (threadIdx.x == 0) t0 = globaltimer_ns();
@@ -167,7 +167,7 @@ __device__ __forceinline__ void bq_solo(BqLoop &s, const BqArgs &a, BqStep st, i
     const int32_t near_n = st.kind == BQ_RELAX ? st.work : 0;
     if (a.mesh && (st.kind == BQ_RELAX || st.kind == BQ_LOMIN) && near_n <= kMeshNear / 4 * 3 &&
         sctl[BQ_LO + (s.g & 1)] <= kMeshLow) {
-      bq_mesh_session(s, a, sctl, *reinterpret_cast<BqMeshSmem *>(smem), ++*session, near_n, t0);
+      bq_mesh_session(s, a, sctl, *reinterpret_cast<BqMeshSmem *>(smem), near_n, t0);
       steps |= 7;  // long enough to check the clock
     } else {
       bq_step<LB>(s, a, st, sctl, 0, 1, smem, red, nullptr);
@@ -199,7 +199,6 @@ __global__ void __launch_bounds__(1024) k_sssp_bq(BqArgs a) {
   __syncthreads();
   BqLoop s{1, 0, 0, 0, 0, bq_clamp((int64_t)a.width0 * a.delta), a.width0, 0, 0, 0, 0};
   int32_t *stop = a.b.ctl + BQ_STOP;
-  int32_t session = 0;  // mesh sessions run (CTA 0)
   LoopClock clk;
   clk.start(a.loop_limit_ns);
   // Grid iterations (one barrier each), numbered for the stop word: the clock
@@ -216,7 +215,7 @@ __global__ void __launch_bounds__(1024) k_sssp_bq(BqArgs a) {
       // has taken its decision from them and arrived at the barrier.
       if (blockIdx.x == 0) {
         if (grid_wait_others(a.bar, gridDim.x, a.err, a.timeout_ns))
-          bq_solo<LB>(s, a, st, smem, red, red + 32, sctl, &session);
+          bq_solo<LB>(s, a, st, smem, red, red + 32, sctl);
         else
           bq_publish(s, a.b.ctl);
       }

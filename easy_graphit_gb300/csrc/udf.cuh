@@ -82,23 +82,23 @@ struct USssp {
           asm volatile("red.relaxed.gpu.global.min.s32 [%0], %1;" ::"l"(__cvta_generic_to_global(dist + d[j])),
                        "r"(np[j])
                        : "memory");
-      // The stamp exchanges of the batch go out together: their answers decide
+      // The stamp claims of the batch go out together: their answers decide
       // the appends, and one after the other they would be B round trips.
       // A near vertex is claimed too where the loop marks its steps (near_tag):
       // threads that lower one vertex together would each queue it, the copies be
       // relaxed together and multiply.
-      int32_t was[B];
+      uint32_t was[B];
 #pragma unroll
       for (int j = 0; j < B; ++j) {
-        const int32_t tag = np[j] < cutoff ? far.near_tag : far.tag_of(np[j]);
-        was[j] = prev[j] > np[j] && far.stamp && tag ? atomicExch(far.stamp + d[j], tag) : 0;
+        const uint32_t tag = np[j] < cutoff ? far.near_tag : far.tag_of(np[j]);
+        was[j] = prev[j] > np[j] && far.stamp && tag ? stamp_claim(far.stamp, d[j], tag) : 0u;
       }
 #pragma unroll
       for (int j = 0; j < B; ++j) {
         if (prev[j] <= np[j]) continue;
         if (np[j] < cutoff) {
-          if (!far.near_tag || was[j] != far.near_tag) out.push(d[j]);
-        } else if (far.stamp && was[j] != far.tag_of(np[j])) {
+          if (!far.near_tag || was[j] < far.near_tag) out.push(d[j]);
+        } else if (far.stamp && was[j] < far.tag_of(np[j])) {
           far.append(d[j], np[j]);
         }
       }
