@@ -464,8 +464,15 @@ __device__ __forceinline__ void bq_mesh_session(BqLoop &s, const BqArgs &a, int3
     sctl[BQ_LO + lo_next] = 0;  // low parks that do not fit, then the write-back
   }
   int32_t in = 0, L = 0, adv = 0, cross = INT_MAX;
-  for (int32_t round = 1;; ++round) {
+  for (int32_t rounds = 1;; ++rounds) {
     __syncthreads();
+    // The session's time slice, and overflows, on a count of all rounds; read at the
+    // end of this one, behind its barriers.  Tested in relaxes alone, on the same
+    // count, it never came up where relaxes and advances take turns (a line of unit
+    // weights at delta 1: every 16th round an advance), and only the horizon, seconds
+    // away, ended the session.
+    if (threadIdx.x == 0 && (rounds & 15) == 0)
+      m.quit = globaltimer_ns() - t0 > kSoloSliceNs || (*(volatile int32_t *)a.err & DEV_ERR_OVERFLOW) != 0;
     const int32_t U = bq_clamp((int64_t)s.cur + a.delta);
     if (n > 0) {
       // ---- relax: near_[in] -> near_[in ^ 1], lo[L], hi
@@ -476,8 +483,6 @@ __device__ __forceinline__ void bq_mesh_session(BqLoop &s, const BqArgs &a, int3
       else
         mesh_relax_pass<2>(s, a, sctl, m, n, in, L, U, n_out, q);
       s.relax++;
-      if (threadIdx.x == 0 && (round & 15) == 0)  // the session's time slice, and overflows
-        m.quit = globaltimer_ns() - t0 > kSoloSliceNs || (*(volatile int32_t *)a.err & DEV_ERR_OVERFLOW) != 0;
       __syncthreads();
       in ^= 1;
       n = min(m.n_near[in], kMeshNear);
@@ -540,7 +545,7 @@ __device__ __forceinline__ void bq_mesh_session(BqLoop &s, const BqArgs &a, int3
       adv++;
       __syncthreads();
       n = min(m.n_near[in], kMeshNear);
-      if (m.full) break;
+      if (m.full || m.quit) break;
     }
   }
   // ---- back to the queues and piles in global memory, a vertex once per pile
