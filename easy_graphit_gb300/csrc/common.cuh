@@ -280,14 +280,31 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 // gpu-scope ordering), not of bandwidth: with a generation word it took four
 // (read it, arrive, publish it, see it), 2.5 us at 304 blocks and 3.1 us at
 // 608; arriving and polling one count takes two, 1.5 us and 2.2 us.  64 bits,
-// because a loop of a 1.5 us barrier passes 2^32 arrivals within seconds.
+// because a loop of a 1.5 us barrier passes 2^32 arrivals within seconds.  The
+// wait reads without acquire semantics and one fence follows it: an acquiring
+// read drops the L1 of its SM, and with most blocks waiting it did so under the
+// ones still at work (BFS on a symmetrized R-MAT 20, a thread per vertex: 91 ms,
+// 81 without).
+//
+// `behind` runs on one thread behind the barrier, before its block goes on: loops
+// fetch the words that every thread needs (counts, the stop word) there and hand
+// them on in shared memory.  Read by every warp of the GPU they are 10^4 requests a
+// word for one line of the L2, answered one after another (BFS on a 1024^2 grid,
+// 2,046 levels of about 1,000 vertices: 24.3 ms with three words read by every warp,
+// 20.0 with two, 12.6 with one thread a block reading them).
 __device__ __forceinline__ uint64_t ld_acquire64(const uint32_t *p) {
   uint64_t v;
   asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ bool grid_barrier(uint32_t *bar, uint32_t nblocks, int32_t *err,
-                                             uint64_t timeout_ns) {
+__device__ __forceinline__ uint64_t ld_relaxed64(const uint32_t *p) {
+  uint64_t v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+template <class Behind>
+__device__ __forceinline__ bool grid_barrier_then(uint32_t *bar, uint32_t nblocks, int32_t *err,
+                                                  uint64_t timeout_ns, const Behind &behind) {
   __syncthreads();
   __shared__ int ok_s;
   if (threadIdx.x == 0) {
@@ -298,7 +315,7 @@ __device__ __forceinline__ bool grid_barrier(uint32_t *bar, uint32_t nblocks, in
     if (old + 1 != end) {
       const uint64_t t0 = globaltimer_ns();
       uint32_t spins = 0;
-      while (ld_acquire64(bar) < end) {
+      while (ld_relaxed64(bar) < end) {
         if ((++spins & 255u) == 0) {
           if (*(volatile int32_t *)err & DEV_ERR_TIMEOUT) { ok_s = 0; break; }
           if (globaltimer_ns() - t0 > timeout_ns) {
@@ -310,9 +327,13 @@ __device__ __forceinline__ bool grid_barrier(uint32_t *bar, uint32_t nblocks, in
       }
     }
     __threadfence();
+    behind();
   }
   __syncthreads();
   return ok_s != 0;
+}
+__device__ __forceinline__ bool grid_barrier(uint32_t *bar, uint32_t nblocks, int32_t *err, uint64_t timeout_ns) {
+  return grid_barrier_then(bar, nblocks, err, timeout_ns, [] {});
 }
 
 // Waits, without arriving, until every other block has arrived at the next
@@ -360,10 +381,11 @@ struct LoopClock {
       atomicOr(err, DEV_ERR_TIMEOUT);
   }
 };
-// True at the top of iteration `iter` once a stop has been set for it.
+// True at the top of iteration `iter` once a stop has been set for it: for the stop
+// word as read behind the closing barrier of the iteration before, or any time since.
+__device__ __forceinline__ bool stop_reached(int32_t stop, int32_t iter) { return stop != 0 && iter >= stop; }
 __device__ __forceinline__ bool stopped(const int32_t *stop, int32_t iter) {
-  const int32_t s = *(volatile const int32_t *)stop;
-  return s != 0 && iter >= s;
+  return stop_reached(*(volatile const int32_t *)stop, iter);
 }
 // The same stop for a reason other than the clock (block 0, before the
 // iteration's closing barrier): a sparse queue that overflowed.

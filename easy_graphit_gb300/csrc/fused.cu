@@ -92,6 +92,7 @@ template <int LB>
 __global__ void __launch_bounds__(1024) k_bfs_fused(FusedArgs a) {
   extern __shared__ int4 smem[];
   __shared__ Stage stage;
+  __shared__ int32_t s_n, s_chunks, s_stop;  // read behind a level's barrier by one thread
   if (threadIdx.x == 0) stage.n = 0;
   __syncthreads();
   int32_t *qs[2] = {a.q0, a.q1};
@@ -99,9 +100,9 @@ __global__ void __launch_bounds__(1024) k_bfs_fused(FusedArgs a) {
   int64_t level = 1;
   LoopClock clk;
   clk.start(a.loop_limit_ns);
-  int32_t n = *(volatile int32_t *)a.cnt3;
+  int32_t n = *(volatile int32_t *)a.cnt3, stop = 0;
   for (;; ++level) {
-    if (n == 0 || stopped(a.stop, (int32_t)level)) break;
+    if (n == 0 || stop_reached(stop, (int32_t)level)) break;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       a.cnt3[(level + 1) % 3] = 0;
       a.hub3[(level + 1) % 3] = 0;
@@ -114,15 +115,19 @@ __global__ void __launch_bounds__(1024) k_bfs_fused(FusedArgs a) {
     run_lb<LB>(a.g, en, n, f, out, smem, blockIdx.x, gridDim.x, hub);
     stage_flush(out);
     clk.tick(a.stop, (int32_t)level, a.err);
-    if (!grid_barrier(a.bar, gridDim.x, a.err, a.timeout_ns)) break;
-    const int32_t chunks = *(volatile int32_t *)hub.cnt;
-    n = *(volatile int32_t *)out.cnt;
-    if (chunks) {  // the level's hubs, by all CTAs
-      lb_hubs(a.g, hub, chunks, f, out, blockIdx.x, gridDim.x);
+    const auto fetch = [&] {
+      s_n = *(volatile int32_t *)out.cnt;
+      s_chunks = *(volatile int32_t *)hub.cnt;
+      s_stop = *(volatile int32_t *)a.stop;
+    };
+    if (!grid_barrier_then(a.bar, gridDim.x, a.err, a.timeout_ns, fetch)) break;
+    if (s_chunks) {  // the level's hubs, by all CTAs
+      lb_hubs(a.g, hub, s_chunks, f, out, blockIdx.x, gridDim.x);
       stage_flush(out);
-      if (!grid_barrier(a.bar, gridDim.x, a.err, a.timeout_ns)) break;
-      n = *(volatile int32_t *)out.cnt;
+      if (!grid_barrier_then(a.bar, gridDim.x, a.err, a.timeout_ns, fetch)) break;
     }
+    n = s_n;
+    stop = s_stop;
     in ^= 1;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) a.stats[0] = (int32_t)(level - 1);
@@ -611,6 +616,10 @@ __global__ void __launch_bounds__(kBfsDoMaxCta, 4) k_bfs_do(DoKernelArgs ka, uin
   __shared__ float s_in[4];    // n, out-degree sum, sum of squares, maximum of this level's frontier
   __shared__ float s_vis[2];   // vertices and out-edges of the frontiers so far (the same in every CTA)
   __shared__ int32_t s_pulls;
+  // read behind a level's barrier by one thread: the next frontier's size and
+  // statistics, this level's hub chunks, the stop word
+  __shared__ int32_t s_n, s_chunks, s_stop;
+  __shared__ unsigned long long s_raw[3];
   const FusedArgs &a = ka.a;
   const DoArgs &d = ka.d;
   float *wsel = reinterpret_cast<float *>(reinterpret_cast<char *>(smem) + do_lb_smem_aligned(lb_bytes));
@@ -620,16 +629,21 @@ __global__ void __launch_bounds__(kBfsDoMaxCta, 4) k_bfs_do(DoKernelArgs ka, uin
     s_pulls = 0;
     stage.n = 0;
   }
+  const auto fetch = [&](int32_t level) {  // words of the frontier that `level` found
+    s_n = *(volatile int32_t *)(a.cnt3 + level % 3);
+    s_chunks = *(volatile int32_t *)(a.hub3 + level % 3);
+    s_stop = *(volatile int32_t *)a.stop;
+    if (d.stats)
+      for (int i = 0; i < 3; ++i) s_raw[i] = *(volatile unsigned long long *)(d.lstat + 4 * (level % 3) + i);
+  };
+  if (threadIdx.x == 0) fetch(0);
   __syncthreads();
   int32_t level = 1;
   LoopClock clk;
   clk.start(a.loop_limit_ns);
   for (;; ++level) {
-    // the frontier statistics are loaded together with its size (one round trip)
-    unsigned long long r = 0ull;
-    if (d.stats && threadIdx.x < 3) r = *(volatile unsigned long long *)(d.lstat + 4 * ((level - 1) % 3) + threadIdx.x);
-    const int32_t n = *(volatile int32_t *)(a.cnt3 + (level - 1) % 3);
-    if (n == 0 || stopped(a.stop, level)) break;
+    const int32_t n = s_n;
+    if (n == 0 || stop_reached(s_stop, level)) break;
     const bool logged = d.feat_log && level - 1 <= d.max_log;
     // The level's direction, decided by warp 0 alone (statistics, features,
     // network) and handed to the CTA by one barrier.
@@ -638,7 +652,7 @@ __global__ void __launch_bounds__(kBfsDoMaxCta, 4) k_bfs_do(DoKernelArgs ka, uin
       bool pull = d.mode == DO_FORCE_PULL ||
                   (d.mode == DO_RULE && ((float)n <= d.threshold * (float)a.g.V) == (d.small_pull != 0));
       if (d.stats) {
-        if (l < 3) s_in[1 + l] = l == 1 ? (float)__longlong_as_double((long long)r) : (float)r;
+        if (l < 3) s_in[1 + l] = l == 1 ? (float)__longlong_as_double((long long)s_raw[l]) : (float)s_raw[l];
         if (l == 0) {
           s_in[0] = (float)n;
           s_stat.sum = s_stat.mx = 0u;
@@ -705,9 +719,9 @@ __global__ void __launch_bounds__(kBfsDoMaxCta, 4) k_bfs_do(DoKernelArgs ka, uin
         }
       }
       if (!chunks) clk.tick(a.stop, level, a.err);
-      ok = grid_barrier(a.bar, gridDim.x, a.err, a.timeout_ns);
+      ok = grid_barrier_then(a.bar, gridDim.x, a.err, a.timeout_ns, [&] { fetch(level); });
       if (!ok || pull || chunks) break;
-      chunks = *(volatile int32_t *)hub.cnt;
+      chunks = s_chunks;
       if (!chunks) break;
     }
     if (!ok) break;
