@@ -187,6 +187,15 @@ struct BcItems {
   const int32_t *cnt, *hcnt;  // items: light, long
   int32_t *wc, *hwc;          // hand-out counters
 };
+// Control words of the loop, read behind a barrier by one thread of the block
+// (grid_barrier_then): the end of the level list, hub chunks, item counts, stop.
+struct BcWords {
+  int32_t end, chunks, light, longs, stop;
+  __device__ __forceinline__ void items(const BcItems &w) {
+    light = *(const volatile int32_t *)w.cnt;
+    longs = *(const volatile int32_t *)w.hcnt;
+  }
+};
 // False when none are left; items are work[i] for i in [i0, i1).
 __device__ __forceinline__ bool bc_take(const BcState &st, const BcItems &w, int32_t n_light, int32_t n_long,
                                         int32_t nwarps, bool &longs, int32_t &i0, int32_t &i1) {
@@ -203,10 +212,12 @@ __device__ __forceinline__ bool bc_take(const BcState &st, const BcItems &w, int
     longs = false;
   }
   if (lane == 0) {
+    // a warp that finds the counter past the end takes nothing: in a level of a few
+    // items the GPU's other 4,000 warps would queue on the counter
     const int32_t left = n_light - *(volatile int32_t *)w.wc;
-    const int32_t per = left > 0 ? (left / 2 + nwarps - 1) / nwarps : 1;
+    const int32_t per = (left / 2 + nwarps - 1) / nwarps;
     B = per < 1 ? 1 : (per > 8 ? 8 : per);
-    b = atomicAdd(w.wc, B);
+    b = left > 0 ? atomicAdd(w.wc, B) : n_light;
   }
   b = __shfl_sync(0xffffffffu, b, 0);
   B = __shfl_sync(0xffffffffu, B, 0);
@@ -218,9 +229,9 @@ __device__ __forceinline__ bool bc_take(const BcState &st, const BcItems &w, int
 // f(v, chunk, first in-edge, end in-edge, whole list in one item) over a
 // phase's items, a warp each.
 template <class Fn>
-__device__ __forceinline__ void bc_each_item(const BcState &st, const BcItems &w, int32_t nwarps, const Fn &f) {
-  const int32_t n_light = min(*(const volatile int32_t *)w.cnt, st.wcap);
-  const int32_t n_long = min(*(const volatile int32_t *)w.hcnt, st.wcap);
+__device__ __forceinline__ void bc_each_item(const BcState &st, const BcItems &w, const BcWords &words, int32_t nwarps,
+                                             const Fn &f) {
+  const int32_t n_light = min(words.light, st.wcap), n_long = min(words.longs, st.wcap);
   bool longs = n_long > 0;
   for (int32_t i0, i1; bc_take(st, w, n_light, n_long, nwarps, longs, i0, i1);)
     for (int32_t i = i0; i < i1; ++i) {
@@ -249,7 +260,11 @@ __device__ __forceinline__ BcItems bc_backward_items(const BcState &st, int32_t 
 __global__ void __launch_bounds__(512, 2) k_bc_batch(DGraph g, BcState st) {
   extern __shared__ int4 smem[];
   __shared__ Stage stage;
-  if (threadIdx.x == 0) stage.n = 0;
+  __shared__ BcWords words;
+  if (threadIdx.x == 0) {
+    stage.n = 0;
+    words.stop = 0;
+  }
   __syncthreads();
   const int32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int32_t nthreads = gridDim.x * blockDim.x;
@@ -273,7 +288,7 @@ __global__ void __launch_bounds__(512, 2) k_bc_batch(DGraph g, BcState st) {
   for (;; ++d) {
     const int32_t e_d = e_next;
     if (e_d == b_d) break;  // Q_d is empty
-    if (stopped(st.stop, d)) {
+    if (stop_reached(words.stop, d)) {
       alive = false;
       break;
     }
@@ -292,7 +307,7 @@ __global__ void __launch_bounds__(512, 2) k_bc_batch(DGraph g, BcState st) {
     // sigma of Q_d from Q_{d-1} (items made by the previous publish)
     if (d > 0) {
       const uint64_t *pm = bc_fr(st, d - 1), *nm = bc_fr(st, d);
-      bc_each_item(st, bc_forward_items(st, d - 1), nwarps,
+      bc_each_item(st, bc_forward_items(st, d - 1), words, nwarps,
                    [&](int32_t v, int32_t, int32_t k0, int32_t k1, bool single) {
         const uint64_t own = __ldcg(nm + v);
         double a0, a1;
@@ -328,18 +343,21 @@ __global__ void __launch_bounds__(512, 2) k_bc_batch(DGraph g, BcState st) {
       out.stage = &stage;
       lb_twce_all(g, en, n, f, out, blockIdx.x, gridDim.x, *reinterpret_cast<TwceSmem *>(smem), hub);
       stage_flush(out);
-      alive = grid_barrier(st.bar, gridDim.x, st.err, st.timeout_ns);
-      const int32_t chunks = *(volatile int32_t *)hub.cnt;
-      if (alive && chunks > 0) {  // the hubs the level set aside, by all CTAs
-        lb_hubs(g, hub, chunks, f, out, blockIdx.x, gridDim.x);
+      const auto fetch = [&] {
+        words.end = *(volatile int32_t *)out.cnt;
+        words.chunks = *(volatile int32_t *)hub.cnt;
+      };
+      alive = grid_barrier_then(st.bar, gridDim.x, st.err, st.timeout_ns, fetch);
+      if (alive && words.chunks > 0) {  // the hubs the level set aside, by all CTAs
+        lb_hubs(g, hub, words.chunks, f, out, blockIdx.x, gridDim.x);
         stage_flush(out);
-        alive = grid_barrier(st.bar, gridDim.x, st.err, st.timeout_ns);
+        alive = grid_barrier_then(st.bar, gridDim.x, st.err, st.timeout_ns, fetch);
       }
     }
     if (!alive) break;
     // publish Q_{d+1}: masks, depths, and its sigma work items
     {
-      e_next = min(*(volatile int32_t *)(st.ctr + 0), st.levcap);
+      e_next = min(words.end, st.levcap);
       const int32_t m = e_next - e_d;
       const int32_t m_up = (m + 31) & ~31;
       uint64_t *nm = bc_fr(st, d + 1);
@@ -361,7 +379,10 @@ __global__ void __launch_bounds__(512, 2) k_bc_batch(DGraph g, BcState st) {
       }
     }
     clk.tick(st.stop, d, st.err);
-    if (!grid_barrier(st.bar, gridDim.x, st.err, st.timeout_ns)) {
+    if (!grid_barrier_then(st.bar, gridDim.x, st.err, st.timeout_ns, [&] {
+          words.items(bc_forward_items(st, d));
+          words.stop = *(volatile int32_t *)st.stop;
+        })) {
       alive = false;
       break;
     }
@@ -373,7 +394,7 @@ __global__ void __launch_bounds__(512, 2) k_bc_batch(DGraph g, BcState st) {
   // ------------------------------------------------------------ backward
   // (iterations numbered on from the forward loop's, for the loop clock)
   for (int32_t dd = L - 1, it = L + 1; alive && dd >= 0; --dd, ++it) {
-    if (stopped(st.stop, it)) break;
+    if (stop_reached(words.stop, it)) break;
     if (tid == 0) {
       st.ctr[3 + ((dd + 1) & 1)] = st.ctr[26 + ((dd + 1) & 1)] = 0;   // consumed by the gather of level dd + 1
       st.ctr[18 + ((dd + 1) & 1)] = st.ctr[30 + ((dd + 1) & 1)] = 0;  // that gather's hand-out
@@ -415,11 +436,12 @@ __global__ void __launch_bounds__(512, 2) k_bc_batch(DGraph g, BcState st) {
         bc_push_items(st, st.ctr + 3 + (dd & 1), st.ctr + 26 + (dd & 1), v, deg);
       }
     }
-    if (!grid_barrier(st.bar, gridDim.x, st.err, st.timeout_ns)) break;
+    if (!grid_barrier_then(st.bar, gridDim.x, st.err, st.timeout_ns, [&] { words.items(bc_backward_items(st, dd)); }))
+      break;
     // gather: dep'[v][s] = 1/sigma[v][s] + sum over deeper in-neighbours
     {
       const uint64_t *lmn = bc_lm(st, dd);
-      bc_each_item(st, bc_backward_items(st, dd), nwarps,
+      bc_each_item(st, bc_backward_items(st, dd), words, nwarps,
                    [&](int32_t v, int32_t c, int32_t k0, int32_t k1, bool single) {
         const uint64_t own = __ldcg(lmn + v);
         double a0, a1;
@@ -439,7 +461,9 @@ __global__ void __launch_bounds__(512, 2) k_bc_batch(DGraph g, BcState st) {
       });
     }
     clk.tick(st.stop, it, st.err);
-    if (!grid_barrier(st.bar, gridDim.x, st.err, st.timeout_ns)) break;
+    if (!grid_barrier_then(st.bar, gridDim.x, st.err, st.timeout_ns,
+                           [&] { words.stop = *(volatile int32_t *)st.stop; }))
+      break;
   }
 }
 
