@@ -408,7 +408,7 @@ __device__ __forceinline__ void mesh_relax_pass(const BqLoop &s, const BqArgs &a
           }
         } else if (to == 1) {
           if (pos < kMeshLow) {
-            atomicMax(stamps + v, lo_mark);
+            stamp_raise(a.b.stamp, v, lo_mark);
             m.lo[L][pos] = make_int4(v, p, db[j], de[j]);
           } else {
             m.full = 1;
@@ -422,7 +422,7 @@ __device__ __forceinline__ void mesh_relax_pass(const BqLoop &s, const BqArgs &a
           }
         } else if (to == 2) {
           if (pos < kMeshHigh) {
-            atomicMax(stamps + v, hi_mark);
+            stamp_raise(a.b.stamp, v, hi_mark);
             m.hi[pos] = v;
           } else if (stamp_claim(a.b.stamp, v, hi_tag) < hi_tag) {
             const int32_t gp = atomicAdd(sctl + BQ_HI + (s.gh & 1), 1);

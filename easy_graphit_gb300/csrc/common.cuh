@@ -214,6 +214,13 @@ __device__ __forceinline__ void pile_append(Stage *st, int32_t *pile, int32_t *c
 __device__ __forceinline__ uint32_t stamp_claim(int32_t *stamp, int32_t v, uint32_t tag) {
   return atomicMax(reinterpret_cast<uint32_t *>(stamp) + v, tag);
 }
+// The same without the answer, and without waiting for one: an atomicMax whose result
+// is not used was waited for in three of the four fused SSSP loops (mesh session on a
+// 200^2 grid, delta 32: 8.2 ms against 7.2).
+__device__ __forceinline__ void stamp_raise(int32_t *stamp, int32_t v, uint32_t tag) {
+  asm volatile("red.relaxed.gpu.global.max.u32 [%0], %1;" ::"l"(__cvta_generic_to_global(stamp + v)), "r"(tag)
+               : "memory");
+}
 
 // Far piles of the single-source delta-stepping queue (bucket_queue.cuh).  A
 // relaxation that lowers P[v] to p at or above the window's cutoff parks v on
