@@ -67,10 +67,13 @@ __device__ __forceinline__ void lb_vertex(const DGraph &g, const Enum &en, int32
   if (i >= n) return;
   const int32_t s = en.at(i);
   const int32_t b = __ldg(g.off + s), e = __ldg(g.off + s + 1);
-  if (e - b <= 4)
+  if (e - b <= 4) {
     do_range(g, f, out, s, b, e, 0, 1);
-  else
-    do_range<kSerialInFlight>(g, f, out, s, b, e, 0, 1);
+    return;
+  }
+  DOut o = out;
+  if (e - b > kStageCap / 2) o.stage = nullptr;  // a hub's thread would fill the stage, then try it for nothing
+  do_range<kSerialInFlight>(g, f, o, s, b, e, 0, 1);
 }
 
 // ---------------------------------------------------------------------- WM
