@@ -810,10 +810,14 @@ gg_status fused_bfs_do(gg_graph *g, const BfsDoPlan &p, int32_t n0, const VData 
 // Largest relax step the SSSP loop runs on one CTA: four frontier entries per
 // thread of the CTA (GG_BQ_SOLO_PER_THREAD overrides; 0 turns the one-CTA mode
 // off), and for the strategies that spread a list over threads at most 16 edges
-// per thread were every entry the graph's longest list -- a step of the whole GPU takes 9 us, and on a skewed graph CTA 0 alone
-// took 975 us for 1,844 vertices with hubs among them and 25 to 110 us for four to
-// forty (R-MAT of 250,000 vertices, TWCE: 1,860 us in all, 910 without).  Pile
-// steps take 32 entries per thread: one load and a compare each.
+// per thread were every entry the graph's longest list -- a step of the whole GPU
+// takes 9 us, and on a skewed graph CTA 0 alone took 975 us for 1,844 vertices with
+// hubs among them and 25 to 110 us for four to forty (R-MAT of 250,000 vertices,
+// TWCE: 1,860 us in all, 910 without) -- or as many entries as one CTA would take
+// anyway, a warp each (WM) or a thread's share of the edges (CM): the counts are in
+// shared memory then (a star of a million leaves, delta 32: WM 38.4 -> 18.4 ms, CM 4.5
+// -> 3.3; symmetrized R-MAT 20: WM 5.1 -> 4.4).  Pile steps take 32 entries per
+// thread: one load and a compare each.
 static int32_t bq_solo_per_thread() {
   static const long env = [] {
     const char *e = getenv("GG_BQ_SOLO_PER_THREAD");
@@ -845,7 +849,10 @@ static BqArgs bq_args(gg_graph *g, gg_frontier *f, const BqBuffers &b, int32_t *
   const int32_t per_thread = bq_solo_per_thread();
   a.solo_max = (per_thread >= 0 ? per_thread : 4) * cta;
   a.solo_pile_max = 8 * a.solo_max;
-  if (per_thread < 0 && g->max_degree > kMeshMaxDegree && lb != GG_LB_VERTEX_BASED) a.solo_max = std::min(a.solo_max, 16 * cta / g->max_degree);
+  if (per_thread < 0 && g->max_degree > kMeshMaxDegree && lb != GG_LB_VERTEX_BASED) {
+    const int32_t one_cta = lb == GG_LB_WM ? cta / 32 : (lb == GG_LB_CM ? cta : 0);
+    a.solo_max = std::max(one_cta, std::min(a.solo_max, 16 * cta / g->max_degree));
+  }
   a.width0 = 16;
   a.hub_list = static_cast<int32_t *>(g->hubs.p);
   a.hub_cap = hub_capacity(g);
