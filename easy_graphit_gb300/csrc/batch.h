@@ -86,7 +86,6 @@ gg_status bsssp_cta_buffers(gg_graph *g, int32_t k, Scratch *sc, CtaBuffers *b);
 gg_status bsssp_cta_run(gg_graph *g, cudaStream_t st, const CtaBuffers &b, int32_t *rows, int32_t k,
                         int32_t delta, bool timed);
 gg_status bsssp_use_cta(gg_graph *g, bool *use);
-gg_status graph_max_degree(gg_graph *g, int32_t *out);
 
 // Device buffers of one batched-SSSP pass; `owned` buffers are freed with it,
 // the others are the graph's reusable app slots.
@@ -112,7 +111,7 @@ struct MsBfsState {
   int32_t *q[3];              // queue of level L in q[L % 3]
   int32_t *cnt4;              // [4] queue count of level L in cnt4[L % 4]
   int32_t *hub_list, *hub3;   // hub chunks of a top-down level and their counts [L % 3]
-  int32_t hub_cap;
+  int32_t hub_cap, hub_slices;
   const int32_t *toff, *tsrc; // in-lists, for bottom-up levels
   int32_t V;
   int32_t bu_div;             // bottom-up when the frontier holds more than V / bu_div vertices (<= 0: never)

@@ -58,7 +58,7 @@ struct BcState {
   int32_t *err;
   uint64_t timeout_ns;
   int32_t *hub_list;             // hub chunks of a relax (counts: ctr[21..23], by level)
-  int32_t hub_cap;
+  int32_t hub_cap, hub_slices;
   int32_t *stats;                // [0] levels
   int32_t *stop;
   uint64_t loop_limit_ns;
@@ -333,7 +333,8 @@ __global__ void __launch_bounds__(512, 2) k_bc_batch(DGraph g, BcState st) {
       const int32_t n = e_d - b_d;
       const Enum en{st.lev + b_d, nullptr, n};
       const UMsBfs f{st.seen, bc_fr(st, d), st.acc, st.qstamp, d + 1};
-      const HubList hub{st.hub_list, st.ctr + 21 + d % 3, st.hub_cap, kHubWidths * (int32_t)blockDim.x};
+      const HubList hub{st.hub_list, st.ctr + 21 + d % 3, st.hub_cap, kHubWidths * (int32_t)blockDim.x,
+                        st.hub_slices};
       DOut out{};
       out.mode = OUT_SPARSE;
       out.q = st.lev;
@@ -600,6 +601,7 @@ static BcState bcb_state(gg_graph *g, const BcBuffers &b, int32_t k) {
   S.ctr = S.loff + kBcMaxLevels + 2;
   S.hub_list = static_cast<int32_t *>(g->hubs.p);
   S.hub_cap = hub_capacity(g);
+  S.hub_slices = slice_limit(g->max_degree);
   S.stats = S.ctr + 8;
   S.stop = S.ctr + 12;
   S.work = b.work;

@@ -292,7 +292,8 @@ __global__ void __launch_bounds__(512, 3) k_msbfs(DGraph g, MsBfsState st) {
     int32_t *qn = ms_q(st, L + 1);
     // top-down: acc[v] |= fr[u] & ~seen[v]; the first toucher queues v
     const UMsBfs f{st.seen, frc, st.acc, st.qstamp, L + 1};
-    const HubList hub{st.hub_list, st.hub3 + L % 3, st.hub_cap, kHubWidths * (int32_t)blockDim.x};
+    const HubList hub{st.hub_list, st.hub3 + L % 3, st.hub_cap, kHubWidths * (int32_t)blockDim.x,
+                      st.hub_slices};
     DOut out{};
     out.mode = OUT_SPARSE;
     out.q = qn;
@@ -460,6 +461,7 @@ MsBfsState msbfs_state(gg_graph *g, const MsBfsBuffers &b, int32_t k, int32_t *d
   S.hub3 = hdr + 16;     // 3
   S.hub_list = static_cast<int32_t *>(g->hubs.p);
   S.hub_cap = hub_capacity(g);
+  S.hub_slices = slice_limit(g->max_degree);
   S.toff = t.off;
   S.tsrc = t.dst;
   S.V = V;

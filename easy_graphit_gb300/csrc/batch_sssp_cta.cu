@@ -740,30 +740,6 @@ gg_status bsssp_cta_run(gg_graph *g, cudaStream_t st, const CtaBuffers &b, int32
   return GG_OK;
 }
 
-__global__ void k_max_degree(const int32_t *__restrict__ off, int32_t V, int32_t *out) {
-  int32_t m = 0;
-  for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
-    m = max(m, __ldg(off + v + 1) - __ldg(off + v));
-  m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
-}
-
-// Largest out-degree of the graph (computed once, then cached).
-gg_status graph_max_degree(gg_graph *g, int32_t *out) {
-  if (g->max_degree < 0) {
-    int32_t *d = g->d_misc + 60;
-    GG_CUDA(cudaMemsetAsync(d, 0, sizeof(int32_t), g->stream));
-    note_launch();
-    k_max_degree<<<g->sm_count * 4, 256, 0, g->stream>>>(g->csr.off, g->csr.V, d);
-    GG_CUDA(cudaGetLastError());
-    GG_CUDA(cudaMemcpyAsync(g->h_pinned + 60, d, sizeof(int32_t), cudaMemcpyDeviceToHost, g->stream));
-    GG_CUDA(cudaStreamSynchronize(g->stream));
-    g->max_degree = g->h_pinned[60];
-  }
-  *out = g->max_degree;
-  return GG_OK;
-}
-
 // The per-source-CTA mode applies when the tuning asks for it, or by default
 // on graphs without hubs (largest out-degree at most kMeshDegree): meshes and
 // road-like graphs, whose diameter makes the lane-per-source kernel barrier-bound.
@@ -774,9 +750,7 @@ gg_status bsssp_use_cta(gg_graph *g, bool *use) {
     *use = mode > 0;
     return GG_OK;
   }
-  int32_t md = 0;
-  GG_TRY(graph_max_degree(g, &md));
-  *use = md <= kMeshDegree;
+  *use = g->max_degree <= kMeshDegree;
   return GG_OK;
 }
 

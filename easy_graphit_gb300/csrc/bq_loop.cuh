@@ -64,7 +64,7 @@ struct BqArgs {
   int32_t fill_target;  // low-pile entries a refill aims for
   int32_t width0;       // first horizon width, in buckets
   int32_t *hub_list;    // hub chunks (HubList); their counts are control words
-  int32_t hub_cap, hub_min;
+  int32_t hub_cap, hub_min, hub_slices;
   int32_t mesh;         // largest out-degree <= 32: one-CTA sessions run in shared memory (bq_mesh_session)
 };
 
@@ -173,7 +173,7 @@ __device__ __forceinline__ void bq_step(BqLoop &s, const BqArgs &a, const BqStep
       return;
     }
     if (lead) ctl[BQ_HUB + (s.relax + 1) % 3] = 0;
-    const HubList hub{a.hub_list, ctl + BQ_HUB + s.relax % 3, a.hub_cap, a.hub_min};
+    const HubList hub{a.hub_list, ctl + BQ_HUB + s.relax % 3, a.hub_cap, a.hub_min, a.hub_slices};
     const int32_t n = (int64_t)st.work > a.qcap ? (int32_t)a.qcap : st.work;  // past qcap only after a flagged overflow
     run_lb<LB>(a.g, Enum{qin, nullptr, n}, n, f, front, smem, rank, nparts, hub);
     if (staged) {

@@ -79,7 +79,7 @@ struct gg_graph {
   const gg_selector *batch_selector[3] = {};  // learned per-level choices of the batched kernels
   gg::Scratch bq_cta;             // batched SSSP with a CTA per source
   gg::Scratch hubs;               // hub chunks of TWCE in the persistent loops (ensure_hubs)
-  int32_t max_degree = -1;        // largest out-degree (-1: not computed yet)
+  int32_t max_degree = 0;         // largest out-degree
 };
 
 struct gg_frontier {

@@ -68,13 +68,13 @@ struct FusedArgs {
   uint64_t loop_limit_ns;
   int32_t *hub_list;  // hub chunks (lb.cuh) of a level
   int32_t *hub3;      // their rotating counts [3]
-  int32_t hub_cap, hub_min;
+  int32_t hub_cap, hub_min, hub_slices;
 };
 
 // The hub list of level `level`; its count is cleared two levels ahead, with
 // the queue's.
 __device__ __forceinline__ HubList level_hubs(const FusedArgs &a, int64_t level) {
-  return HubList{a.hub_list, a.hub3 + level % 3, a.hub_cap, a.hub_min};
+  return HubList{a.hub_list, a.hub3 + level % 3, a.hub_cap, a.hub_min, a.hub_slices};
 }
 
 __device__ __forceinline__ DOut sparse_out(const FusedArgs &a, int32_t *q, int64_t it, Stage *stage) {
@@ -315,6 +315,7 @@ static FusedArgs make_args(gg_graph *g, gg_frontier *f, const VData &vd, int cta
   a.hub3 = g->d_misc + 49;
   a.hub_cap = hub_capacity(g);
   a.hub_min = kHubWidths * cta;
+  a.hub_slices = slice_limit(g->max_degree);
   return a;
 }
 
@@ -857,7 +858,8 @@ static BqArgs bq_args(gg_graph *g, gg_frontier *f, const BqBuffers &b, int32_t *
   a.hub_list = static_cast<int32_t *>(g->hubs.p);
   a.hub_cap = hub_capacity(g);
   a.hub_min = kHubWidths * cta;
-  a.mesh = g->max_degree >= 0 && g->max_degree <= kMeshMaxDegree && a.solo_max > 0;
+  a.hub_slices = slice_limit(g->max_degree);
+  a.mesh = g->max_degree <= kMeshMaxDegree && a.solo_max > 0;
   // Low-pile entries of a refill.  A mesh session reads them at every advance
   // (2048^2 grid, delta 8: 1123 ms with 2,048, 580 with 1,024, 398 with 512); the
   // other form pays more for a refill.
@@ -871,8 +873,6 @@ gg_status fused_sssp(gg_graph *g, const gg_schedule *s, int32_t n0, int32_t delt
   if (!fused_supported(s)) return GG_OK;
   const int cta = s->cta_size;
   GG_TRY(ensure_hubs(g));
-  int32_t max_degree = 0;
-  GG_TRY(graph_max_degree(g, &max_degree));  // kept with the graph
   const bool prepared = !iters;
   if (!prepared) GG_TRY(bq_start(pq->bq, n0, g->stream));
   BqArgs a = bq_args(g, pq->frontier, pq->bq, vd.dist, delta, cta, s->load_balancing);
@@ -934,9 +934,7 @@ __global__ void k_multi_seed(VData vd, int32_t sssp, const int32_t *__restrict__
 }
 
 gg_status fused_multi_setup(gg_graph *g) {
-  int32_t max_degree = 0;
-  GG_TRY(graph_max_degree(g, &max_degree));
-  if (max_degree <= kMeshMaxDegree)
+  if (g->max_degree <= kMeshMaxDegree)
     GG_CUDA(cudaFuncSetAttribute(k_sssp_bq<GG_LB_TWCE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)bq_smem(GG_LB_TWCE, 512, true)));
   return GG_OK;
@@ -959,7 +957,7 @@ gg_status fused_multi_enqueue(gg_graph *g, cudaStream_t st, bool sssp, const int
   const int cta = 512;
   FusedArgs a = make_args(g, f, vd, cta);
   a.delta = delta;
-  const bool mesh = sssp && g->max_degree >= 0 && g->max_degree <= kMeshMaxDegree;
+  const bool mesh = sssp && g->max_degree <= kMeshMaxDegree;
   const size_t smem = sssp ? bq_smem(GG_LB_TWCE, cta, mesh) : twce_smem_bytes(cta);
   const void *kernel = sssp ? (const void *)k_sssp_bq<GG_LB_TWCE> : (const void *)k_bfs_fused<GG_LB_TWCE>;
   int per_sm = 0;

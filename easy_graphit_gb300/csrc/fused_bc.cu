@@ -28,7 +28,7 @@ struct BcArgs {
   float *out;
   int32_t *cnt3, *hub3;         // queue and hub-chunk counts, rotating by level / edge pass
   int32_t *hub_list;
-  int32_t hub_cap, hub_min;
+  int32_t hub_cap, hub_min, hub_slices;
   uint32_t *bar;
   int32_t *err, *stats, *stop;
   uint64_t timeout_ns, loop_limit_ns;
@@ -97,7 +97,7 @@ __global__ void k_bc_setup(BcArgs a) {
 template <int LB, class F>
 __device__ __forceinline__ bool bc_pass(const BcArgs &a, const int32_t *q, int32_t n, const F &f, const DOut &out,
                                         int4 *smem, int32_t pass) {
-  const HubList hub{a.hub_list, a.hub3 + pass % 3, a.hub_cap, a.hub_min};
+  const HubList hub{a.hub_list, a.hub3 + pass % 3, a.hub_cap, a.hub_min, a.hub_slices};
   if (blockIdx.x == 0 && threadIdx.x == 0) a.hub3[(pass + 1) % 3] = 0;
   run_lb<LB>(a.g, Enum{q, nullptr, n}, n, f, out, smem, blockIdx.x, gridDim.x, hub);
   if (out.stage) stage_flush(out);
@@ -193,6 +193,7 @@ gg_status fused_bc(gg_graph *g, const gg_schedule *s, int32_t src, int32_t *dept
   a.hub_list = static_cast<int32_t *>(g->hubs.p);
   a.hub_cap = hub_capacity(g);
   a.hub_min = kHubWidths * cta;
+  a.hub_slices = slice_limit(g->max_degree);
   a.bar = g->d_bar;
   a.err = g->d_err;
   a.stats = g->d_misc + 44;

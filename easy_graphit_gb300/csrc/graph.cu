@@ -518,6 +518,14 @@ extern "C" {
 
 // Everything gg_graph_create sets up; on failure the caller releases what was
 // made (gg_graph_destroy takes a partly built graph).
+__global__ void k_max_degree(const int32_t *__restrict__ off, int32_t V, int32_t *out) {
+  int32_t m = 0;
+  for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
+    m = max(m, __ldg(off + v + 1) - __ldg(off + v));
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
+}
+
 static gg_status graph_init(gg_graph *g, const int32_t *offsets, const int32_t *dst, const int32_t *weights,
                             int32_t V, int64_t E, uint32_t flags) {
   GG_CUDA(cudaGetDevice(&g->device));
@@ -557,7 +565,12 @@ static gg_status graph_init(gg_graph *g, const int32_t *offsets, const int32_t *
   GG_CUDA(cudaEventCreate(&g->ev1));
   GG_CUDA(cudaEventCreate(&g->ev2));
   GG_CUDA(cudaEventCreate(&g->ev3));
+  note_launch();
+  k_max_degree<<<std::max(1, std::min(ceil_div(V, 256), g->sm_count * 4)), 256, 0, st>>>(s.off, V, g->d_misc + 60);
+  GG_CUDA(cudaGetLastError());
+  GG_CUDA(cudaMemcpyAsync(g->h_pinned + 60, g->d_misc + 60, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   GG_CUDA(cudaStreamSynchronize(st));  // the COO source column is built on first use (ensure_coo)
+  g->max_degree = g->h_pinned[60];
   return GG_OK;
 }
 

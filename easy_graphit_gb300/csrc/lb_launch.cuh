@@ -157,7 +157,8 @@ void launch_twce(const EdgeLaunch &L, const F &f, const HubList &hub) {
   int grid = res;
   if (L.n_host >= 0) {
     const int64_t nv = ceil_div(L.n_host, L.cta / kStage1);
-    if (nv < (int64_t)kTwceWaves * res) grid = (int)(nv * std::max<int64_t>(1, kTwceWaves * (int64_t)res / nv));
+    if (nv < (int64_t)kTwceWaves * res)
+      grid = (int)(nv * std::max<int64_t>(1, std::min<int64_t>(kTwceWaves * (int64_t)res / nv, hub.slices)));
   }
   note_launch();
   k<<<grid, L.cta, sm, L.graph->stream>>>(L.g, L.en, f, L.out, hub);
@@ -171,6 +172,8 @@ gg_status launch_lb(const EdgeLaunch &L, const F &f) {
   const int sms = G->sm_count;
   const int64_t n = L.n_host;
   if (n == 0 && L.lb != GG_LB_EDGE_ONLY) return GG_OK;
+  HubList hub;
+  if (!L.pull || G->symmetric) hub.slices = slice_limit(G->max_degree);  // in-lists of a directed graph are not bounded
   switch (L.lb) {
     case GG_LB_EDGE_ONLY: {
       if (L.g.nbuckets > 0) {
@@ -194,7 +197,7 @@ gg_status launch_lb(const EdgeLaunch &L, const F &f) {
       break;
     }
     case GG_LB_TWCE: {
-      launch_twce(L, f, HubList{});
+      launch_twce(L, f, hub);
       break;
     }
     case GG_LB_ETWC: {
@@ -204,7 +207,6 @@ gg_status launch_lb(const EdgeLaunch &L, const F &f) {
       const int64_t maxc = (int64_t)L.g.E / chunk + (n < 0 ? L.g.V : n) + 1;
       GG_TRY(etwc_scratch(G, maxc, &chunks, &cnt));
       GG_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t), st));
-      HubList hub;
       hub.list = chunks;
       hub.cnt = cnt;
       hub.cap = (int32_t)maxc;
