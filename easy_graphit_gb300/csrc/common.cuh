@@ -128,6 +128,7 @@ struct DOut {
   int32_t epoch;
   int32_t *err;
   Stage *stage;  // shared memory, or null: append directly
+  bool few;      // no list is longer than kStage1 edges
 
   __device__ __forceinline__ void sparse(int32_t v) const {
     if (stage && stage->add(v)) return;
