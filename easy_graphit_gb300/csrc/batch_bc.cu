@@ -259,10 +259,11 @@ __device__ __forceinline__ BcItems bc_backward_items(const BcState &st, int32_t 
 
 __global__ void __launch_bounds__(512, 2) k_bc_batch(DGraph g, BcState st) {
   extern __shared__ int4 smem[];
-  __shared__ Stage stage;
+  __shared__ StageMem stage_mem;
+  Stage &stage = stage_mem.s;
   __shared__ BcWords words;
   if (threadIdx.x == 0) {
-    stage.n = 0;
+    stage.init(kStageCap);
     words.stop = 0;
   }
   __syncthreads();

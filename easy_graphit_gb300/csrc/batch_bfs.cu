@@ -236,8 +236,9 @@ __global__ void __launch_bounds__(512, 3) k_msbfs(DGraph g, MsBfsState st) {
   __shared__ unsigned long long s_act;
   __shared__ unsigned long long s_stat[3];
   __shared__ MsLong long_;
-  __shared__ Stage stage;
-  if (threadIdx.x == 0) stage.n = 0;  // the first level's barrier comes before any append
+  __shared__ StageMem stage_mem;
+  Stage &stage = stage_mem.s;
+  if (threadIdx.x == 0) stage.init(kStageCap);  // the first level's barrier comes before any append
   const int32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int32_t nthreads = gridDim.x * blockDim.x;
   const int32_t lane = threadIdx.x & 31;

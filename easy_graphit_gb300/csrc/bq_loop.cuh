@@ -65,6 +65,7 @@ struct BqArgs {
   int32_t width0;       // first horizon width, in buckets
   int32_t *hub_list;    // hub chunks (HubList); their counts are control words
   int32_t hub_cap, hub_min, hub_slices;
+  int32_t stage_cap, stage_at;  // the three stages: entries each, where they start in shared memory
   int32_t mesh;         // largest out-degree <= 32: one-CTA sessions run in shared memory (bq_mesh_session)
 };
 
@@ -130,7 +131,7 @@ __device__ __forceinline__ BqStep bq_decide(const BqLoop &s, const int32_t *ctl,
 // copy in a one-CTA session.  `stages`: three in shared memory, empty.
 template <int LB>
 __device__ __forceinline__ void bq_step(BqLoop &s, const BqArgs &a, const BqStep &st, int32_t *ctl,
-                                        int32_t rank, int32_t nparts, int4 *smem, int32_t *red, Stage *stages) {
+                                        int32_t rank, int32_t nparts, int4 *smem, int32_t *red, Stage *const *stages) {
   const bool lead = rank == 0 && threadIdx.x == 0;
   if (lead) {
     ctl[BQ_NEAR + (s.it + 1) % 3] = 0;
@@ -147,8 +148,8 @@ __device__ __forceinline__ void bq_step(BqLoop &s, const BqArgs &a, const BqStep
   // appends are staged where many CTAs share the counts; one CTA has them in
   // shared memory anyway
   const bool staged = nparts > 1;
-  if (staged) front.stage = &stages[0];
-  Stage *st_lo = staged ? &stages[1] : nullptr, *st_hi = staged ? &stages[2] : nullptr;
+  if (staged) front.stage = stages[0];
+  Stage *st_lo = staged ? stages[1] : nullptr, *st_hi = staged ? stages[2] : nullptr;
   const int32_t lo_next = (s.g + 1) & 1;
   if (st.kind == BQ_RELAX || st.kind == BQ_HUBS) {
     const bool hubs = st.kind == BQ_HUBS;

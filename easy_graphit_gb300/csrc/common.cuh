@@ -92,21 +92,42 @@ __device__ __forceinline__ bool cas(int32_t *p, int32_t expect, int32_t v) {
 // that one word, which the L2 takes one after another (the widest level of a BFS
 // on the directed R-MAT 22, 1.1 M vertices found, with a stage of 1,024 entries,
 // half of them appended directly: 101 us pulled and 772 pushed; with 2,048 70 and
-// 448).  Appends past kStageCap go to the queue directly; the count is read first, or
+// 448).  Appends past its end go to the queue directly; the count is read first, or
 // whoever walks a hub alone would pay for two atomics an append (BFS on a star of a
 // million leaves, a thread per vertex 1,287 -> 1,170 ms, a warp per vertex 48.7 -> 44.9).
 constexpr int32_t kStageCap = 2048;
-struct Stage {
-  int32_t n, base;
-  int32_t buf[kStageCap];
+struct alignas(16) Stage {  // `cap` entries follow it in shared memory
+  int32_t n, cap, base, pad_;
+  __device__ __forceinline__ int32_t *buf() { return reinterpret_cast<int32_t *>(this + 1); }
+  __device__ __forceinline__ void init(int32_t entries) {
+    n = 0;
+    cap = entries;
+  }
   // Stages v; false when the stage is full.
   __device__ __forceinline__ bool add(int32_t v) {
-    if (*(volatile int32_t *)&n >= kStageCap) return false;
+    if (*(volatile int32_t *)&n >= cap) return false;
     const int32_t at = agg_inc(&n);
-    if (at >= kStageCap) return false;
-    buf[at] = v;
+    if (at >= cap) return false;
+    buf()[at] = v;
     return true;
   }
+};
+// Entries of each of a kernel's several stages: four a thread, at least 512.  With
+// 2,048 whatever the CTA, the many small CTAs of an SM leave little of it to the L1
+// (SSSP, a thread per vertex, 0.5 M vertices of degree 40: CTAs of 128 3.9 -> 1.8 ms,
+// of 64 2.8 -> 1.9).
+__host__ __device__ constexpr int32_t stage_cap(int32_t cta) {
+  return cta <= 128 ? 512 : (cta < 512 ? 4 * cta : kStageCap);
+}
+// The i-th of them in dynamic shared memory behind `used` bytes, and the bytes of all.
+__device__ __forceinline__ Stage *stage_at(void *smem, int32_t used, int32_t cap, int i) {
+  return reinterpret_cast<Stage *>(static_cast<char *>(smem) + (used + 15) / 16 * 16 + i * (16 + 4 * cap));
+}
+inline size_t with_stages(size_t used, int32_t cap, int n) { return (used + 15) / 16 * 16 + n * (16 + 4 * (size_t)cap); }
+
+struct StageMem {  // one of kStageCap entries in static shared memory
+  Stage s;
+  int32_t buf[kStageCap];
 };
 
 // Output frontier writer: the enqueue_* family of gpu_intrinsics.h:95-110.
@@ -172,14 +193,14 @@ struct DOut {
 // it.  Appends after it need a barrier first (every caller ends its step at one).
 __device__ __forceinline__ void stage_flush(Stage *st, int32_t *q, int32_t *cnt, int64_t cap, int32_t *err) {
   __syncthreads();
-  const int32_t n = min(st->n, kStageCap);
+  const int32_t n = min(st->n, st->cap);
   if (n == 0) return;
   if (threadIdx.x == 0) st->base = atomicAdd(cnt, n);
   __syncthreads();
   const int32_t base = st->base;
   for (int32_t i = threadIdx.x; i < n; i += blockDim.x) {
     if (base + i < cap)
-      q[base + i] = st->buf[i];
+      q[base + i] = st->buf()[i];
     else
       atomicOr(err, DEV_ERR_OVERFLOW);
   }
@@ -191,7 +212,7 @@ __device__ __forceinline__ void stage_flush(const DOut &out) {
 // The same in the middle of a step, when fewer than `room` entries are left.  The
 // whole CTA calls it behind a barrier, with another one before its next append.
 __device__ __forceinline__ void stage_make_room(const DOut &out, int32_t room) {
-  if (out.stage && out.stage->n > kStageCap - room) {
+  if (out.stage && out.stage->n > out.stage->cap - room) {
     stage_flush(out);
     __syncthreads();
   }
@@ -252,15 +273,15 @@ struct DFar {
     else
       pile_append(hi_stage, hi, hi_cnt, cap, v, err);
   }
-  // Sends what the CTA staged (all of it, or when less than `room` is left); the
-  // whole CTA calls it, as stage_flush and stage_make_room.
+  // Sends what the CTA staged (all of it, or when less than half is left); the whole
+  // CTA calls it, as stage_flush and stage_make_room.
   __device__ __forceinline__ void flush() const {
     if (!lo_stage) return;
     stage_flush(lo_stage, lo, lo_cnt, cap, err);
     stage_flush(hi_stage, hi, hi_cnt, cap, err);
   }
-  __device__ __forceinline__ void make_room(int32_t room) const {
-    if (!lo_stage || (lo_stage->n <= kStageCap - room && hi_stage->n <= kStageCap - room)) return;
+  __device__ __forceinline__ void make_room() const {  // at half a stage
+    if (!lo_stage || (lo_stage->n <= lo_stage->cap / 2 && hi_stage->n <= hi_stage->cap / 2)) return;
     flush();
     __syncthreads();
   }

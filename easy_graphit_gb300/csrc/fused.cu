@@ -91,9 +91,10 @@ __device__ __forceinline__ DOut sparse_out(const FusedArgs &a, int32_t *q, int64
 template <int LB>
 __global__ void __launch_bounds__(1024) k_bfs_fused(FusedArgs a) {
   extern __shared__ int4 smem[];
-  __shared__ Stage stage;
+  __shared__ StageMem stage_mem;
+  Stage &stage = stage_mem.s;
   __shared__ int32_t s_n, s_chunks, s_stop;  // read behind a level's barrier by one thread
-  if (threadIdx.x == 0) stage.n = 0;
+  if (threadIdx.x == 0) stage.init(kStageCap);
   __syncthreads();
   int32_t *qs[2] = {a.q0, a.q1};
   int in = 0;
@@ -199,8 +200,10 @@ __global__ void __launch_bounds__(1024) k_sssp_bq(BqArgs a) {
   extern __shared__ int4 smem[];
   __shared__ int32_t red[33];
   __shared__ int32_t sctl[BQ_STOP];  // counts and minima of a one-CTA session
-  __shared__ Stage stages[3];        // appends of a step: frontier, low pile, high pile
-  if (threadIdx.x < 3) stages[threadIdx.x].n = 0;
+  // appends of a step: frontier, low pile, high pile
+  Stage *const stages[3] = {stage_at(smem, a.stage_at, a.stage_cap, 0), stage_at(smem, a.stage_at, a.stage_cap, 1),
+                            stage_at(smem, a.stage_at, a.stage_cap, 2)};
+  if (threadIdx.x < 3) stage_at(smem, a.stage_at, a.stage_cap, threadIdx.x)->init(a.stage_cap);
   __syncthreads();
   BqLoop s{1, 0, 0, 0, 0, bq_clamp((int64_t)a.width0 * a.delta), a.width0, 0, 0, 0, 0};
   int32_t *stop = a.b.ctl + BQ_STOP;
@@ -611,7 +614,8 @@ template <int LB>
 __global__ void __launch_bounds__(kBfsDoMaxCta, 4) k_bfs_do(DoKernelArgs ka, uint32_t lb_bytes) {
   extern __shared__ int4 smem[];
   __shared__ DoStat s_stat;
-  __shared__ Stage stage;
+  __shared__ StageMem stage_mem;
+  Stage &stage = stage_mem.s;
   __shared__ float s_x[16 + 64];
   __shared__ int32_t s_pull;
   __shared__ float s_in[4];    // n, out-degree sum, sum of squares, maximum of this level's frontier
@@ -628,7 +632,7 @@ __global__ void __launch_bounds__(kBfsDoMaxCta, 4) k_bfs_do(DoKernelArgs ka, uin
   if (threadIdx.x == 0) {
     s_vis[0] = s_vis[1] = 0.f;
     s_pulls = 0;
-    stage.n = 0;
+    stage.init(kStageCap);
   }
   const auto fetch = [&](int32_t level) {  // words of the frontier that `level` found
     s_n = *(volatile int32_t *)(a.cnt3 + level % 3);
@@ -864,6 +868,8 @@ static BqArgs bq_args(gg_graph *g, gg_frontier *f, const BqBuffers &b, int32_t *
   // (2048^2 grid, delta 8: 1123 ms with 2,048, 580 with 1,024, 398 with 512); the
   // other form pays more for a refill.
   a.fill_target = a.mesh ? 512 : 1024;
+  a.stage_cap = a.mesh ? kStageCap : stage_cap(cta);  // a mesh session's memory leaves one CTA an SM anyway
+  a.stage_at = (int32_t)bq_smem(lb, cta, a.mesh);
   return a;
 }
 
@@ -876,7 +882,7 @@ gg_status fused_sssp(gg_graph *g, const gg_schedule *s, int32_t n0, int32_t delt
   const bool prepared = !iters;
   if (!prepared) GG_TRY(bq_start(pq->bq, n0, g->stream));
   BqArgs a = bq_args(g, pq->frontier, pq->bq, vd.dist, delta, cta, s->load_balancing);
-  const size_t sm = bq_smem(s->load_balancing, cta, a.mesh);
+  const size_t sm = with_stages(a.stage_at, a.stage_cap, 3);
   switch (s->load_balancing) {
     case GG_LB_VERTEX_BASED: GG_TRY(coop_launch(g, prepared, k_sssp_bq<GG_LB_VERTEX_BASED>, cta, sm, a)); break;
     case GG_LB_WM: GG_TRY(coop_launch(g, prepared, k_sssp_bq<GG_LB_WM>, cta, sm, a)); break;
@@ -936,7 +942,7 @@ __global__ void k_multi_seed(VData vd, int32_t sssp, const int32_t *__restrict__
 gg_status fused_multi_setup(gg_graph *g) {
   if (g->max_degree <= kMeshMaxDegree)
     GG_CUDA(cudaFuncSetAttribute(k_sssp_bq<GG_LB_TWCE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)bq_smem(GG_LB_TWCE, 512, true)));
+                                 (int)with_stages(bq_smem(GG_LB_TWCE, 512, true), kStageCap, 3)));
   return GG_OK;
 }
 
@@ -958,7 +964,8 @@ gg_status fused_multi_enqueue(gg_graph *g, cudaStream_t st, bool sssp, const int
   FusedArgs a = make_args(g, f, vd, cta);
   a.delta = delta;
   const bool mesh = sssp && g->max_degree <= kMeshMaxDegree;
-  const size_t smem = sssp ? bq_smem(GG_LB_TWCE, cta, mesh) : twce_smem_bytes(cta);
+  const size_t smem = sssp ? with_stages(bq_smem(GG_LB_TWCE, cta, mesh), mesh ? kStageCap : stage_cap(cta), 3)
+                           : twce_smem_bytes(cta);
   const void *kernel = sssp ? (const void *)k_sssp_bq<GG_LB_TWCE> : (const void *)k_bfs_fused<GG_LB_TWCE>;
   int per_sm = 0;
   GG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, cta, smem));

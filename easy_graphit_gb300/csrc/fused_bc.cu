@@ -112,8 +112,9 @@ __device__ __forceinline__ bool bc_pass(const BcArgs &a, const int32_t *q, int32
 template <int LB>
 __global__ void __launch_bounds__(1024) k_bc_fused(BcArgs a) {
   extern __shared__ int4 smem[];
-  __shared__ Stage stage;
-  if (threadIdx.x == 0) stage.n = 0;
+  __shared__ StageMem stage_mem;
+  Stage &stage = stage_mem.s;
+  if (threadIdx.x == 0) stage.init(kStageCap);
   __syncthreads();
   const int32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
   LoopClock clk;

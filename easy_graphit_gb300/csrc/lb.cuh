@@ -72,8 +72,12 @@ __device__ __forceinline__ void lb_vertex(const DGraph &g, const Enum &en, int32
     return;
   }
   DOut o = out;
-  if (e - b > kStageCap / 2) o.stage = nullptr;  // a hub's thread would fill the stage, then try it for nothing
-  do_range<kSerialInFlight>(g, f, o, s, b, e, 0, 1);
+  F h = f;
+  if (e - b > kStageCap / 2) {  // a hub's thread would fill the stages, then try them for nothing
+    o.stage = nullptr;
+    if constexpr (lb_batch<F>::value) h.stage_parks(nullptr, nullptr);
+  }
+  do_range<kSerialInFlight>(g, h, o, s, b, e, 0, 1);
 }
 
 // ---------------------------------------------------------------------- WM
@@ -229,8 +233,8 @@ __device__ __forceinline__ void lb_twce(const DGraph &g, const Enum &en, int32_t
 // functor that parks, of its piles.
 template <class F>
 __device__ __forceinline__ void lb_make_room(const F &f, const DOut &out) {
-  stage_make_room(out, kStageCap / 2);
-  if constexpr (lb_batch<F>::value) f.make_room(kStageCap / 2);
+  if (out.stage) stage_make_room(out, out.stage->cap / 2);
+  if constexpr (lb_batch<F>::value) f.make_room();
 }
 
 // TWCE over n vertices by CTA `rank` of `nparts`: whole

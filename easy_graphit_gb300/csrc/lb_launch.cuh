@@ -25,14 +25,14 @@ constexpr uint32_t kStagedGrid = 64;
 template <class F>
 struct KernelStages {
   static constexpr int kStages = !F::kPushes ? 0 : (lb_batch<F>::value ? 3 : 1);
-  Stage st[kStages > 0 ? kStages : 1];
+  StageMem st[kStages > 0 ? kStages : 1];
   __device__ __forceinline__ void begin(F &f, DOut &out) {
     if constexpr (kStages > 0) {
-      if (threadIdx.x < kStages) st[threadIdx.x].n = 0;
+      if (threadIdx.x < kStages) st[threadIdx.x].s.init(kStageCap);
       __syncthreads();
       if ((out.mode == OUT_SPARSE || out.mode == OUT_SPARSE_DEDUP) && !(out.few && gridDim.x <= kStagedGrid))
-        out.stage = &st[0];
-      if constexpr (kStages == 3) f.stage_parks(&st[1], &st[2]);
+        out.stage = &st[0].s;
+      if constexpr (kStages == 3) f.stage_parks(&st[1].s, &st[2].s);
     }
   }
   __device__ __forceinline__ void end(const F &f, const DOut &out) {

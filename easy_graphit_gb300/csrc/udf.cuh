@@ -219,8 +219,8 @@ struct EdgeF {
     if (PULL) return u.apply(d, s, w) ? s : -1;
     return u.apply(s, d, w) ? d : -1;
   }
-  __device__ __forceinline__ void make_room(int32_t room) const {
-    if constexpr (kBatch) u.far.make_room(room);
+  __device__ __forceinline__ void make_room() const {
+    if constexpr (kBatch) u.far.make_room();
   }
   __device__ __forceinline__ void flush() const {
     if constexpr (kBatch) u.far.flush();
