@@ -471,8 +471,8 @@ __device__ __forceinline__ void bq_mesh_session(BqLoop &s, const BqArgs &a, int3
     // end of this one, behind its barriers.  Tested in relaxes alone, on the same
     // count, it never came up where relaxes and advances take turns (a line of unit
     // weights at delta 1: every 16th round an advance), and only the horizon, seconds
-    // away, ended the session.
-    if (threadIdx.x == 0 && (rounds & 15) == 0)
+    // away, ended the session.  64 rounds are 0.1 to 0.5 ms.
+    if (threadIdx.x == 0 && (rounds & 63) == 0)
       m.quit = globaltimer_ns() - t0 > kSoloSliceNs || (*(volatile int32_t *)a.err & DEV_ERR_OVERFLOW) != 0;
     const int32_t U = bq_clamp((int64_t)s.cur + a.delta);
     if (n > 0) {
