@@ -531,12 +531,58 @@ struct UBfsNote {
 // in-edges, and tests its vertex's first kPullFirst in-neighbours, all in flight
 // together -- where a pull level pays, the frontier is large and most vertices
 // end there.  The lists still open are finished by 8-lane groups, four vertices
-// at a time.  An 8-lane group per vertex from the start needed a round trip per
+// at a time; those longer than kPullLong are set aside for the whole CTA, as in
+// ms_bottom_up (batch_bfs.cu): walked by a group, the hubs that a level does not reach
+// held it up alone (every level pulled, symmetrized R-MAT 20 1.82 -> 0.36 ms, directed
+// R-MAT 22 2.21 -> 0.74; from 128 edges 0.37 and 0.72).  16 or 32 in flight a group
+// gives 0.30 and 0.27 there, but its registers cost every other level 3 to 8 %.  An
+// 8-lane group per vertex from the start needed a round trip per
 // 4 vertices of a warp just to skip the visited ones (directed R-MAT 22, the
 // level that finds 1.1 M vertices: 650 us, 470 with staged appends, now 63).
 constexpr int kPullFirst = 4;
+constexpr int32_t kPullLong = 512;
+constexpr int32_t kPullLongMax = 256;  // set aside per CTA; more are walked by groups
+struct PullLong {
+  int32_t n, first;  // vertices set aside; first edge found of the one being walked
+  int32_t v[kPullLongMax];
+};
+// The lists do_pull_level set aside, one after another by the whole CTA, in list
+// order up to the first hit; vertices without one become -1 in lg.v.  Not inlined: the
+// loop of a pull level has its 32 registers a thread to itself.
+__device__ __noinline__ void do_pull_long(const int32_t *__restrict__ toff, const int32_t *__restrict__ tdst,
+                                          int32_t *parent, int32_t *depth, int32_t level, PullLong &lg) {
+  const int32_t nl = min(lg.n, kPullLongMax), T = blockDim.x;
+  for (int32_t i = 0; i < nl; ++i) {
+    const int32_t v = lg.v[i], ke = __ldg(toff + v + 1);
+    int32_t first = INT_MAX;
+    for (int64_t k0 = __ldg(toff + v) + kPullFirst; k0 < ke; k0 += 4 * T) {
+      int32_t u[4], mine = INT_MAX;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) u[j] = k0 + j * T + threadIdx.x < ke ? __ldg(tdst + k0 + j * T + threadIdx.x) : -1;
+#pragma unroll
+      for (int j = 3; j >= 0; --j)
+        if (u[j] >= 0 && __ldcg(depth + u[j]) == level - 1) mine = (int32_t)k0 + j * T + (int32_t)threadIdx.x;
+      mine = __reduce_min_sync(0xffffffffu, mine);
+      if ((threadIdx.x & 31) == 0 && mine != INT_MAX) atomicMin(&lg.first, mine);
+      __syncthreads();
+      first = lg.first;
+      __syncthreads();  // read by all before the next round's finds or the reset
+      if (first != INT_MAX) break;
+    }
+    if (threadIdx.x == 0) {
+      lg.first = INT_MAX;
+      if (first != INT_MAX) {
+        parent[v] = __ldg(tdst + first);
+        depth[v] = level;
+      } else {
+        lg.v[i] = -1;
+      }
+    }
+    __syncthreads();
+  }
+}
 __device__ __forceinline__ void do_pull_level(const FusedArgs &a, const DoArgs &d, int32_t level, const DOut &out,
-                                              DoAcc *acc) {
+                                              DoAcc *acc, PullLong &lg) {
   const int32_t lane = threadIdx.x & 31, sub = lane & 7, gi = lane >> 3;
   const uint32_t gmask = 0xFFu << (gi * 8);
   const int32_t prev = level - 1, V = a.g.V;
@@ -565,7 +611,16 @@ __device__ __forceinline__ void do_pull_level(const FusedArgs &a, const DoArgs &
 #pragma unroll
     for (int j = kPullFirst - 1; j >= 0; --j)
       if (du[j] == prev) hit = u[j];
-    uint32_t open = __ballot_sync(0xffffffffu, hit < 0 && ke - kb > kPullFirst);
+    bool more = hit < 0 && ke - kb > kPullFirst;
+    if (more && ke - kb > kPullLong) {
+      const int32_t at = agg_inc(&lg.n);
+      if (at < kPullLongMax) {
+        lg.v[at] = v;
+        more = false;
+      }
+    }
+    __syncwarp();
+    uint32_t open = __ballot_sync(0xffffffffu, more);
     while (open) {
       int32_t l[4];  // the next four open vertices, a group each (-1: none)
 #pragma unroll
@@ -625,6 +680,7 @@ __global__ void __launch_bounds__(kBfsDoMaxCta, 4) k_bfs_do(DoKernelArgs ka, uin
   // statistics, this level's hub chunks, the stop word
   __shared__ int32_t s_n, s_chunks, s_stop;
   __shared__ unsigned long long s_raw[3];
+  __shared__ PullLong s_long;
   const FusedArgs &a = ka.a;
   const DoArgs &d = ka.d;
   float *wsel = reinterpret_cast<float *>(reinterpret_cast<char *>(smem) + do_lb_smem_aligned(lb_bytes));
@@ -672,6 +728,8 @@ __global__ void __launch_bounds__(kBfsDoMaxCta, 4) k_bfs_do(DoKernelArgs ka, uin
       }
       if (l == 0) {
         s_pull = pull;
+        s_long.n = 0;
+        s_long.first = INT_MAX;
         if (blockIdx.x == 0) {
           a.cnt3[(level + 1) % 3] = 0;
           a.hub3[(level + 1) % 3] = 0;
@@ -705,7 +763,15 @@ __global__ void __launch_bounds__(kBfsDoMaxCta, 4) k_bfs_do(DoKernelArgs ka, uin
           run_lb<LB>(a.g, en, n, f, out, smem, blockIdx.x, gridDim.x, hub);
       } else {
         if (threadIdx.x == 0) ++s_pulls;
-        do_pull_level(a, d, level, out, stat);
+        do_pull_level(a, d, level, out, stat, s_long);
+        __syncthreads();
+        const int32_t nl = min(s_long.n, kPullLongMax);
+        if (nl > 0) do_pull_long(d.t.off, d.t.dst, a.vd.parent, a.vd.depth, level, s_long);
+        for (int32_t i = threadIdx.x; i < nl; i += blockDim.x)
+          if (const int32_t v = s_long.v[i]; v >= 0) {
+            out.sparse(v);
+            acc.note((uint32_t)(__ldg(a.g.off + v + 1) - __ldg(a.g.off + v)));
+          }
       }
       if (d.stats) do_fold(&s_stat, acc);
       stage_flush(out);  // its first barrier also ends the CTA's statistics
