@@ -46,6 +46,7 @@ struct BcState {
   int64_t *work;                 // (v << 32 | chunk)
   int32_t wcap;
   int32_t chunk;                 // in-edges per work item (the graph's batch tuning)
+  int32_t light;                 // longest list that is one light work item: kBcLight or the chunk
   int32_t *ctr;                  // [0] level-list end, [1..2] forward items, [3..4] backward items,
                                  // [16..19] hand-out counters, [20] end of Q_0, [21..23] hub chunks;
                                  // [24..27] long items and [28..31] their hand-out, as [1..4], [16..19]
@@ -65,13 +66,13 @@ struct BcState {
 };
 
 // Appends the work items of this lane's vertex (degree deg, -1 for a lane
-// without one); the whole warp calls it together.  Lists up to kBcLight edges
+// without one); the whole warp calls it together.  Lists up to st.light edges
 // are one item at the front of the work array (count wcnt), longer ones items of
 // st.chunk edges from its back (count hcnt): the two are handed out differently.
 __device__ __forceinline__ void bc_push_items(const BcState &st, int32_t *wcnt, int32_t *hcnt, int32_t v,
                                               int32_t deg) {
   const int32_t lane = threadIdx.x & 31;
-  const bool light = deg >= 0 && deg <= kBcLight;
+  const bool light = deg >= 0 && deg <= st.light;
   const uint32_t lights = __ballot_sync(0xffffffffu, light);
   if (lights) {
     int32_t base = 0;
@@ -85,7 +86,7 @@ __device__ __forceinline__ void bc_push_items(const BcState &st, int32_t *wcnt, 
         atomicOr(st.err, DEV_ERR_OVERFLOW);
     }
   }
-  const int32_t nch = deg > kBcLight ? (deg + st.chunk - 1) / st.chunk : 0;
+  const int32_t nch = deg > st.light ? (deg + st.chunk - 1) / st.chunk : 0;
   if (!__any_sync(0xffffffffu, nch > 0)) return;
   int32_t incl = nch;
 #pragma unroll
@@ -238,7 +239,7 @@ __device__ __forceinline__ void bc_each_item(const BcState &st, const BcItems &w
       const int64_t it = __ldcg(st.work + i);
       const int32_t v = (int32_t)(it >> 32), c = (int32_t)(uint32_t)it;
       const int32_t kb = __ldg(st.toff + v), ke = __ldg(st.toff + v + 1);
-      if (ke - kb <= kBcLight)
+      if (ke - kb <= st.light)
         f(v, 0, kb, ke, true);
       else
         f(v, c, kb + c * st.chunk, min(ke, kb + (c + 1) * st.chunk), ke - kb <= st.chunk);
@@ -608,6 +609,7 @@ static BcState bcb_state(gg_graph *g, const BcBuffers &b, int32_t k) {
   S.work = b.work;
   S.wcap = (int32_t)bc_wcap(g);
   S.chunk = effective_tuning(g, GG_BATCH_BC, 1).chunk;
+  S.light = std::min(kBcLight, S.chunk);
   S.depth = b.depth;
   S.sigma = b.vals;
   S.dep = b.vals + (size_t)kBcWidth * V;

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 import oracle
-from easy_graphit_gb300 import BatchPlan, GraphT, HostGraph, bc_batch
+from easy_graphit_gb300 import BatchPlan, GraphT, HostGraph, bc_batch, set_batch_tuning
 from tests.conftest import rel_l1
 
 pytestmark = pytest.mark.gpu
@@ -34,4 +34,18 @@ def test_few_items(name, nsrc):
         for s in range(nsrc):
             assert rel_l1(rows[s], ref[s]) <= TOL
             assert rel_l1(out[s].cpu().numpy(), ref[s]) <= TOL
+    g.close()
+
+
+@pytest.mark.parametrize("chunk", [32, 64, 128, 256])
+def test_item_sizes(chunk):
+    """The tuning's chunk bounds every work item, also where it is below a light item's size."""
+    hg = HostGraph.rmat(9, 40, symmetrize=True)
+    g = GraphT(hg, symmetric=True)
+    off, dst = np.array(hg.offsets), np.array(hg.dst)
+    srcs = hg.pick_sources(5)
+    set_batch_tuning(g, "bc", chunk=chunk)
+    rows, _ = bc_batch(g, srcs)
+    for s, row in zip(srcs, rows):
+        assert rel_l1(row, oracle.bc(off, dst, int(s))) <= TOL
     g.close()
