@@ -87,6 +87,8 @@ __device__ __forceinline__ void ms_fold(const MsAcc &t, unsigned long long *s_ac
 // the whole CTA.  With a group per vertex and 8 in flight, a hub that one source
 // does not reach was walked alone for 2.4 ms, whatever the level held (1 M
 // vertices; a level that chose bottom-up with such a hub in it: 3.2 ms of 4.9).
+// Lengths of 256 / 512 / 2,048: symmetrized R-MAT 20 1.03 / 0.92 / 0.99 ms, 22 3.76 / 3.13 /
+// 3.06, directed 20 0.81 / 0.81 / 0.84; 64 lists a CTA instead of 256: 22 4.85.
 constexpr int32_t kMsLong = 512;
 constexpr int32_t kMsLongMax = 256;  // set aside per CTA; more are walked by groups
 struct MsLong {

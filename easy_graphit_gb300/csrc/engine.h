@@ -48,7 +48,9 @@ struct TrialOut {
   int32_t err;                        // device status word
 };
 constexpr int32_t kPinnedInts = 64;         // h_pinned: small copies
-constexpr size_t kStageBytes = 60 * 1024;   // h_stage: results up to this size
+// h_stage: results up to this size.  BFS of 7,000 vertices with parents 92 us unstaged,
+// 89 staged; of 400,000 212 and 313: the copy out of it costs more than it saves.
+constexpr size_t kStageBytes = 60 * 1024;
 }  // namespace gg
 
 struct gg_graph {
