@@ -8,6 +8,9 @@
  *  - The reference reports errors with exit(-1)/assert (support.h:4-10,
  *    graph.h:251-253, operators.cpp:543,646).  Every entry point here returns a
  *    gg_status instead; gg_last_error() gives the message of the calling thread.
+ *    A call that returns an error may have written to its output arrays: results
+ *    are copied out together with the status word, not after it (a wait more, 8 us
+ *    of a BFS of 100 to 300 us).
  *  - The reference owns all device memory (cudaMalloc, never freed).  Here each
  *    handle owns its device memory and releases it in its *_destroy call.  Input
  *    pointers may be host or device memory (copied with cudaMemcpyDefault); the
