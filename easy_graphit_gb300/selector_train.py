@@ -1,8 +1,8 @@
 """Trains the learned schedule selector on timings generated by the engine.
 
     python -m easy_graphit_gb300.selector_train [--out easy_graphit_gb300/selector_model.bin]
-    python -m easy_graphit_gb300.selector_train --batched-bfs [--out .../selector_batched_bfs.bin]
-    python -m easy_graphit_gb300.selector_train --fused-bfs [--out .../selector_fused_bfs.bin]
+    python -m easy_graphit_gb300.selector_train --batched-bfs --grids 256,512,1536 [--out .../selector_batched_bfs.bin]
+    python -m easy_graphit_gb300.selector_train --fused-bfs --grids 256,512,1536 [--out .../selector_fused_bfs.bin]
 
 --batched-bfs trains the per-level direction of the batched BFS instead: on
 each training graph, 64 sources are traversed with every level top-down and
@@ -18,7 +18,9 @@ level pushed and then pulled (gg_bfs_collect_directions); held-out graphs
 compare the network with bfs.cpp's two schedules and with its hybrid rule fused.
 
 Training graphs: R-MAT at scales 18 to 24 with skew a in [0.45, 0.75] (b = c =
-(0.95 - a) / 2) and 2-D grids, GAPBS-seeded; for each, BFS and SSSP runs
+(0.95 - a) / 2) and 2-D grids, GAPBS-seeded (the direction networks' up to 1536^2: with
+256^2 and 512^2 alone, where pulling costs no more, the held-out 1024^2 grid was pulled,
+24.6 ms against 19.1); for each, BFS and SSSP runs
 (delta 32) and CC.  At every iteration the engine times all 36 candidate
 schedules on the same state (gg_selector_collect); the fastest candidate's
 (direction, load balancing, frontier type) is the label.  Training is
