@@ -66,6 +66,7 @@ struct BqArgs {
   int32_t *hub_list;    // hub chunks (HubList); their counts are control words
   int32_t hub_cap, hub_min, hub_slices;
   int32_t stage_cap, stage_at;  // the three stages: entries each, where they start in shared memory
+  int32_t near_cap;     // frontier entries a mesh session takes: at most kMeshNear
   int32_t mesh;         // largest out-degree <= 32: one-CTA sessions run in shared memory (bq_mesh_session)
 };
 
@@ -401,7 +402,7 @@ __device__ __forceinline__ void mesh_relax_pass(const BqLoop &s, const BqArgs &a
         }
         const int32_t pos = mesh_places(to, cnt);
         if (to == 0) {
-          if (pos < kMeshNear) {
+          if (pos < a.near_cap) {
             m.near_[in ^ 1][pos] = make_int4(v, p, db[j], de[j]);
           } else {
             m.full = 1;
@@ -486,7 +487,7 @@ __device__ __forceinline__ void bq_mesh_session(BqLoop &s, const BqArgs &a, int3
       s.relax++;
       __syncthreads();
       in ^= 1;
-      n = min(m.n_near[in], kMeshNear);
+      n = min(m.n_near[in], a.near_cap);
       const bool leave = m.full || m.quit;
       const bool flush = m.n_hi > kMeshHigh / 2;
       __syncthreads();
@@ -532,7 +533,7 @@ __device__ __forceinline__ void bq_mesh_session(BqLoop &s, const BqArgs &a, int3
         const int32_t pos = mesh_places(to, cnt);
         if (to == 1) m.lo[L ^ 1][pos] = x;
         if (to == 0) {
-          if (pos < kMeshNear) {
+          if (pos < a.near_cap) {
             m.near_[in][pos] = x;
           } else {
             m.full = 1;
@@ -545,7 +546,7 @@ __device__ __forceinline__ void bq_mesh_session(BqLoop &s, const BqArgs &a, int3
       s.adv++;
       adv++;
       __syncthreads();
-      n = min(m.n_near[in], kMeshNear);
+      n = min(m.n_near[in], a.near_cap);
       if (m.full || m.quit) break;
     }
   }

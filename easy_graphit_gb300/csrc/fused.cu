@@ -171,7 +171,7 @@ __device__ __forceinline__ void bq_solo(BqLoop &s, const BqArgs &a, BqStep st, i
   __syncthreads();
   for (int32_t steps = 1;; ++steps) {
     const int32_t near_n = st.kind == BQ_RELAX ? st.work : 0;
-    if (a.mesh && (st.kind == BQ_RELAX || st.kind == BQ_LOMIN) && near_n <= kMeshNear / 4 * 3 &&
+    if (a.mesh && (st.kind == BQ_RELAX || st.kind == BQ_LOMIN) && near_n <= a.near_cap / 4 * 3 &&
         sctl[BQ_LO + (s.g & 1)] <= kMeshLow) {
       bq_mesh_session(s, a, sctl, *reinterpret_cast<BqMeshSmem *>(smem), near_n, t0);
       steps |= 7;  // long enough to check the clock
@@ -929,6 +929,11 @@ static BqArgs bq_args(gg_graph *g, gg_frontier *f, const BqBuffers &b, int32_t *
   a.hub_cap = hub_capacity(g);
   a.hub_min = kHubWidths * cta;
   a.hub_slices = slice_limit(g->max_degree);
+  // A session gives the frontier back to the GPU where it is more than the CTA was
+  // meant to take alone (1024^2 grid, delta 2,000, waves of 1,500 vertices: CTAs of 128
+  // 37.7 ms held to 2,048 entries, 24.3 to 512; of 256 27.8 and 23.6; with 256 entries
+  // CTAs of 64 lose on narrower waves, 47 against 55 ms on 700^2 at delta 128).
+  a.near_cap = std::min(kMeshNear, std::max(512, a.solo_max));
   a.mesh = g->max_degree <= kMeshMaxDegree && a.solo_max > 0;
   // Low-pile entries of a refill.  A mesh session reads them at every advance
   // (2048^2 grid, delta 8: 1123 ms with 2,048, 580 with 1,024, 398 with 512); the

@@ -75,7 +75,7 @@ __device__ __forceinline__ void lb_vertex(const DGraph &g, const Enum &en, int32
   F h = f;
   if (e - b > kStageCap / 2) {  // a hub's thread would fill the stages, then try them for nothing
     o.stage = nullptr;
-    if constexpr (lb_batch<F>::value) h.stage_parks(nullptr, nullptr);
+    if constexpr (lb_batch<F>::value) h.alone();
   }
   do_range<kSerialInFlight>(g, h, o, s, b, e, 0, 1);
 }

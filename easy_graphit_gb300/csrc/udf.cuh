@@ -232,6 +232,16 @@ struct EdgeF {
       u.far.hi_stage = hi;
     }
   }
+  // For a thread that walks a hub alone: appends go directly, and its near improvements
+  // are queued without a claim, whose answers it would wait for batch after batch (a
+  // star of a million leaves at delta 2,000, a thread per vertex: 318 -> 276 ms; directed
+  // R-MAT 22 63.0 -> 60.6).
+  __device__ __forceinline__ void alone() {
+    if constexpr (kBatch) {
+      u.far.lo_stage = u.far.hi_stage = nullptr;
+      u.far.near_tag = 0;
+    }
+  }
   // Only used when kBatch; the source filter (in_src) is checked by the caller.
   template <int B, class G, class Out>
   __device__ __forceinline__ void relax_range(const G &g, const Out &out, int32_t s, int32_t b, int32_t e,
