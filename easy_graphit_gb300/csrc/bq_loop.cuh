@@ -290,7 +290,7 @@ __device__ __forceinline__ void bq_step(BqLoop &s, const BqArgs &a, const BqStep
 // a session's relax of 250 vertices takes 5,000 cycles, of 8 2,300, an advance
 // over a pile of 900 3,900 (bq_step: 7,300 a step).
 constexpr int32_t kMeshMaxDegree = 32;
-constexpr int32_t kMeshNear = 2048;  // frontier entries a session holds
+constexpr int32_t kMeshNear = 1024;  // frontier entries a session holds
 constexpr int32_t kMeshLow = 2048;   // low-pile entries
 constexpr int32_t kMeshHigh = 1024;  // high parks buffered between flushes
 struct BqMeshSmem {

@@ -929,10 +929,11 @@ static BqArgs bq_args(gg_graph *g, gg_frontier *f, const BqBuffers &b, int32_t *
   a.hub_cap = hub_capacity(g);
   a.hub_min = kHubWidths * cta;
   a.hub_slices = slice_limit(g->max_degree);
-  // A session gives the frontier back to the GPU where it is more than the CTA was
-  // meant to take alone (1024^2 grid, delta 2,000, waves of 1,500 vertices: CTAs of 128
-  // 37.7 ms held to 2,048 entries, 24.3 to 512; of 256 27.8 and 23.6; with 256 entries
-  // CTAs of 64 lose on narrower waves, 47 against 55 ms on 700^2 at delta 128).
+  // A session gives the frontier back where it is more than four entries a thread (512
+  // at least, 1,024 at most): 1024^2 grid, delta 2,000, waves of 1,500 vertices, CTAs of
+  // 64 / 128 / 256 / 512 with 2,048 entries 54.3 / 37.7 / 27.8 / 24.7 ms, so 26.5 / 23.5 / 23.4 /
+  // 20.8; with 256 entries CTAs of 64 lose on narrower waves (700^2, delta 128: 47
+  // against 55), with 512 those of 256 (1024^2, delta 300: 34.0 against 37.1).
   a.near_cap = std::min(kMeshNear, std::max(512, a.solo_max));
   a.mesh = g->max_degree <= kMeshMaxDegree && a.solo_max > 0;
   // Low-pile entries of a refill.  A mesh session reads them at every advance
