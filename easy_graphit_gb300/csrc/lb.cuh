@@ -37,6 +37,16 @@ struct lb_batch<F, decltype(void(F::kBatch))> {
   static constexpr bool value = F::kBatch;
 };
 
+// Whether a functor pulls (EdgeF).
+template <class F, class = void>
+struct lb_pulls {
+  static constexpr bool value = false;
+};
+template <class F>
+struct lb_pulls<F, decltype(void(F::kPulls))> {
+  static constexpr bool value = F::kPulls;
+};
+
 // Edges [b, e) of source s processed by `width` cooperating threads (rank r).
 // A functor with a batched range relax (push, no per-edge source test beyond
 // the first) takes the whole range at once, B edges of a thread in flight.
@@ -67,7 +77,8 @@ __device__ __forceinline__ void lb_vertex(const DGraph &g, const Enum &en, int32
   if (i >= n) return;
   const int32_t s = en.at(i);
   const int32_t b = __ldg(g.off + s), e = __ldg(g.off + s + 1);
-  if (e - b <= 4) {
+  // a pull appends the thread's own vertex at most
+  if (lb_pulls<F>::value || e - b <= 4) {
     do_range(g, f, out, s, b, e, 0, 1);
     return;
   }

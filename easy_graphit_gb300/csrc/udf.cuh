@@ -199,7 +199,7 @@ struct EdgeF {
   static constexpr bool kRunSums = PULL && sums_of<U>::value;
   __device__ __forceinline__ float term(int32_t d) const { return u.term(d); }
   __device__ __forceinline__ void add(int32_t s, float x) const { u.add(s, x); }
-  static constexpr bool kWeight = U::kWeight;
+  static constexpr bool kWeight = U::kWeight, kPulls = PULL;
   static constexpr bool kPushes = U::kPushes;  // whether apply ever tracks a vertex
   // push direction with a UDF that has a batched range relax (its to() filter
   // passes every vertex, so the range needs no per-edge destination test)
