@@ -7,8 +7,6 @@
 // Sparse-queue counts rotate through three slots: iteration L reads slot
 // (L-1)%3, appends to slot L%3 and clears slot (L+1)%3, whose last reader
 // finished before the previous barrier -- one barrier per iteration.
-#include <cooperative_groups/reduce.h>
-
 #include <cstdlib>
 
 #include "batch.h"
