@@ -66,6 +66,7 @@ struct BqArgs {
   int32_t *hub_list;    // hub chunks (HubList); their counts are control words
   int32_t hub_cap, hub_min, hub_slices;
   int32_t stage_cap, stage_at;  // the three stages: entries each, where they start in shared memory
+  int32_t alone_max;    // frontier entries up to which hubs' threads queue near vertices unclaimed
   int32_t near_cap;     // frontier entries a mesh session takes: at most kMeshNear
   int32_t mesh;         // largest out-degree <= 32: one-CTA sessions run in shared memory (bq_mesh_session)
 };
@@ -159,9 +160,10 @@ __device__ __forceinline__ void bq_step(BqLoop &s, const BqArgs &a, const BqStep
       front.q = qin;
       front.cnt = ctl + BQ_NEAR + (s.it + 2) % 3;
     }
+    const uint32_t near_tag = bq_near_tag(s.relax - (hubs ? 1 : 0));
     const DFar far{a.b.stamp, a.b.lo[s.g & 1], ctl + BQ_LO + (s.g & 1), a.b.hi[s.gh & 1],
                    ctl + BQ_HI + (s.gh & 1), bq_lo_tag(s.g), bq_hi_tag(s.gh), s.hz, a.b.V, a.err, st_lo, st_hi,
-                   bq_near_tag(s.relax - (hubs ? 1 : 0))};
+                   near_tag, !hubs && st.work <= a.alone_max ? 0u : near_tag};
     const EdgeF<USssp, false> f{USssp{a.dist, U, far}, DIn{IN_ALL, nullptr, nullptr},
                                 DIn{IN_ALL, nullptr, nullptr}, false};
     if (hubs) {

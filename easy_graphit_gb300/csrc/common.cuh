@@ -262,6 +262,9 @@ struct DFar {
   // vertex every time.  With it a vertex is queued once a step, and a park that
   // another thread of the step decided on an older distance is refused.
   uint32_t near_tag;
+  // The same for a thread that walks a hub alone: near_tag, or 0 in a step whose
+  // queue holds what its threads find unclaimed too (BqArgs::alone_max).
+  uint32_t near_alone;
 
   __device__ __forceinline__ uint32_t tag_of(int32_t p) const { return p < horizon ? lo_tag : hi_tag; }
   __device__ __forceinline__ void park(int32_t v, int32_t p) const {

@@ -927,6 +927,10 @@ static BqArgs bq_args(gg_graph *g, gg_frontier *f, const BqBuffers &b, int32_t *
   a.hub_cap = hub_capacity(g);
   a.hub_min = kHubWidths * cta;
   a.hub_slices = slice_limit(g->max_degree);
+  // What unclaimed finds of a step can fill beside the V claimed ones: every edge of
+  // its vertices.  In wide steps the threads lower a vertex together and would each
+  // queue it (complete graph of 1,100 vertices, its second step: 90 entries a vertex).
+  a.alone_max = (int32_t)std::min<int64_t>(INT_MAX, (f->cap - g->csr.V) / std::max(1, g->max_degree));
   // A session gives the frontier back where it is more than four entries a thread (512
   // at least, 1,024 at most): 1024^2 grid, delta 2,000, waves of 1,500 vertices, CTAs of
   // 64 / 128 / 256 / 512 with 2,048 entries 54.3 / 37.7 / 27.8 / 24.7 ms, so 26.5 / 23.5 / 23.4 /

@@ -232,14 +232,14 @@ struct EdgeF {
       u.far.hi_stage = hi;
     }
   }
-  // For a thread that walks a hub alone: appends go directly, and its near improvements
-  // are queued without a claim, whose answers it would wait for batch after batch (a
-  // star of a million leaves at delta 2,000, a thread per vertex: 318 -> 276 ms; directed
-  // R-MAT 22 63.0 -> 60.6).
+  // For a thread that walks a hub alone: appends go directly, and in a step of few
+  // vertices its near improvements are queued without a claim, whose answers it would
+  // wait for batch after batch (a star of a million leaves at delta 2,000, a thread per
+  // vertex: 318 -> 276 ms).
   __device__ __forceinline__ void alone() {
     if constexpr (kBatch) {
       u.far.lo_stage = u.far.hi_stage = nullptr;
-      u.far.near_tag = 0;
+      u.far.near_tag = u.far.near_alone;
     }
   }
   // Only used when kBatch; the source filter (in_src) is checked by the caller.
