@@ -546,11 +546,6 @@ static gg_status graph_init(gg_graph *g, const int32_t *offsets, const int32_t *
   GG_CUDA(cudaMemsetAsync(g->d_misc, 0, sizeof(int32_t) * 128, st));
   GG_CUDA(cudaMallocHost(&g->h_pinned, sizeof(int32_t) * kPinnedInts + 256 + kStageBytes));
   GG_CUDA(cudaMemcpyAsync(s.off, offsets, sizeof(int32_t) * (V + 1), cudaMemcpyDefault, st));
-  // the longest list, before the edges: what its kernel and copy take is hidden behind theirs
-  note_launch();
-  k_max_degree<<<std::max(1, std::min(ceil_div(V, 256), g->sm_count * 4)), 256, 0, st>>>(s.off, V, g->d_misc + 60);
-  GG_CUDA(cudaGetLastError());
-  GG_CUDA(cudaMemcpyAsync(g->h_pinned + 60, g->d_misc + 60, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   if (E) {
     GG_CUDA(cudaMemcpyAsync(s.dst, dst, sizeof(int32_t) * E, cudaMemcpyDefault, st));
     if (weights) {
@@ -561,6 +556,11 @@ static gg_status graph_init(gg_graph *g, const int32_t *offsets, const int32_t *
       GG_CUDA(cudaStreamSynchronize(st));
     }
   }
+  // the longest list, while the host sets up the rest
+  note_launch();
+  k_max_degree<<<std::max(1, std::min(ceil_div(V, 256), g->sm_count * 4)), 256, 0, st>>>(s.off, V, g->d_misc + 60);
+  GG_CUDA(cudaGetLastError());
+  GG_CUDA(cudaMemcpyAsync(g->h_pinned + 60, g->d_misc + 60, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   GG_CUDA(dev_alloc(&g->d_err, sizeof(int32_t), st));
   GG_CUDA(dev_alloc(&g->d_bar, sizeof(uint32_t) * 2, st));
   GG_CUDA(cudaMemsetAsync(g->d_err, 0, sizeof(int32_t), st));
