@@ -430,12 +430,6 @@ gg_status run_bfs(gg_graph *g, const gg_app_schedule *s, const int32_t *srcs, in
   return check_device_error(g, "bfs");
 }
 
-// Host-driven steps claim near vertices as the fused loop's do (DFar::near_tag) on graphs
-// with longer lists than this: unclaimed, the threads that lower a vertex together each
-// queue it and the copies multiply (complete graph of 400 vertices: more than the queue's
-// six a vertex; R-MAT 18 symmetrized, delta 2,000, TWCE 0.91 -> 0.78 ms).  A grid's few edges a vertex make few copies, and a claim
-// is one more round trip (R-MAT 9, TWCE: 430 -> 462 us).
-constexpr int32_t kUnclaimedDegree = 8;
 gg_status run_sssp(gg_graph *g, const gg_app_schedule *s, const int32_t *srcs, int32_t nsrc,
                    int32_t delta, int32_t *dist, gg_stats *st) {
   const int32_t src = nsrc == 1 ? srcs[0] : -1;
@@ -467,7 +461,7 @@ gg_status run_sssp(gg_graph *g, const gg_app_schedule *s, const int32_t *srcs, i
   }
   LoopTimer lt(g);
   Chooser ch{g, s};
-  for (int32_t step = 0;; ++step) {
+  for (;;) {
     bool fin = false;
     GG_TRY(pq_finished(pq, &fin));
     if (fin) break;
@@ -476,11 +470,7 @@ gg_status run_sssp(gg_graph *g, const gg_app_schedule *s, const int32_t *srcs, i
     GG_TRY(frontier_size(pq->frontier, &n));
     const gg_schedule *sc = nullptr;
     GG_TRY(ch.choose(pq->frontier, n, &sc));
-    vd.far = pq_far(pq);
-    if (g->max_degree > kUnclaimedDegree) {
-      vd.far.near_tag = bq_near_tag(step);
-      vd.far.near_alone = (int64_t)n * g->max_degree <= pq->frontier->cap - g->csr.V ? 0u : vd.far.near_tag;
-    }
+    vd.far = pq_step_far(pq, n);
     GG_TRY(edgeset_apply_impl(g, sc, GG_UDF_SSSP_RELAX, GG_FILTER_NONE, pq->frontier, pq->frontier,
                               true, vd, pq_cutoff(pq), false));
     if (st) st->iterations++;

@@ -112,6 +112,7 @@ struct gg_pq {
   int64_t advances = 0;
   gg::BqBuffers bq;                // far piles (bucket_queue.cuh), also used by the fused loop
   int32_t gen_lo = 0, gen_hi = 0;  // pile generations of the host-driven queue
+  int32_t steps = 0;               // host-driven relaxes that claim near vertices
   int32_t horizon = INT_MAX;
   int32_t width = 16;              // horizon width in buckets
 };
@@ -226,6 +227,8 @@ gg_status pq_reset(gg_pq *pq, int32_t init_priority, int32_t delta, int32_t src)
 void pq_reset_host(gg_pq *pq, int32_t init_priority, int32_t delta);  // its host state alone
 int32_t pq_cutoff(const gg_pq *pq);
 DFar pq_far(const gg_pq *pq);  // far piles the relax parks into
+// The same for the next relax of a host-driven loop, over n frontier vertices (-1: unknown).
+DFar pq_step_far(gg_pq *pq, int64_t n);
 
 // ---- fused.cu: whole-loop persistent kernels (fuse_kernel, operators.cpp:652-672).
 // *ran is false when the schedule has no device-side form (the caller then

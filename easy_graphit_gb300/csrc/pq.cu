@@ -57,6 +57,23 @@ DFar pq_far(const gg_pq *pq) {
               b.V, pq->g->d_err};
 }
 
+// Host-driven steps claim near vertices as the fused loop's do (DFar::near_tag) on graphs
+// with longer lists than this: unclaimed, the threads that lower a vertex together each
+// queue it and the copies multiply (complete graph of 400 vertices: more than the queue's
+// six a vertex; R-MAT 18 symmetrized, delta 2,000, TWCE 0.91 -> 0.78 ms).  A grid's few
+// edges a vertex make few copies, and a claim is one more round trip (R-MAT 9, TWCE: 430
+// -> 462 us).
+constexpr int32_t kUnclaimedDegree = 8;
+DFar pq_step_far(gg_pq *pq, int64_t n) {
+  DFar far = pq_far(pq);
+  const gg_graph *g = pq->g;
+  if (g->max_degree > kUnclaimedDegree) {
+    far.near_tag = bq_near_tag(pq->steps++);
+    far.near_alone = n >= 0 && n * g->max_degree <= pq->frontier->cap - g->csr.V ? 0u : far.near_tag;
+  }
+  return far;
+}
+
 // dequeueReadySet's advance (gpu_priority_queue.h:125-149) over the far piles.
 gg_status pq_advance(gg_pq *pq) {
   gg_graph *g = pq->g;
@@ -185,6 +202,7 @@ void pq_reset_host(gg_pq *pq, int32_t init_priority, int32_t delta) {
   pq->advances = 0;
   pq->gen_lo = 0;
   pq->gen_hi = 0;
+  pq->steps = 0;
   pq->width = 16;
   pq->horizon = bq_clamp((int64_t)init_priority + (int64_t)pq->width * delta);
   pq->frontier->fmt = GG_FMT_SPARSE;
@@ -266,7 +284,7 @@ gg_status gg_edgeset_apply_priority(gg_graph *g, const gg_schedule *s, gg_pq *pq
   GG_CHECK_ARG(g && s && pq, "bad arguments");
   VData d = to_vdata(vd);
   d.dist = pq->prio;
-  d.far = pq_far(pq);
+  d.far = pq_step_far(pq, -1);
   GG_TRY(edgeset_apply_impl(g, s, GG_UDF_SSSP_RELAX, GG_FILTER_NONE, pq->frontier, pq->frontier,
                             true, d, pq_cutoff(pq), false));
   return check_device_error(g, "apply_priority");

@@ -4,7 +4,8 @@ import numpy as np
 import pytest
 
 import oracle
-from easy_graphit_gb300 import GraphT, HostGraph, SimpleGPUSchedule as T, sssp, sssp_multi
+from easy_graphit_gb300 import (UDF, VUDF, GraphT, HostGraph, PriorityQueue, SimpleGPUSchedule as T, VertexData,
+                                edgeset_apply, sssp, sssp_multi, vertexset_apply)
 
 pytestmark = pytest.mark.gpu
 LB = T.load_balancing_type
@@ -32,4 +33,21 @@ def test_distances_and_advances(n, wmax, delta):
     each = np.minimum(ref, oracle.sssp_dijkstra(off, dst, w, n - 1))
     np.testing.assert_array_equal(sssp_multi(g, np.array([0, n - 1], np.int32), delta,
                                              T().configLoadBalancing(LB.TWCE), False)[0], each)
+    g.close()
+
+
+@pytest.mark.parametrize("lb", [LB.VERTEX_BASED, LB.TWC, LB.TWCE])
+def test_through_operators(lb):
+    import torch
+    hg = dense(400, 255)
+    g = GraphT(hg)
+    off, dst, w = np.array(hg.offsets), np.array(hg.dst), np.array(hg.weights)
+    for src, delta in ((0, 32), (7, 2000)):
+        sp = torch.empty(400, dtype=torch.int32, device="cuda")
+        pq = PriorityQueue(g, sp, 0, delta, src)
+        vertexset_apply(g, VUDF.SSSP_RESET, VertexData(dist=sp, src=src))
+        while not pq.finished():
+            edgeset_apply(T().configLoadBalancing(lb)).from_(pq.dequeue()).apply_priority(g, UDF.SSSP_RELAX, pq)
+        pq.close()
+        np.testing.assert_array_equal(sp.cpu().numpy(), oracle.sssp_dijkstra(off, dst, w, src))
     g.close()
